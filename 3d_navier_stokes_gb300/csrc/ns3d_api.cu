@@ -8,6 +8,7 @@
 #include <complex>
 #include <vector>
 
+#include "fxfft.cuh"
 #include "ns3d_base.h"
 
 namespace ns3d {
@@ -24,32 +25,47 @@ bool supported_n(int N) {
     }
 }
 
-// e^{-2 pi i m / n}: quarter-turn reduction so that 1, -i, -1, i are exact,
-// then cos/sin of the residual angle evaluated in long double.
-void twiddle_table(int n, double* re, double* im) {
+// cos and sin of 2 pi m / n, m < n: quarter-turn reduction so that 0 and +-1 are
+// exact, then cos/sin of the residual angle evaluated in long double.
+static void unit_circle(int n, long m, long double* co, long double* si) {
     const long double half_pi = acosl(-1.0L) / 2.0L;
+    const long q = (4 * m) / n, r = 4 * m - q * n;
+    long double c, s;
+    if (2 * r <= n) {
+        const long double phi = half_pi * (long double)r / (long double)n;
+        c = cosl(phi);
+        s = sinl(phi);
+    } else {
+        const long double phi = half_pi * (long double)(n - r) / (long double)n;
+        c = sinl(phi);
+        s = cosl(phi);
+    }
+    switch (q) {
+        case 0: *co = c; *si = s; break;
+        case 1: *co = -s; *si = c; break;
+        case 2: *co = -c; *si = -s; break;
+        default: *co = s; *si = -c; break;
+    }
+}
+// e^{-2 pi i m / n} in FP64
+void twiddle_table(int n, double* re, double* im) {
     for (long m = 0; m < n; ++m) {
-        long q = (4 * m) / n;
-        long r = 4 * m - q * n;
-        long double cs, sn;
-        if (2 * r <= n) {
-            long double phi = half_pi * (long double)r / (long double)n;
-            cs = cosl(phi);
-            sn = sinl(phi);
-        } else {
-            long double phi = half_pi * (long double)(n - r) / (long double)n;
-            cs = sinl(phi);
-            sn = cosl(phi);
-        }
-        double c = (double)cs, s = (double)sn, cr, sr;
-        switch (q) {
-            case 0: cr = c; sr = s; break;
-            case 1: cr = -s; sr = c; break;
-            case 2: cr = -c; sr = -s; break;
-            default: cr = s; sr = -c; break;
-        }
-        re[m] = cr;
-        im[m] = -sr;
+        long double c, s;
+        unit_circle(n, m, &c, &s);
+        re[m] = (double)c;
+        im[m] = -(double)s;
+    }
+}
+// the same as packed 62-bit integers (fxfft.cuh): four ints per entry
+void fx_twiddle_table(int n, int* out) {
+    for (long m = 0; m < n; ++m) {
+        long double c, s;
+        unit_circle(n, m, &c, &s);
+        const q64 qc = (q64)roundl(c * 4611686018427387904.0L), qs = (q64)roundl(-s * 4611686018427387904.0L);
+        out[4 * m] = fx_hi(qc);
+        out[4 * m + 1] = fx_lo(qc);
+        out[4 * m + 2] = fx_hi(qs);
+        out[4 * m + 3] = fx_lo(qs);
     }
 }
 

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "ns3d_base.h"
+#include "fx_passes.cuh"
 #include "ns3d_kernels.cuh"
 
 namespace ns3d {
@@ -31,6 +32,7 @@ namespace ns3d {
 
 // e^{-2 pi i m / n} with the quarter-turn reduction used by the transforms.
 void twiddle_table(int n, double* re, double* im);
+void fx_twiddle_table(int n, int* out);   // packed integers of the FP64 engines
 // 4D FP32 tensor map without swizzle (ns3d_misc.cu)
 bool encode_map4_f32(CUtensorMap* map, void* base, const uint64_t dims[4], const uint64_t strides[3],
                      const uint32_t box[4]);
@@ -80,7 +82,7 @@ class Impl final : public Base {
         for (void* q : {(void*)U_, (void*)UT_, (void*)ACC_, (void*)W_, (void*)tw_, (void*)tab_, (void*)part_,
                         (void*)mout_, (void*)stage_, (void*)real_, (void*)sd_, (void*)TAU_, (void*)F_,
                         (void*)tau_real_, (void*)sgs_part_, (void*)K_, (void*)dpart_, (void*)plan_out_.ranges, (void*)plan_in_.ranges,
-                        (void*)zg_b_, (void*)zg_P_, (void*)xt_items_})
+                        (void*)zg_b_, (void*)zg_P_, (void*)xt_items_, (void*)aux_})
             if (q) cudaFree(q);
         if (sd_host_) cudaFreeHost(sd_host_);
         if (mout_host_) cudaFreeHost(mout_host_);
@@ -122,10 +124,14 @@ class Impl final : public Base {
         NS3D_CK(cudaEventCreate(&ev0_));
         NS3D_CK(cudaEventCreate(&ev1_));
         // twiddles
-        std::vector<double> re(N), im(N);
-        twiddle_table(N, re.data(), im.data());
         std::vector<cx<T>> h(N);
-        for (int m = 0; m < N; ++m) { h[m].x = T(re[m]); h[m].y = T(im[m]); }
+        if constexpr (sizeof(T) == 8) {
+            fx_twiddle_table(N, reinterpret_cast<int*>(h.data()));
+        } else {
+            std::vector<double> re(N), im(N);
+            twiddle_table(N, re.data(), im.data());
+            for (int m = 0; m < N; ++m) { h[m].x = T(re[m]); h[m].y = T(im[m]); }
+        }
         NS3D_CK(cudaMemcpyAsync(tw_, h.data(), sizeof(cx<T>) * N, cudaMemcpyHostToDevice, s_));
         // step state
         for (int m = 0; m < M_; ++m) {
@@ -137,10 +143,23 @@ class Impl final : public Base {
         }
         NS3D_CK(cudaMemcpyAsync(sd_, sd_host_, sizeof(StepDev) * M_, cudaMemcpyHostToDevice, s_));
         // opt-in shared memory sizes
-        NS3D_CK(cudaFuncSetAttribute(k_xinv<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_xi()));
+        if constexpr (sizeof(T) == 8) {
+            NS3D_CK(cudaFuncSetAttribute(k_xinv_fx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, fxinv_smem<N>()));
+            // 1/k2 and the x rows' wavenumbers (fx_passes.cuh)
+            std::vector<double> aux(G::KC2 + 1 + N);
+            for (int k2 = 1; k2 <= G::KC2; ++k2) aux[k2] = 1.0 / k2;
+            for (int i = 0; i < N; ++i) aux[G::KC2 + 1 + i] = i <= N / 2 ? i : i - N;
+            NS3D_CK(cudaMalloc(&aux_, sizeof(double) * aux.size()));
+            NS3D_CK(cudaMemcpy(aux_, aux.data(), sizeof(double) * aux.size(), cudaMemcpyHostToDevice));
+        } else {
+            NS3D_CK(cudaFuncSetAttribute(k_xinv<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_xi()));
+        }
         NS3D_CK(cudaFuncSetAttribute(k_ypass<T, N, true, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_a()));
         NS3D_CK(cudaFuncSetAttribute(k_ypass<T, N, false, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_af()));
-        NS3D_CK(cudaFuncSetAttribute(k_zpass<T, N, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_z()));
+        if constexpr (sizeof(T) == 8)
+            NS3D_CK(cudaFuncSetAttribute(k_zfx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, zfx_smem<N>()));
+        else
+            NS3D_CK(cudaFuncSetAttribute(k_zpass<T, N, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_z()));
         if constexpr (zline_ok<T, N>()) {
             NS3D_CK(cudaFuncSetAttribute(k_zline<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_zl()));
             int per_sm = 0, nsm = 0, dev = 0;
@@ -192,8 +211,7 @@ class Impl final : public Base {
         }
         set_xfwd_attrs<INT_IFRK4>();
         set_xfwd_attrs<INT_RK4CN>();
-        NS3D_CK(cudaFuncSetAttribute(k_xfwd<T, N, INT_TAB, X_STAGE1, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     smem_x()));
+        set_xfwd_attr<INT_TAB, X_STAGE1>();
         tables(0, 0, M_);
         NS3D_CK(cudaGetLastError());
         NS3D_CK(cudaStreamSynchronize(s_));
@@ -223,14 +241,21 @@ class Impl final : public Base {
         return NS3D_OK;
     }
 
+    template <int INTEG, int MODE>
+    void set_xfwd_attr() {
+        if constexpr (sizeof(T) == 8)
+            cudaFuncSetAttribute(k_xfwd_fx<N, INTEG, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, fxfwd_smem<N>());
+        else
+            cudaFuncSetAttribute(k_xfwd<T, N, INTEG, MODE, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
+    }
     template <int INTEG>
     void set_xfwd_attrs() {
-        cudaFuncSetAttribute(k_xfwd<T, N, INTEG, X_STAGE1, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
-        cudaFuncSetAttribute(k_xfwd<T, N, INTEG, X_STAGE2, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
-        cudaFuncSetAttribute(k_xfwd<T, N, INTEG, X_STAGE3, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
-        cudaFuncSetAttribute(k_xfwd<T, N, INTEG, X_STAGE4, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
-        cudaFuncSetAttribute(k_xfwd<T, N, INTEG, X_RHS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
-        cudaFuncSetAttribute(k_xfwd<T, N, INTEG, X_PLAIN, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
+        set_xfwd_attr<INTEG, X_STAGE1>();
+        set_xfwd_attr<INTEG, X_STAGE2>();
+        set_xfwd_attr<INTEG, X_STAGE3>();
+        set_xfwd_attr<INTEG, X_STAGE4>();
+        set_xfwd_attr<INTEG, X_RHS>();
+        set_xfwd_attr<INTEG, X_PLAIN>();
     }
 
     // each launcher covers members [m0, m0 + cnt); `in` points at member 0's arrays
@@ -246,7 +271,11 @@ class Impl final : public Base {
                 return;
             }
         }
-        k_xinv<T, N, V><<<dim3(NTX, G::NKY, cnt), TX * PX::P, smem_xi(), s_>>>(in + (size_t)m0 * 3 * G::FS, Wm(m0), tw_);
+        const cx<T>* src = in + (size_t)m0 * 3 * G::FS;
+        if constexpr (sizeof(T) == 8)
+            k_xinv_fx<N><<<dim3(NTX, G::NKY, 6 * cnt), fxinv_threads<N>(), fxinv_smem<N>(), s_>>>(src, Wm(m0), tw_, aux_);
+        else
+            k_xinv<T, N, V><<<dim3(NTX, G::NKY, cnt), TX * PX::P, smem_xi(), s_>>>(src, Wm(m0), tw_);
     }
     void p2(int m0, int cnt) {
         k_ypass<T, N, true, V><<<dim3(NTA, N, 6 * cnt), TA * PY::P, smem_a(), s_>>>(Wm(m0), tw_);
@@ -278,8 +307,11 @@ class Impl final : public Base {
                 return;
             }
         }
-        k_zpass<T, N, 0><<<dim3((unsigned)((long long)N * N / 2 / ZP), cnt), 3 * PA::P * ZP, smem_z(), s_>>>(
-            Wm(m0), tw_, nullptr, sdm(m0), want_umax);
+        if constexpr (sizeof(T) == 8)
+            k_zfx<N><<<dim3((unsigned)((long long)N * N / 2 / zfx_pairs<N>()), cnt), zfx_threads<N>(), zfx_smem<N>(), s_>>>(
+                Wm(m0), tw_, sdm(m0), want_umax);
+        else
+            k_zpass<T, N, 0><<<dim3((unsigned)((long long)N * N / 2 / ZP), cnt), 3 * PA::P * ZP, smem_z(), s_>>>(Wm(m0), tw_, nullptr, sdm(m0), want_umax);
     }
     void set_zform(int z) override {
         const int zn = (zline_ok<T, N>() && z == 0) ? 0 : (zgemm_ok<T, N>() && z == 2) ? 2 : 1;
@@ -296,15 +328,28 @@ class Impl final : public Base {
     }
     template <int INTEG, int MODE>
     void p5x(int m0, int cnt, cx<T>* out) {
-        k_xfwd<T, N, INTEG, MODE, V><<<dim3(NTXF, G::NKY, cnt), TXF * PX::P, smem_x(), s_>>>(
-            Wm(m0), Um(m0), UTm(m0), out ? out + (size_t)m0 * 3 * G::FS : ACCm(m0), tw_, sdm(m0), tabm(m0),
-            (les_ && MODE <= X_STAGE4) ? F_ : nullptr, nullptr, nullptr, RkStage{});
+        cx<T>* acc = out ? out + (size_t)m0 * 3 * G::FS : ACCm(m0);
+        const dim3 grid(NTXF, G::NKY, cnt);
+        if constexpr (sizeof(T) == 8)
+            k_xfwd_fx<N, INTEG, MODE><<<grid, fxfwd_threads<N>(), fxfwd_smem<N>(), s_>>>(
+                Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0), aux_, nullptr, nullptr, RkStage{});
+        else
+            k_xfwd<T, N, INTEG, MODE, V><<<grid, TXF * PX::P, smem_x(), s_>>>(
+                Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0), (les_ && MODE <= X_STAGE4) ? F_ : nullptr,
+                nullptr, nullptr, RkStage{});
     }
     // RK5-family stage epilogue s (0-based) of members [m0, m0 + cnt)
     void p5tab(int s, int m0, int cnt) {
-        k_xfwd<T, N, INT_TAB, X_STAGE1, V><<<dim3(NTXF, G::NKY, cnt), TXF * PX::P, smem_x(), s_>>>(
-            Wm(m0), Um(m0), UTm(m0), ACCm(m0), tw_, sdm(m0), tabm(m0), les_ ? F_ : nullptr,
-            K_ + (size_t)m0 * 18 * G::FS, dpart_ + (size_t)m0 * 3 * NTXF * G::NKY, rk_stage(s, dp5()));
+        const dim3 grid(NTXF, G::NKY, cnt);
+        cx<T>* K = K_ + (size_t)m0 * 18 * G::FS;
+        double* dpart = dpart_ + (size_t)m0 * 3 * NTXF * G::NKY;
+        if constexpr (sizeof(T) == 8)
+            k_xfwd_fx<N, INT_TAB, X_STAGE1><<<grid, fxfwd_threads<N>(), fxfwd_smem<N>(), s_>>>(
+                Wm(m0), Um(m0), UTm(m0), ACCm(m0), tw_, sdm(m0), tabm(m0), aux_, K, dpart, rk_stage(s, dp5()));
+        else
+            k_xfwd<T, N, INT_TAB, X_STAGE1, V><<<grid, TXF * PX::P, smem_x(), s_>>>(
+                Wm(m0), Um(m0), UTm(m0), ACCm(m0), tw_, sdm(m0), tabm(m0), les_ ? F_ : nullptr, K, dpart,
+                rk_stage(s, dp5()));
     }
     template <int MODE>
     void p5(int m0, int cnt, cx<T>* out = nullptr) {
@@ -321,6 +366,7 @@ class Impl final : public Base {
     // (single run): real-space u, network, r2c of the six tau components,
     // divergence, energy-budget flag. The term is then held for the 4 stages.
     void launch_sgs() {
+      if constexpr (sizeof(T) == 4) {   // attach_les refuses FP64 runs
         p1(U_, 0, 1); p2(0, 1);
         k_zpass<T, N, 1><<<(unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_>>>(
             W_, tw_, real_, nullptr, 0);
@@ -335,6 +381,7 @@ class Impl final : public Base {
         }
         k_sgs_div<T, N><<<kSgsParts, 256, 0, s_>>>(TAU_, U_, F_, sgs_part_);
         k_sgs_flag<><<<1, 32, 0, s_>>>(sgs_part_, kSgsParts, sd_, les_->status_word());
+      }
     }
     static constexpr int kSgsParts = 512;
 
@@ -497,7 +544,8 @@ class Impl final : public Base {
             return NS3D_ERR_UNSUPPORTED;
         }
         const char* kNames[6] = {"k_xinv", "k_ypass_inv",
-                                 zform_ == 0 ? "k_zline" : zform_ == 2 ? "k_zgemm" : "k_zpass", "k_ypass_fwd",
+                                 zform_ == 0 ? "k_zline" : zform_ == 2 ? "k_zgemm" : "k_zpass",
+                                 "k_ypass_fwd",
                                  "k_xfwd", "k_misc"};
         std::vector<cudaEvent_t> ev(2 * 6 * 4 + 2);
         for (auto& e : ev) NS3D_CK(cudaEventCreate(&e));
@@ -1097,6 +1145,7 @@ class Impl final : public Base {
     int zg_ctas_ = 0;
     CUtensorMap xmap_[2];          // P1 tensor-tile form: U and UT as [3 M][N kx][N ky][2 NZP] FP32
     CUtensorMap wmap_;             // and W as [6 M][N x][N ky][2 NZP] FP32 (its outputs)
+    double* aux_ = nullptr;        // FP64 x passes: 1/k2 and the x wavenumbers
     int xt_ctas_ = 1;
     int* xt_items_ = nullptr;      // P1 tensor-tile form: compact list of the x tiles inside the circle
     int xt_nvalid_ = 0;

@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "fft_engine.cuh"
+#include "fxfft.cuh"
 #include "stats.cuh"
 #include "tma.cuh"
 
@@ -126,10 +127,14 @@ template <typename T, int N, int V = 0, bool INV = true> constexpr int tile_a() 
     return sizeof(T) == 4 ? clip_tile<YPlan<T, N, INV>::A::P, (INV ? TileVar<V>::A : TileVar<V>::AF)>()
                           : (YPlan<T, N, INV>::A::P * 8 <= 512 ? 8 : 4);
 }
+// FP64 x passes (fx_passes.cuh), on the z lines' plan: pencils per CTA. Inverse (one
+// field per CTA): 8, or 4 where that makes more than 256 threads. Forward (three groups
+// of threads): 8 up to 384 threads (256^3: 0.212 ms per launch, 0.250 with 4 pencils and
+// two CTAs per SM), else 4.
+template <int N, bool FWD = false> constexpr int fx_tile() { return Plans<N>::A::P * 8 <= (FWD ? 128 : 256) ? 8 : 4; }
 template <typename T, int N, int V = 0, bool FWD = false> constexpr int tile_x() {
-    constexpr int P = PlansV<N, V>::X::P;
-    return sizeof(T) == 4 ? clip_tile<P, (FWD ? TileVar<V>::XF : TileVar<V>::X)>()
-                          : (P * 8 <= 256 ? 8 : (P * 4 <= 512 ? 4 : 2));
+    if constexpr (sizeof(T) == 8) return fx_tile<N, FWD>();
+    else return clip_tile<PlansV<N, V>::X::P, (FWD ? TileVar<V>::XF : TileVar<V>::X)>();
 }
 // line pairs per CTA of the z pass (>= 96 threads)
 template <int N> constexpr int zpairs() {
@@ -292,8 +297,8 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         load(0, X);
         load(1, Y);
         ikx(Y, B);
-        PL::inv(B, sbuf, p, tw, sidx, sync);
-        PL::inv(X, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
         store(0, X);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = B[s] - mul_i(X[s]) * fky;
@@ -303,14 +308,14 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
             staged(2, Z);
             ikx(Z, B);
         }
-        PL::inv(B, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fkz - B[s];
         store(4, B);
-        PL::inv(Y, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(Y, sbuf, p, tw, sidx, sync);
         store(1, Y);
         staged(2, X);   // uz
-        PL::inv(X, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
         store(2, X);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fky - mul_i(Y[s]) * fkz;
@@ -324,20 +329,20 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         load(1, Y);
         load(2, Z);
         ikx(Y, B);
-        PL::inv(B, sbuf, p, tw, sidx, sync);
-        PL::inv(X, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
         store(0, X);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = B[s] - mul_i(X[s]) * fky;
         store(5, B);
         ikx(Z, B);
-        PL::inv(B, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fkz - B[s];
         store(4, B);
-        PL::inv(Y, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(Y, sbuf, p, tw, sidx, sync);
         store(1, Y);
-        PL::inv(Z, sbuf, p, tw, sidx, sync);
+        line_fft<PL, true, false, TT, NT>(Z, sbuf, p, tw, sidx, sync);
         store(2, Z);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(Z[s]) * fky - mul_i(Y[s]) * fkz;
@@ -347,7 +352,7 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
     cx<T> X[E], B[E];
     // ux
     load(0, X);
-    PL::inv(X, sbuf, p, tw, sidx, sync);
+    line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
     store(0, X);
     // wz = T(i kx uy) - i ky T(ux)
     {
@@ -355,7 +360,7 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         staged(1, Y);
         ikx(Y, B);
     }
-    PL::inv(B, sbuf, p, tw, sidx, sync);
+    line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
     for (int s = 0; s < E; ++s) B[s] = B[s] - mul_i(X[s]) * fky;
     store(5, B);
@@ -365,16 +370,16 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         staged(2, Z);
         ikx(Z, B);
     }
-    PL::inv(B, sbuf, p, tw, sidx, sync);
+    line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
     for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fkz - B[s];
     store(4, B);
     // uy, uz, then wx = i ky T(uz) - i kz T(uy)
     staged(1, X);
-    PL::inv(X, sbuf, p, tw, sidx, sync);
+    line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
     store(1, X);
     staged(2, B);
-    PL::inv(B, sbuf, p, tw, sidx, sync);
+    line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
     store(2, B);
 #pragma unroll
     for (int s = 0; s < E; ++s) B[s] = mul_i(B[s]) * fky - mul_i(X[s]) * fkz;
@@ -628,10 +633,11 @@ k_xinv_tma(const __grid_constant__ CUtensorMap map, int c0, const __grid_constan
 // Forward: inputs every y, outputs only where ky^2 + kz^2 <= KC^2.
 // ---------------------------------------------------------------------------
 // CTAs per SM the y pass is compiled for: 1024 threads per SM (64 registers per
-// thread), 512 (128 registers) for plans of more than 16 elements per thread
+// thread), 512 (128 registers) for plans of more than 16 elements per thread and
+// for FP64 (its 64-bit integer elements take twice the registers)
 template <typename T, int N, int V, bool INV> constexpr int ypass_minb() {
     constexpr int nt = tile_a<T, N, V, INV>() * YPlan<T, N, INV>::A::P;
-    constexpr int per_sm = YPlan<T, N, INV>::A::E > 16 ? 512 : 1024;
+    constexpr int per_sm = YPlan<T, N, INV>::A::E > 16 || sizeof(T) == 8 ? 512 : 1024;
     return per_sm / nt > 0 ? per_sm / nt : 1;
 }
 template <typename T, int N, bool INV, int V = 0>
@@ -662,8 +668,7 @@ k_ypass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw) {
         if (INV) in = in && (ky * ky <= rem);
         v[s] = in ? base[(long long)jj * G::NZP] : czero<T>();
     }
-    if (INV) PL::template inv<true>(v, sbuf, p, tw, sidx, sync);
-    else PL::template fwd<true>(v, sbuf, p, tw, sidx, sync);
+    line_fft<PL, INV, true, TT, TT * P>(v, sbuf, p, tw, sidx, sync);
     if (colok) {
 #pragma unroll
         for (int s = 0; s < E; ++s) {
@@ -742,7 +747,7 @@ k_zpass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, T* __restrict__ rea
                 }
                 v[s] = z;
             }
-            PL::inv(v, sb, p, tw, sidx, sync);
+            line_fft<PL, true, false, 1, 3 * P * ZP>(v, sb, p, tw, sidx, sync);
             T* ra = Rl + (L * 6 + 2 * g) * N;
             T* rb = ra + N;
 #pragma unroll
@@ -809,7 +814,7 @@ k_zpass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, T* __restrict__ rea
         cx<T> v[E];
 #pragma unroll
         for (int s = 0; s < E; ++s) v[s] = mk(ra[p + P * s], rb[p + P * s]);
-        PL::fwd(v, sb, p, tw, sidx, sync);
+        line_fft<PL, false, false, 1, 3 * P * ZP>(v, sb, p, tw, sidx, sync);
 #pragma unroll
         for (int s = 0; s < E; ++s) sb[sidx(p + P * s)] = v[s];
         __syncthreads();
@@ -1250,6 +1255,32 @@ __device__ __forceinline__ void xfwd_rk4_epilogue(cx<T> (&F)[3][E], int p, int k
       }
     }
 }
+// DP5CN: a block's three error sums in a fixed order: warp shuffles, then the warps'
+// sums in order; blocks with a partly filled warp add their threads in order
+template <int NT>
+__device__ __forceinline__ void dp_block_sum(const double (&es)[3], double* __restrict__ dpart) {
+    constexpr bool full = NT % 32 == 0;
+    __shared__ double red[full ? NT / 32 : NT][3];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double v = es[c];
+        if (full) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) red[wid][c] = v;
+        } else {
+            red[threadIdx.x][c] = v;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        constexpr int n = full ? NT / 32 : NT;
+        double v = 0.0;
+        for (int w = 0; w < n; ++w) v += red[w][threadIdx.x];
+        dpart[threadIdx.x] = v;
+    }
+}
 // ---------------------------------------------------------------------------
 // P5: forward FFT along x of the 3 product fields, then per mode the Leray
 // projection, dealias mask and RK stage update. grid (ntile, NKY).
@@ -1308,7 +1339,7 @@ k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ U
     }
     xfwd_prefetch_state<T, N, INTEG, MODE, E, P, TT>(U, ACC, K, rs, p, t, ky, kz0, j);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) PL::fwd(F[c], sbuf, p, tw, sidx, sync);
+    for (int c = 0; c < 3; ++c) line_fft<PL, false, false, TT, TT * P>(F[c], sbuf, p, tw, sidx, sync);
     if (INTEG != INT_TAB && !colok) return;
 
     T h = T(0);
@@ -1524,32 +1555,7 @@ k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ U
         }
     }
     if constexpr (INTEG == INT_TAB) {
-        if (rs.kind == 2) {
-            // fixed-order block reduction: warp shuffles (full warps; the
-            // block size is a power of two), then the warps' sums in order;
-            // blocks of fewer than 32 threads add their threads in order
-            __shared__ double red[32][3];
-            const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-            const bool full = blockDim.x >= 32;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                double v = es[c];
-                if (full) {
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-                    if (lane == 0) red[wid][c] = v;
-                } else {
-                    red[threadIdx.x][c] = v;
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x < 3) {
-                const int n = full ? (int)(blockDim.x >> 5) : (int)blockDim.x;
-                double v = 0.0;
-                for (int w = 0; w < n; ++w) v += red[w][threadIdx.x];
-                dpart[threadIdx.x] = v;
-            }
-        }
+        if (rs.kind == 2) dp_block_sum<TT * P>(es, dpart);
     }
 }
 
