@@ -226,13 +226,20 @@ __device__ __forceinline__ void fx_warp_bound(FxBound& b, unsigned mask) {
 // A line transform of the passes, v: the thread's E elements (see fft_stages).
 // STRIDED passes: the block's NT threads hold TT lines, thread = p TT + t. Line
 // passes (TT = 1): P consecutive threads hold a line. `tw` is the engine's table.
-// FP32 lines run in floating point. The FP64 result is scaled by 2^-kadd.
+// FP32 lines run in floating point. The FP64 result is scaled by 2^-kadd; its slots
+// outside the kept band are taken as zero in an inverse transform and left as they
+// were by a forward one.
 // ---------------------------------------------------------------------------
 template <class PL, bool INV, bool PK, int TT, int NT, typename SIdx, typename Sync, int E>
 __device__ __forceinline__ void line_fft(cx<float> (&v)[E], cx<float>* sbuf, int p, const cx<float>* __restrict__ tw,
                                          SIdx sidx, Sync sync) {
     if constexpr (INV) PL::template inv<PK>(v, sbuf, p, tw, sidx, sync);
     else PL::template fwd<PK>(v, sbuf, p, tw, sidx, sync);
+}
+// slot s of every thread lies outside the kept band |k| <= KC = N / 3: a quarter of the
+// slots of 16, neither converted nor added (256^3 y passes 0.272 + 0.142 -> 0.255 + 0.132 ms)
+template <class PL> constexpr bool fx_outside(int s) {
+    return PL::P * s > PL::N / 3 && PL::P * s + PL::P - 1 < PL::N - PL::N / 3;
 }
 template <class PL, bool INV, bool PK, int TT, int NT, typename SIdx, typename Sync, int E>
 __device__ __forceinline__ void line_fft(cx<double> (&v)[E], cx<double>* sbuf, int p,
@@ -262,6 +269,8 @@ __device__ __forceinline__ void line_fft(cx<double> (&v)[E], cx<double>* sbuf, i
     cx<q64> a[E];
 #pragma unroll
     for (int s = 0; s < E; ++s) {
+        a[s] = mk<q64>(0, 0);
+        if (INV && fx_outside<PL>(s)) continue;
         // the inverse transform is the forward one with real and imaginary parts exchanged
         const q64 x = fx_from(v[s].x, sc.k), y = fx_from(v[s].y, sc.k);
         a[s] = INV ? mk<q64>(y, x) : mk<q64>(x, y);
@@ -271,6 +280,7 @@ __device__ __forceinline__ void line_fft(cx<double> (&v)[E], cx<double>* sbuf, i
     const int k = (sc.k == -4096 ? 0 : sc.k) + kadd;
 #pragma unroll
     for (int s = 0; s < E; ++s) {
+        if (!INV && fx_outside<PL>(s)) continue;
         const double x = fx_to(a[s].x, k), y = fx_to(a[s].y, k);
         v[s] = INV ? mk(y, x) : mk(x, y);
     }

@@ -665,7 +665,7 @@ k_ypass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw) {
         const int jj = p + P * s;
         const int ky = kof<N>(jj);
         bool in = colok;
-        if (INV) in = in && (ky * ky <= rem);
+        if (INV) in = in && (ky * ky <= rem) && !(P * s > G::KC && P * s + P - 1 < N - G::KC);
         v[s] = in ? base[(long long)jj * G::NZP] : czero<T>();
     }
     line_fft<PL, INV, true, TT, TT * P>(v, sbuf, p, tw, sidx, sync);
@@ -674,6 +674,7 @@ k_ypass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw) {
         for (int s = 0; s < E; ++s) {
             const int jj = p + P * s;
             const int ky = kof<N>(jj);
+            if (!INV && P * s > G::KC && P * s + P - 1 < N - G::KC) continue;   // |ky| > KC in every thread
             if (INV || ky * ky <= rem) base[(long long)jj * G::NZP] = v[s];
         }
     }
