@@ -29,6 +29,9 @@ template <int N>
 __global__ void __launch_bounds__(fxinv_threads<N>(), fx_ctas(512, fxinv_threads<N>()))
 k_xinv_fx(const cx<double>* __restrict__ U, cx<double>* __restrict__ W, const cx<double>* __restrict__ tw,
           const double* __restrict__ aux) {
+    const long long dep = pdl_begin();
+    U += dep;
+    W += dep;
     using G = Geo<N>;
     using PL = typename Plans<N>::A;
     constexpr int TT = fx_tile<N>(), E = PL::E, P = PL::P, NT = TT * P;
@@ -101,6 +104,15 @@ k_xfwd_fx(const cx<double>* __restrict__ W, cx<double>* __restrict__ U, cx<doubl
           cx<double>* __restrict__ ACC, const cx<double>* __restrict__ tw, const StepDev* __restrict__ sd,
           const cx<double>* __restrict__ tab, const double* __restrict__ aux, cx<double>* __restrict__ K,
           double* __restrict__ dpart, const RkStage rs) {
+    const long long dep = pdl_begin();
+    W += dep;
+    U += dep;
+    UT += dep;
+    ACC += dep;
+    sd += dep;
+    tab += dep;
+    K += dep;
+    dpart += dep;
     using G = Geo<N>;
     using PL = typename Plans<N>::A;
     using C = cx<double>;
@@ -288,6 +300,9 @@ __device__ __forceinline__ q64 fx_cross(FxSplit a, int a4, FxSplit b, FxSplit c,
 template <int N>
 __global__ void __launch_bounds__(zfx_threads<N>(), zfx_minb<N>())
 k_zfx(cx<double>* __restrict__ W, const cx<double>* __restrict__ tw, StepDev* __restrict__ sd, int want_umax) {
+    const long long dep = pdl_begin();
+    W += dep;
+    sd += dep;
     using G = Geo<N>;
     using PL = typename Plans<N>::A;
     constexpr int E = PL::E, P = PL::P, ZP = zfx_pairs<N>(), XS = zpad<N>();

@@ -226,6 +226,9 @@ constexpr size_t xinv_smem() {
 template <typename T, int N, int V = 0>
 __global__ void __launch_bounds__(tile_x<T, N, V>() * PlansV<N, V>::X::P, TileVar<V>::MINB_XI)
 k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restrict__ tw) {
+    const long long dep = pdl_begin();
+    U += dep;
+    W += dep;
     using G = Geo<N>;
     using PL = typename PlansV<N, V>::X;
     constexpr int TT = tile_x<T, N, V>();
@@ -448,6 +451,7 @@ template <typename T, int N, int V>
 __global__ void __launch_bounds__(xtma_tile<T, N, V>() * PlansV<N, V>::X::P, xtma_minb<T, N, V>())
 k_xinv_tma(const __grid_constant__ CUtensorMap map, int c0, const __grid_constant__ CUtensorMap wmap, int cw,
            const cx<T>* __restrict__ tw, StepDev* __restrict__ sd, const int* __restrict__ xitems, int nvalid, int cnt) {
+    sd += pdl_begin();
     using G = Geo<N>;
     using PL = typename PlansV<N, V>::X;
     constexpr int TT = xtma_tile<T, N, V>();
@@ -643,6 +647,7 @@ template <typename T, int N, int V, bool INV> constexpr int ypass_minb() {
 template <typename T, int N, bool INV, int V = 0>
 __global__ void __launch_bounds__(tile_a<T, N, V, INV>() * YPlan<T, N, INV>::A::P, ypass_minb<T, N, V, INV>())
 k_ypass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw) {
+    W += pdl_begin();
     using G = Geo<N>;
     using PL = typename YPlan<T, N, INV>::A;
     constexpr int TT = tile_a<T, N, V, INV>();
@@ -706,6 +711,9 @@ template <typename T, int N, int MODE>
 __global__ void __launch_bounds__(3 * Plans<N>::A::P * zpairs<N>())
 k_zpass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, T* __restrict__ real,
         StepDev* __restrict__ sd, int want_umax) {
+    const long long dep = pdl_begin();
+    W += dep;
+    real += dep;
     using G = Geo<N>;
     using PL = typename Plans<N>::A;
     constexpr int E = PL::E, P = PL::P, ZP = zpairs<N>();
@@ -917,6 +925,9 @@ template <typename T, int N>
 __global__ void __launch_bounds__(ZLINE_WARPS * 32, zline_xbuf_in_stage<N>() ? 3 : 2)
 k_zline(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, StepDev* __restrict__ sd, int want_umax,
         int nmem) {
+    const long long dep = pdl_begin();
+    W += dep;
+    sd += dep;
     using G = Geo<N>;
     using PL = typename ZPlan<N>::A;
     constexpr int E = PL::E, P = PL::P, GPW = zline_gpw<N>(), GW = zline_gw<N>(), GT = 32 * GW;
@@ -1296,6 +1307,16 @@ k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ U
        cx<T>* __restrict__ ACC, const cx<T>* __restrict__ tw, const StepDev* __restrict__ sd,
        const cx<T>* __restrict__ tab, const cx<T>* __restrict__ sgs, cx<T>* __restrict__ K,
        double* __restrict__ dpart, const RkStage rs) {
+    const long long dep = pdl_begin();
+    W += dep;
+    U += dep;
+    UT += dep;
+    ACC += dep;
+    sd += dep;
+    tab += dep;
+    sgs += dep;
+    K += dep;
+    dpart += dep;
     using G = Geo<N>;
     using PL = typename PlansV<N, V>::X;
     constexpr int TT = tile_x<T, N, V, true>();
@@ -1567,6 +1588,9 @@ k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ U
 // ---------------------------------------------------------------------------
 template <typename T, int N>
 __global__ void k_tables(cx<T>* __restrict__ tab, StepDev* __restrict__ sd, int integ, int vp, int use_cfl) {
+    const long long dep = pdl_begin();
+    tab += dep;
+    sd += dep;
     using G = Geo<N>;
     sd += blockIdx.y;   // ensemble member
     tab += (long long)blockIdx.y * (G::KC2 + 1);
@@ -1605,6 +1629,9 @@ __global__ void k_tables(cx<T>* __restrict__ tab, StepDev* __restrict__ sd, int 
 // ---------------------------------------------------------------------------
 template <typename T, int N>
 __global__ void k_step_end(cx<T>* __restrict__ U, StepDev* __restrict__ sd, int force_k, int use_cfl, int dp) {
+    const long long dep = pdl_begin();
+    U += dep;
+    sd += dep;
     using G = Geo<N>;
     U += (long long)blockIdx.x * 3 * G::FS;   // one CTA per ensemble member
     sd += blockIdx.x;
@@ -1679,6 +1706,9 @@ __global__ void k_step_end(cx<T>* __restrict__ U, StepDev* __restrict__ sd, int 
 // ---------------------------------------------------------------------------
 template <typename T, int N>
 __global__ void k_dp_ctl(const double* __restrict__ dpart, int nparts, StepDev* __restrict__ sd) {
+    const long long dep = pdl_begin();
+    dpart += dep;
+    sd += dep;
     __shared__ double red[3][256];
     sd += blockIdx.x;
     dpart += (long long)blockIdx.x * nparts * 3;
@@ -1726,6 +1756,10 @@ __global__ void k_dp_ctl(const double* __restrict__ dpart, int nparts, StepDev* 
 // only the dealiased sphere is copied. grid (x, members)
 template <typename T, int N>
 __global__ void k_dp_commit(cx<T>* __restrict__ U, const cx<T>* __restrict__ ACC, const StepDev* __restrict__ sd) {
+    const long long dep = pdl_begin();
+    U += dep;
+    ACC += dep;
+    sd += dep;
     using G = Geo<N>;
     const long long mem = blockIdx.y;
     if (!sd[mem].dp_accept) return;
