@@ -130,6 +130,7 @@ __device__ __forceinline__ void bfly(cx<T> e, cx<T> o, cx<T>& lo, cx<T>& hi) {
         hi = e - t;
     } else {
         constexpr bool tri = (R % 3 == 0);
+        static_assert(tri ? k * 12 % R == 0 : k * 16 % R == 0, "no constant for this angle");
         constexpr int idx = tri ? (k * 12 / R) : (k * 16 / R);
         constexpr double cd = tri ? kC12[idx] : kC16[idx];
         constexpr double sd = tri ? kS12[idx] : kS16[idx];

@@ -111,6 +111,7 @@ __device__ __forceinline__ void bfly(cx<q64> e, cx<q64> o, cx<q64>& lo, cx<q64>&
     } else {
         constexpr bool tri = (R % 3 == 0);
         constexpr int n = tri ? 12 : 16, idx = k * n / R;
+        static_assert(k * n % R == 0, "no constant for this angle");
         constexpr q64 c = tri ? kQC12[idx % 12] : kQC16[idx % 16];
         constexpr q64 s = tri ? kQC12[(idx + 9) % 12] : kQC16[(idx + 12) % 16];   // sin x = cos(x - 90 degrees)
         t = fx_cmul(o, fx_hi(c), fx_lo(c), fx_hi(-s), fx_lo(-s));                  // W = c - i s

@@ -112,6 +112,9 @@ template <> struct TileVar<6> { static constexpr int A = 16, AF = 16, X = 8, XF 
 // with it (0.058 -> 0.060 ms). The z lines hold three fields per line and keep 12.
 template <typename T, int N, bool INV> struct YPlan { using A = typename Plans<N>::A; };
 template <> struct YPlan<float, 96, true> { using A = Plan<96, 24, 12, 8>; };
+// 384 points in FP32: 24 elements and one stage less in both directions (inverse 0.308 ->
+// 0.286, forward 0.143 -> 0.129 ms; even at 192)
+template <bool INV> struct YPlan<float, 384, INV> { using A = Plan<384, 24, 8, 8, 6>; };
 template <int N> struct AltX { using X = typename Plans<N>::X; };
 template <> struct AltX<64> { using X = Plan<64, 16, 16, 4>; };
 template <> struct AltX<128> { using X = Plan<128, 16, 16, 8>; };
@@ -877,7 +880,11 @@ constexpr int ZLINE_WARPS = 4;
 // the line kernel's plan: the y-pass plan (at 512^3 two warps per line with 8
 // elements per lane, 128 registers and twice the warps per SM, measured 8 %
 // slower than one warp with 16 elements)
+// 384 points: 24 elements per lane, which saves a stage and its exchange, at two CTAs per
+// SM (0.716 -> 0.588 ms per launch; the radices in other orders 0.71 - 0.92 ms). Not at 192
+// (8 x 8 x 3: 0.083 -> 0.095 ms) or 96 points (eight members, 8 x 12: 0.091 -> 0.141 ms).
 template <int N> struct ZPlan { using A = typename Plans<N>::A; };
+template <> struct ZPlan<384> { using A = Plan<384, 24, 8, 8, 6>; };
 template <int N> constexpr int zline_gw() { return ZPlan<N>::A::P > 32 ? ZPlan<N>::A::P / 32 : 1; }
 template <int N> constexpr int zline_gpw() { return ZPlan<N>::A::P <= 32 ? 32 / ZPlan<N>::A::P : 1; }
 // the real Nz line as a half-length complex transform (a plan of N/2 points on the
@@ -896,7 +903,7 @@ template <int N> constexpr bool zline_half_nz() {
 template <typename T, int N>
 constexpr bool zline_ok() {
     constexpr int P = ZPlan<N>::A::P;
-    return sizeof(T) == 4 && ZPlan<N>::A::E <= 16 &&
+    return sizeof(T) == 4 && ZPlan<N>::A::E <= 24 &&
            (P <= 32 ? (32 % P == 0 && ((long long)N * N) % (32 / P) == 0) : P == 64);
 }
 // With several lines per warp (N <= 256) the exchange buffers live in the
@@ -904,6 +911,7 @@ constexpr bool zline_ok() {
 // per warp by a fifth (3 CTAs per SM instead of 2 at 168 registers); 512- and
 // 1024-point lines (16 elements per lane, over 200 registers) keep their own.
 template <int N> constexpr bool zline_xbuf_in_stage() { return zline_gpw<N>() > 1; }
+template <int N> constexpr int zline_minb() { return zline_xbuf_in_stage<N>() && ZPlan<N>::A::E <= 16 ? 3 : 2; }
 template <int N> constexpr int zline_stage_elems() {
     constexpr int a = zline_gpw<N>() * 6 * Geo<N>::NZP, b = zline_gpw<N>() * zpad<N>();
     return ((zline_xbuf_in_stage<N>() && b > a ? b : a) + 15) / 16 * 16;
@@ -922,7 +930,7 @@ template <typename T, int N> constexpr size_t zline_smem() {
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(ZLINE_WARPS * 32, zline_xbuf_in_stage<N>() ? 3 : 2)
+__global__ void __launch_bounds__(ZLINE_WARPS * 32, zline_minb<N>())
 k_zline(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, StepDev* __restrict__ sd, int want_umax,
         int nmem) {
     const long long dep = pdl_begin();
