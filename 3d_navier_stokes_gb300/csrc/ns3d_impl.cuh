@@ -903,19 +903,24 @@ class Impl final : public Base {
     // ------------------------------------------------------- real space
     ns3d_status real_space_host(double* u, double* w) override {
         ns3d_status st = ensure_real();
+        if (st == NS3D_OK) st = ensure_stage();
         if (st != NS3D_OK) return st;
-        double* du = nullptr;
-        size_t rb = sizeof(double) * 3 * (size_t)N * N * (N + 2);
-        NS3D_CK(cudaMalloc(&du, 2 * rb));
         p1(U_, m_, 1); p2(m_, 1);
         pass(k_zpass<T, N, 1>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
             Wm(m_), tw_, real_, nullptr, 0);
-        k_real_unpack<T, N><<<grid_for((long long)N * N * (N + 2)), 256, 0, s_>>>(real_, du, du + rb / sizeof(double));
+        // a reference real array has the bytes of a Fourier one: both pass through the staging buffer
+        const size_t rb = sizeof(double) * 3 * (size_t)N * N * (N + 2);
+        static_assert(24LL * N * N * (N + 2) == kRefBytes, "");
+        double* d = reinterpret_cast<double*>(stage_);
         cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess && u) e = cudaMemcpyAsync(u, du, rb, cudaMemcpyDeviceToHost, s_);
-        if (e == cudaSuccess && w) e = cudaMemcpyAsync(w, du + rb / sizeof(double), rb, cudaMemcpyDeviceToHost, s_);
+        for (int c = 0; c < 2; ++c) {
+            double* dst = c ? w : u;
+            if (!dst || e != cudaSuccess) continue;
+            k_real_unpack<T, N><<<grid_for((long long)N * N * (N + 2)), 256, 0, s_>>>(real_, c ? nullptr : d, c ? d : nullptr);
+            e = cudaGetLastError();
+            if (e == cudaSuccess) e = cudaMemcpyAsync(dst, d, rb, cudaMemcpyDeviceToHost, s_);
+        }
         if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
-        cudaFree(du);
         if (e != cudaSuccess) {
             set_err("real_space: %s", cudaGetErrorString(e));
             return NS3D_ERR_CUDA;
