@@ -1,10 +1,25 @@
-// fx_passes.cuh — the x and z passes of the FP64 engines, on the 64-bit integer
-// line transforms of fxfft.cuh (the y passes are k_ypass with line_fft). Layouts and
-// launch grids are those of the FP32 passes in ns3d_kernels.cuh.
+// fx_passes.cuh — the passes of the FP64 engines, on the 64-bit integer line transforms
+// of fxfft.cuh. Layouts and launch grids are those of the FP32 passes in
+// ns3d_kernels.cuh; the work array W holds integers.
 #pragma once
 #include "ns3d_kernels.cuh"
 
 namespace ns3d {
+
+// Scales of the lines of W after each pass, member after member (fx_scales_ints ints each):
+// one per line of the pass that wrote it.
+struct FxScales {
+    int* x;   // after P1: [6 fields][N ky][NZP]
+    int* y;   // after P2: [6][N x][NZP]
+    int* z;   // after P3: [3][N x][N y]
+    int* w;   // after P4: [3][N x][NZP]
+};
+template <int N> constexpr long long fx_scales_ints() { return 15LL * N * Geo<N>::NZP + 3LL * N * N; }
+template <int N> __device__ __forceinline__ FxScales fx_scales(int* base, long long member) {
+    int* b = base + member * fx_scales_ints<N>();
+    constexpr long long c = (long long)N * Geo<N>::NZP;
+    return FxScales{b, b + 6 * c, b + 15 * c, b + 12 * c};
+}
 
 // ---------------------------------------------------------------------------
 // x passes: the z lines' plan (16 elements per thread where N allows, one or two
@@ -16,6 +31,13 @@ template <int N> constexpr int fxinv_threads() { return fx_tile<N>() * Plans<N>:
 template <int N> constexpr int fxfwd_threads() { return 3 * fx_tile<N, true>() * Plans<N>::A::P; }
 constexpr int fx_log2(int n) { return n <= 1 ? 0 : 1 + fx_log2(n / 2); }
 constexpr int fx_ctas(int per_sm, int threads) { return per_sm / threads < 1 ? 1 : per_sm / threads; }
+// CTAs per SM the passes are compiled for. Inverse: 640 threads (96 registers) from 16
+// threads per line, 512 below (256^3 0.164 -> 0.160 ms, 128^3 0.0253 against 0.0258).
+// Forward: two CTAs of 384 threads or one of 768 (80 registers, a few spills, but one
+// CTA's transforms under the other's FP64 work: 256^3 0.208 -> 0.166 ms, 512^3 1.96 ->
+// 1.51 ms), 576 threads with smaller CTAs (128^3 0.0395 -> 0.0343 ms, 0.0411 with 768).
+template <int N> constexpr int fxinv_ctas() { return fx_ctas(Plans<N>::A::P >= 16 ? 640 : 512, fxinv_threads<N>()); }
+template <int N> constexpr int fxfwd_ctas() { return fx_ctas(fxfwd_threads<N>() >= 384 ? 768 : 576, fxfwd_threads<N>()); }
 template <int N> constexpr int fxinv_smem() { return N * fx_tile<N>() * 16; }
 template <int N> constexpr int fxfwd_smem() { return 3 * N * fx_tile<N, true>() * 16; }
 
@@ -26,18 +48,19 @@ template <int N> constexpr int fxfwd_smem() { return 3 * N * fx_tile<N, true>() 
 // the six transforms in one CTA; 256^3: 0.19 against 0.25 ms). The inputs' second and
 // third reads hit L2.
 template <int N>
-__global__ void __launch_bounds__(fxinv_threads<N>(), fx_ctas(512, fxinv_threads<N>()))
-k_xinv_fx(const cx<double>* __restrict__ U, cx<double>* __restrict__ W, const cx<double>* __restrict__ tw,
-          const double* __restrict__ aux) {
+__global__ void __launch_bounds__(fxinv_threads<N>(), fxinv_ctas<N>())
+k_xinv_fx(const cx<double>* __restrict__ U, cx<q64>* __restrict__ W, int* __restrict__ scales,
+          const int4* __restrict__ tw, const double* __restrict__ aux) {
     const long long dep = pdl_begin();
     U += dep;
     W += dep;
+    scales += dep;
     using G = Geo<N>;
     using PL = typename Plans<N>::A;
     constexpr int TT = fx_tile<N>(), E = PL::E, P = PL::P, NT = TT * P;
     constexpr bool kPow2 = (N & (N - 1)) == 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<double>* sbuf = reinterpret_cast<cx<double>*>(smem_raw);
+    cx<q64>* sbuf = reinterpret_cast<cx<q64>*>(smem_raw);
     const int t = threadIdx.x % TT, p = threadIdx.x / TT;
     const int kz0 = blockIdx.x * TT, kz = kz0 + t;
     const int ky = (int)blockIdx.y - G::KC;
@@ -84,12 +107,82 @@ k_xinv_fx(const cx<double>* __restrict__ U, cx<double>* __restrict__ W, const cx
         for (int s = 0; s < E; ++s)
             if (!(P * s > G::KC && P * s + P - 1 < N - G::KC)) v[s] = v[s] * (1.0 / ((double)N * N * N));
     }
-    // 1/N^3 of a power of two goes into the exponent
-    line_fft<PL, true, false, TT, NT>(v, sbuf, p, tw, sidx, sync, kPow2 ? 3 * fx_log2(N) : 0);
+    const int k = fx_scale(fx_line_bound<P, TT, NT>(fx_bound(v), sync), 0, kFxFlush);
+    cx<q64> a[E];
+#pragma unroll
+    for (int s = 0; s < E; ++s)
+        // an inverse transform is the forward one with real and imaginary parts exchanged
+        a[s] = fx_outside<PL>(s) ? mk<q64>(0, 0) : mk<q64>(fx_from(v[s].y, k), fx_from(v[s].x, k));
+    PL::template fwd<false>(a, sbuf, p, tw, sidx, sync);
     if (rem >= 0) {
 #pragma unroll
-        for (int s = 0; s < E; ++s) W[off + (long long)(p + P * s) * xs] = v[s];
+        for (int s = 0; s < E; ++s) W[off + (long long)(p + P * s) * xs] = mk<q64>(a[s].y, a[s].x);
+        // 1/N^3 of a power of two goes into the scale
+        if (p == 0)
+            fx_scales<N>(scales, blockIdx.z / 6).x[((long long)f * N + j) * G::NZP + kz] =
+                k + (kPow2 && k != kFxZero && k != kFxBad ? 3 * fx_log2(N) : 0);
     }
+}
+
+// P2 / P4: FFT along y in place, grid and masks of k_ypass; the elements of a line come
+// with scales of their own (per ky after P1, per y after P3).
+template <int N> constexpr int fxy_tile() { return Plans<N>::A::P * 8 <= 512 ? 8 : 4; }
+template <int N> constexpr int fxy_threads() { return fxy_tile<N>() * Plans<N>::A::P; }
+// 512 threads per SM (128 registers); 640 with at most 12 elements per thread (192^3 0.118 ->
+// 0.114 ms; 256^3, 16 elements: 0.201 against 0.207 ms)
+template <int N> constexpr int fxy_ctas() { return fx_ctas(Plans<N>::A::E <= 12 ? 640 : 512, fxy_threads<N>()); }
+template <int N, bool INV>
+__global__ void __launch_bounds__(fxy_threads<N>(), fxy_ctas<N>())
+k_ypass_fx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict__ tw) {
+    const long long dep = pdl_begin();
+    W += dep;
+    scales += dep;
+    using G = Geo<N>;
+    using PL = typename Plans<N>::A;
+    constexpr int TT = fxy_tile<N>(), E = PL::E, P = PL::P, NT = TT * P;
+    constexpr int NF = INV ? 6 : 3;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cx<q64>* sbuf = reinterpret_cast<cx<q64>*>(smem_raw);
+    const int t = threadIdx.x % TT, p = threadIdx.x / TT;
+    const int kz = blockIdx.x * TT + t, i = blockIdx.y;
+    const bool colok = kz <= G::KC;
+    const int rem = G::KC2 - kz * kz;
+    const int mem = blockIdx.z / NF, f = blockIdx.z % NF;
+    cx<q64>* base = W + ((long long)mem * 6 + f) * G::FS + (long long)i * N * G::NZP + kz;
+    const FxScales sc = fx_scales<N>(scales, mem);
+    const int* kin = INV ? sc.x + (long long)f * N * G::NZP + kz : sc.z + ((long long)f * N + i) * N;
+    StridedIdx<TT, PL::R1> sidx{t};
+    SyncBlock sync;
+    cx<q64> a[E];
+    int ke[E];
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+        const int jj = p + P * s, ky = kof<N>(jj);
+        a[s] = mk<q64>(0, 0);
+        ke[s] = kFxZero;
+        if (INV && fx_outside<PL>(s)) continue;
+        if (colok && (!INV || ky * ky <= rem)) {
+            a[s] = base[(long long)jj * G::NZP];
+            ke[s] = kin[INV ? (long long)jj * G::NZP : jj];
+        }
+    }
+    const int k = fx_scale_of(fx_line_bound<P, TT, NT>(fx_bound(a, ke), sync), 0);
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+        if (INV && fx_outside<PL>(s)) continue;
+        const cx<q64> v = fx_align(a[s], ke[s], k);
+        a[s] = INV ? mk<q64>(v.y, v.x) : v;
+    }
+    PL::template fwd<false>(a, sbuf, p, tw, sidx, sync);
+    if (!colok) return;
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+        const int jj = p + P * s, ky = kof<N>(jj);
+        if (!INV && fx_outside<PL>(s)) continue;
+        if (INV) base[(long long)jj * G::NZP] = mk<q64>(a[s].y, a[s].x);
+        else if (ky * ky <= rem) base[(long long)jj * G::NZP] = a[s];
+    }
+    if (p == 0) (INV ? sc.y : sc.w)[((long long)f * N + i) * G::NZP + kz] = k;
 }
 
 // P5: three groups of threads transform one component each, leave the rows of the band in
@@ -99,13 +192,15 @@ k_xinv_fx(const cx<double>* __restrict__ U, cx<double>* __restrict__ W, const cx
 // formed once per thread. Three groups instead of one after the other: 24 -> 14 us per
 // launch at 32^3, 0.226 -> 0.212 ms at 256^3.
 template <int N, int INTEG, int MODE>
-__global__ void __launch_bounds__(fxfwd_threads<N>(), fx_ctas(384, fxfwd_threads<N>()))
-k_xfwd_fx(const cx<double>* __restrict__ W, cx<double>* __restrict__ U, cx<double>* __restrict__ UT,
-          cx<double>* __restrict__ ACC, const cx<double>* __restrict__ tw, const StepDev* __restrict__ sd,
+__global__ void __launch_bounds__(fxfwd_threads<N>(), fxfwd_ctas<N>())
+k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* __restrict__ U,
+          cx<double>* __restrict__ UT, cx<double>* __restrict__ ACC, const int4* __restrict__ tw,
+          const StepDev* __restrict__ sd,
           const cx<double>* __restrict__ tab, const double* __restrict__ aux, cx<double>* __restrict__ K,
           double* __restrict__ dpart, const RkStage rs) {
     const long long dep = pdl_begin();
     W += dep;
+    scales += dep;
     U += dep;
     UT += dep;
     ACC += dep;
@@ -146,22 +241,29 @@ k_xfwd_fx(const cx<double>* __restrict__ W, cx<double>* __restrict__ U, cx<doubl
     {
         const int kz = kz0 + t;
         const bool colok = kz <= G::KC && ky * ky + kz * kz <= G::KC2;
-        const C* src = W + g * G::FS + (long long)j * G::NZP + kz;
-        C v[E];
+        const cx<q64>* src = W + g * G::FS + (long long)j * G::NZP + kz;
+        const int* kin = fx_scales<N>(scales, blockIdx.z).w + (long long)g * N * G::NZP + kz;
+        cx<q64> a[E];
+        int ke[E];
 #pragma unroll
-        for (int s = 0; s < E; ++s) v[s] = colok ? src[(long long)(p + P * s) * xs] : czero<double>();
+        for (int s = 0; s < E; ++s) {
+            a[s] = colok ? src[(long long)(p + P * s) * xs] : mk<q64>(0, 0);
+            ke[s] = colok ? kin[(p + P * s) * G::NZP] : kFxZero;
+        }
         // the state rows of this tile into L2 (the groups share the rows)
         if (g == 0) xfwd_prefetch_state<double, N, INTEG, MODE, E, P, TT>(U, ACC, K, rs, p, t, ky, kz0, j);
         StridedIdx<TT, PL::R1> sidx{t};
-        if constexpr (NG % 32 == 0) {
-            const SyncGroup sync{1 + g, NG};
-            line_fft<PL, false, false, TT, NT>(v, sbuf, p, tw, sidx, sync);
-        } else {
-            line_fft<PL, false, false, TT, NT>(v, sbuf, p, tw, sidx, SyncBlock());
-        }
+        auto transform = [&](auto sync) {
+            const int k = fx_scale_of(fx_line_bound<P, TT, NT>(fx_bound(a, ke), sync), 0);
 #pragma unroll
-        for (int s = 0; s < E; ++s)
-            if (!(P * s > G::KC && P * s + P - 1 < N - G::KC)) sbuf[(p + P * s) * TT + t] = v[s];
+            for (int s = 0; s < E; ++s) a[s] = fx_align(a[s], ke[s], k);
+            PL::template fwd<false>(a, reinterpret_cast<cx<q64>*>(sbuf), p, tw, sidx, sync);
+#pragma unroll
+            for (int s = 0; s < E; ++s)
+                if (!fx_outside<PL>(s)) sbuf[(p + P * s) * TT + t] = fx_to_any(a[s], k);
+        };
+        if constexpr (NG % 32 == 0) transform(SyncGroup{1 + g, NG});
+        else transform(SyncBlock());
     }
     __syncthreads();
 
@@ -262,8 +364,8 @@ k_xfwd_fx(const cx<double>* __restrict__ W, cx<double>* __restrict__ U, cx<doubl
 }
 
 // ---------------------------------------------------------------------------
-// P3 for FP64 (fxfft.cuh): the whole line stays in 64-bit integers between the
-// load and the store. A CTA takes ZP pairs of adjacent lines; three groups of P
+// P3, MODE as in k_zpass (0: c2r, u x w, r2c; 1: c2r to real_out [6][N][N][N]; 2: r2c of
+// real_out [3][N][N][N]). A CTA takes ZP pairs of adjacent lines; three groups of P
 // threads own one complex transform each. Per line the velocity and the vorticity
 // get one scale each (2^60 bounds the L1 norm of every component), group g turns
 // fields 2g, 2g+1 into real space, the threads form u x w >> 60 from the 32-bit
@@ -297,11 +399,21 @@ __device__ __forceinline__ q64 fx_cross(FxSplit a, int a4, FxSplit b, FxSplit c,
     return madw(a4, b.ad, mid >> 29) - mulw(c4, d.ad);
 }
 
-template <int N>
+// scale of a product spectrum (twice itself) from the scales of u and w and the line's shift
+__device__ __forceinline__ int fx_product_scale(int2 k, int sh) {
+    if (k.x == kFxBad || k.y == kFxBad) return kFxBad;
+    if (k.x == kFxZero || k.y == kFxZero) return kFxZero;
+    return k.x + k.y - 60 - sh + 1;
+}
+
+template <int N, int MODE>
 __global__ void __launch_bounds__(zfx_threads<N>(), zfx_minb<N>())
-k_zfx(cx<double>* __restrict__ W, const cx<double>* __restrict__ tw, StepDev* __restrict__ sd, int want_umax) {
+k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict__ tw, double* __restrict__ real,
+      StepDev* __restrict__ sd, int want_umax) {
     const long long dep = pdl_begin();
     W += dep;
+    scales += dep;
+    real += dep;
     sd += dep;
     using G = Geo<N>;
     using PL = typename Plans<N>::A;
@@ -313,39 +425,43 @@ k_zfx(cx<double>* __restrict__ W, const cx<double>* __restrict__ tw, StepDev* __
     cx<q64>* buf = reinterpret_cast<cx<q64>*>(smem_raw);   // [ZP][2 lines][3 groups][XS]
     __shared__ FxBound bound[ZP][6][NW];                    // a line's L1 norm per field
     __shared__ uint2 count[ZP][3][NW];                      // a real line's sums (P > 32)
-    __shared__ int2 scale[ZP][2];                           // per line: ku, kw (bad lines: ku = kBad)
-    constexpr int kBad = 1 << 20;
+    __shared__ int2 scale[ZP][2];                           // per line: ku, kw
     const int p = threadIdx.x % P;
     const int g = (threadIdx.x / P) % 3;
     const int lp = threadIdx.x / (3 * P);
     const long long la = 2 * ((long long)blockIdx.x * ZP + lp);
-    const int4* twq = reinterpret_cast<const int4*>(tw);
+    const FxScales sc = fx_scales<N>(scales, blockIdx.y);
     PaddedIdx sidx;
     SyncLine<P> sync;
 
-    int shx = 0, shy = 0;
+    int kA = 0, kB = 0;   // scales of what a group writes
     // lines a and b to real space, then the products back: one copy of the transform's code
     // (instruction fetch is a cost of these long unrolled bodies)
 #pragma unroll 1
-    for (int L = 0; L < 3; ++L) {
+    for (int L = MODE == 2 ? 2 : 0; L < (MODE == 1 ? 2 : 3); ++L) {
         cx<q64>* sb;
         cx<q64> a[E];
         if (L < 2) {
             sb = buf + ((lp * 2 + L) * 3 + g) * XS;
-            const cx<double>* A = W + (long long)(2 * g) * G::FS + (la + L) * G::NZP;
-            const cx<double>* B = A + G::FS;
-            cx<double> ra[NLOW], rb[NLOW];
+            const cx<q64>* A = W + (long long)(2 * g) * G::FS + (la + L) * G::NZP;
+            const int* kin = sc.y + ((long long)2 * g * N + (la + L) / N) * G::NZP;
+            constexpr long long kf = (long long)N * G::NZP;   // to the next field's scales
+            cx<q64> ra[NLOW], rb[NLOW];
+            int kea[NLOW], keb[NLOW];
 #pragma unroll
             for (int s = 0; s < NLOW; ++s) {
                 const int m = p + P * s;
-                ra[s] = rb[s] = czero<double>();
+                ra[s] = rb[s] = mk<q64>(0, 0);
+                kea[s] = keb[s] = kFxZero;
                 if (m <= G::KC) {
                     ra[s] = A[m];
-                    rb[s] = B[m];
-                    if (m == 0) ra[s].y = rb[s].y = 0.0;   // c2r takes the real part of the mean
+                    rb[s] = A[G::FS + m];
+                    kea[s] = kin[m];
+                    keb[s] = kin[kf + m];
+                    if (m == 0) ra[s].y = rb[s].y = 0;   // c2r takes the real part of the mean
                 }
             }
-            FxBound ba = fx_bound(ra), bb = fx_bound(rb);
+            FxBound ba = fx_bound(ra, kea), bb = fx_bound(rb, keb);
             fx_warp_bound<1, (P < 32 ? P : 32)>(ba, 0xffffffffu);
             fx_warp_bound<1, (P < 32 ? P : 32)>(bb, 0xffffffffu);
             if (p % 32 == 0) {
@@ -353,36 +469,36 @@ k_zfx(cx<double>* __restrict__ W, const cx<double>* __restrict__ tw, StepDev* __
                 bound[lp][2 * g + 1][p / 32] = bb;
             }
             __syncthreads();
-            // the scales: every mode but the mean counts twice (its conjugate), so half of 2^60 per component
+            // one scale each for u and w: every mode but the mean counts twice (its conjugate), so a
+            // component's modes sum to half of 2^60
             int kk[2];
-            bool bad = false;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                int e = -4096;
+                kk[h] = kFxZero;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     FxBound b = bound[lp][3 * h + c][0];
 #pragma unroll
                     for (int w = 1; w < NW; ++w) b = fx_join(b, bound[lp][3 * h + c][w]);
-                    e = max(e, fx_exponent(b));
+                    kk[h] = min(kk[h], fx_scale_of(b, 2));
                 }
-                const FxScale sc = fx_scale(e);
-                kk[h] = sc.k;
-                bad = bad || sc.bad;
             }
-            const int ku = kk[0] - 2, kw = kk[1] - 2;
-            if (p == 0 && g == 0) scale[lp][L] = make_int2(bad ? kBad : ku, kw);
+            const int ku = kk[0], kw = kk[1];
+            if (p == 0 && g == 0) scale[lp][L] = make_int2(ku, kw);
             const int ka = g < 2 ? ku : kw, kb = g < 1 ? ku : kw;
+            if (MODE == 1) {
+                kA = ka;
+                kB = kb;
+            }
 #pragma unroll
             for (int s = 0; s < E; ++s) a[s] = mk<q64>(0, 0);
 #pragma unroll
             for (int s = 0; s < NLOW; ++s) {
                 const int m = p + P * s;
-                const q64 ax = fx_from(ra[s].x, ka), ay = fx_from(ra[s].y, ka);
-                const q64 bx = fx_from(rb[s].x, kb), by = fx_from(rb[s].y, kb);
+                const cx<q64> va = fx_align(ra[s], kea[s], ka), vb = fx_align(rb[s], keb[s], kb);
                 // a + i b at m, conj(a) + i conj(b) at N - m, real and imaginary parts exchanged (inverse)
-                a[s] = mk<q64>(ay + bx, ax - by);
-                if (m > 0 && m <= G::KC) sb[sidx(N - m)] = mk<q64>(bx - ay, ax + by);
+                a[s] = mk<q64>(va.y + vb.x, va.x - vb.y);
+                if (m > 0 && m <= G::KC) sb[sidx(N - m)] = mk<q64>(vb.x - va.y, va.x + vb.y);
             }
             sync();
 #pragma unroll
@@ -390,96 +506,122 @@ k_zfx(cx<double>* __restrict__ W, const cx<double>* __restrict__ tw, StepDev* __
                 if (P * s + P - 1 >= N - G::KC && p + P * s >= N - G::KC) a[s] = sb[sidx(p + P * s)];
             sync();
         } else {
-            // u x w: (ux, uy), (uz, wx), (wy, wz) -> (Nx, Ny), (Nz, -)
-            double um = 0.0;
-            for (int idx = threadIdx.x; idx < ZP * 2 * N; idx += 3 * P * ZP) {
-                const int line = idx / N, n = idx % N;   // line = pair 2 + L
-                cx<q64>* r = buf + line * 3 * XS + sidx(n);
-                const cx<q64> v1 = r[0], v2 = r[XS], v3 = r[2 * XS];
-                const FxSplit ux = fx_split(v1.x), uy = fx_split(v1.y), uz = fx_split(v2.x);
-                const FxSplit wx = fx_split(v2.y), wy = fx_split(v3.x), wz = fx_split(v3.y);
-                const int ux4 = 4 * ux.ad, uy4 = 4 * uy.ad, uz4 = 4 * uz.ad;
-                r[0] = mk<q64>(fx_cross(uy, uy4, wz, uz, uz4, wy), fx_cross(uz, uz4, wx, ux, ux4, wz));
-                r[XS].x = fx_cross(ux, ux4, wy, uy, uy4, wx);
-                if (want_umax) {
-                    const int ku = scale[line / 2][line % 2].x;
-                    const q64 sp = llabs(v1.x) + llabs(v1.y) + llabs(v2.x);
-                    // lines of tiny values were taken as zero (ku far below the exponent range)
-                    if (ku > -2000 && ku < kBad) um = fmax(um, fx_to(sp, ku));
-                }
-            }
-            if (want_umax) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) um = fmax(um, __shfl_xor_sync(0xffffffffu, um, o));
-                if ((threadIdx.x & 31) == 0) Bits<double>::amax(&sd[blockIdx.y].umax_bits, um);
-            }
-            __syncthreads();
-
             // forward: group 0 -> line a (Nx + i Ny), 1 -> line b, 2 -> Nz_a + i Nz_b
             cx<q64>* ba = buf + lp * 6 * XS;   // line a's buffers; line b's 3 XS further
             sb = g == 0 ? ba : g == 1 ? ba + 3 * XS : ba + XS;
-            unsigned hx = 0u, hy = 0u;
-#pragma unroll
-            for (int s = 0; s < E; ++s) {
-                a[s] = sb[sidx(p + P * s)];
-                if (g == 2) a[s].y = sb[3 * XS + sidx(p + P * s)].x;
-                hx += ((unsigned)abs((int)(a[s].x >> 32)) >> 10) + 1u;
-                hy += ((unsigned)abs((int)(a[s].y >> 32)) >> 10) + 1u;
-            }
-            // |x| < 2^42 per count: a shift of the bit length over 18 bounds the line's sum by 2^60
-#pragma unroll
-            for (int o = 1; o < (P < 32 ? P : 32); o <<= 1) {
-                hx += __shfl_xor_sync(0xffffffffu, hx, o);
-                hy += __shfl_xor_sync(0xffffffffu, hy, o);
-            }
-            if constexpr (NW > 1) {
-                if (p % 32 == 0) count[lp][g][p / 32] = make_uint2(hx, hy);
-                __syncthreads();
-                hx = hy = 0u;
-#pragma unroll
-                for (int w = 0; w < NW; ++w) {
-                    hx += count[lp][g][w].x;
-                    hy += count[lp][g][w].y;
+            if constexpr (MODE == 0) {
+                // u x w: (ux, uy), (uz, wx), (wy, wz) -> (Nx, Ny), (Nz, -)
+                double um = 0.0;
+                for (int idx = threadIdx.x; idx < ZP * 2 * N; idx += 3 * P * ZP) {
+                    const int line = idx / N, n = idx % N;   // line = pair 2 + L
+                    cx<q64>* r = buf + line * 3 * XS + sidx(n);
+                    const cx<q64> v1 = r[0], v2 = r[XS], v3 = r[2 * XS];
+                    const FxSplit ux = fx_split(v1.x), uy = fx_split(v1.y), uz = fx_split(v2.x);
+                    const FxSplit wx = fx_split(v2.y), wy = fx_split(v3.x), wz = fx_split(v3.y);
+                    const int ux4 = 4 * ux.ad, uy4 = 4 * uy.ad, uz4 = 4 * uz.ad;
+                    r[0] = mk<q64>(fx_cross(uy, uy4, wz, uz, uz4, wy), fx_cross(uz, uz4, wx, ux, ux4, wz));
+                    r[XS].x = fx_cross(ux, ux4, wy, uy, uy4, wx);
+                    if (want_umax) {
+                        const q64 sp = llabs(v1.x) + llabs(v1.y) + llabs(v2.x);
+                        um = fmax(um, fx_to_any(mk<q64>(sp, 0), scale[line / 2][line % 2].x).x);
+                    }
                 }
-            }
-            shx = max(0, 14 - __clz(hx));
-            shy = max(0, 14 - __clz(hy));
-            const q64 rx = (1ll << shx) >> 1, ry = (1ll << shy) >> 1;
+                if (want_umax) {
 #pragma unroll
-            for (int s = 0; s < E; ++s) a[s] = mk<q64>((a[s].x + rx) >> shx, (a[s].y + ry) >> shy);
+                    for (int o = 16; o > 0; o >>= 1) um = fmax(um, __shfl_xor_sync(0xffffffffu, um, o));
+                    if ((threadIdx.x & 31) == 0) Bits<double>::amax(&sd[blockIdx.y].umax_bits, um);
+                }
+                __syncthreads();
+
+                unsigned hx = 0u, hy = 0u;
+#pragma unroll
+                for (int s = 0; s < E; ++s) {
+                    a[s] = sb[sidx(p + P * s)];
+                    if (g == 2) a[s].y = sb[3 * XS + sidx(p + P * s)].x;
+                    hx += ((unsigned)abs((int)(a[s].x >> 32)) >> 10) + 1u;
+                    hy += ((unsigned)abs((int)(a[s].y >> 32)) >> 10) + 1u;
+                }
+                // |x| < 2^42 per count: a shift of the bit length over 18 bounds the line's sum by 2^60
+#pragma unroll
+                for (int o = 1; o < (P < 32 ? P : 32); o <<= 1) {
+                    hx += __shfl_xor_sync(0xffffffffu, hx, o);
+                    hy += __shfl_xor_sync(0xffffffffu, hy, o);
+                }
+                if constexpr (NW > 1) {
+                    if (p % 32 == 0) count[lp][g][p / 32] = make_uint2(hx, hy);
+                    __syncthreads();
+                    hx = hy = 0u;
+#pragma unroll
+                    for (int w = 0; w < NW; ++w) {
+                        hx += count[lp][g][w].x;
+                        hy += count[lp][g][w].y;
+                    }
+                }
+                const int shx = max(0, 14 - __clz(hx)), shy = max(0, 14 - __clz(hy));
+                const q64 rx = (1ll << shx) >> 1, ry = (1ll << shy) >> 1;
+#pragma unroll
+                for (int s = 0; s < E; ++s) a[s] = mk<q64>((a[s].x + rx) >> shx, (a[s].y + ry) >> shy);
+                // the spectra's scales (one more for the halves)
+                const int2 s0 = scale[lp][g == 1 ? 1 : 0], s1 = scale[lp][g == 0 ? 0 : 1];
+                kA = fx_product_scale(s0, shx);
+                kB = fx_product_scale(s1, shy);
+            } else {
+                constexpr long long kReal = (long long)N * N * N;
+                const double* r0 = real + (g == 2 ? 2 * kReal : 0) + (g == 1 ? la + 1 : la) * N;
+                const double* r1 = real + (g == 2 ? 2 * kReal : kReal) + (g == 0 ? la : la + 1) * N;
+                cx<double> v[E];
+#pragma unroll
+                for (int s = 0; s < E; ++s) v[s] = mk(r0[p + P * s], r1[p + P * s]);
+                FxBound b = fx_bound(v);
+                fx_warp_bound<1, (P < 32 ? P : 32)>(b, 0xffffffffu);
+                if constexpr (NW > 1) {
+                    if (p % 32 == 0) bound[lp][g][p / 32] = b;
+                    __syncthreads();
+                    b = bound[lp][g][0];
+#pragma unroll
+                    for (int w = 1; w < NW; ++w) b = fx_join(b, bound[lp][g][w]);
+                }
+                const int k = fx_scale(b, 1, kFxFlush);
+#pragma unroll
+                for (int s = 0; s < E; ++s) a[s] = mk<q64>(fx_from(v[s].x, k), fx_from(v[s].y, k));
+                kA = kB = k == kFxZero || k == kFxBad ? k : k + 1;
+            }
             sync();
         }
-        PL::template fwd<false>(a, sb, p, twq, sidx, sync);
-        if (L < 2) {
+        PL::template fwd<false>(a, sb, p, tw, sidx, sync);
+        if (L < 2 && MODE == 0) {
 #pragma unroll
             for (int s = 0; s < E; ++s) sb[sidx(p + P * s)] = mk<q64>(a[s].y, a[s].x);
             // the line's real space is complete, and its bounds are read
+            __syncthreads();
+        } else if (L < 2) {
+            double* r = real + (long long)2 * g * N * N * N + (la + L) * N;
+#pragma unroll
+            for (int s = 0; s < E; ++s) {
+                r[p + P * s] = fx_to_any(mk<q64>(a[s].y, 0), kA).x;
+                r[(long long)N * N * N + p + P * s] = fx_to_any(mk<q64>(a[s].x, 0), kB).x;
+            }
             __syncthreads();
         } else {
 #pragma unroll
             for (int s = 0; s < E; ++s)   // only the slots read below: N - m
                 if (P * s + P - 1 >= N - G::KC || s == 0) sb[sidx(p + P * s)] = a[s];
             sync();
-            const int2 s0 = scale[lp][g == 1 ? 1 : 0], s1 = scale[lp][g == 0 ? 0 : 1];   // of the two outputs' lines
-            cx<double>* outA = W + (g == 2 ? 2 * G::FS : 0) + (g == 1 ? la + 1 : la) * G::NZP;
-            cx<double>* outB = W + (g == 2 ? 2 * G::FS : G::FS) + (g == 0 ? la : la + 1) * G::NZP;
-            // the spectra's scales (one more for the halves); out of the exponent range: zero below
-            // (and for lines taken as zero), NaN above
-            const int kA = s0.x + s0.y - 60 - shx + 1, kB = s1.x + s1.y - 60 - shy + 1;
-            const bool tinyA = kA > 1020 || min(s0.x, s0.y) < -2000, tinyB = kB > 1020 || min(s1.x, s1.y) < -2000;
-            const bool bad = s0.x == kBad || s1.x == kBad || (!tinyA && kA < -900) || (!tinyB && kB < -900);
+            const int fA = g == 2 ? 2 : 0, fB = g == 2 ? 2 : 1;
+            const long long lA = g == 1 ? la + 1 : la, lB = g == 0 ? la : la + 1;
+            cx<q64>* outA = W + fA * G::FS + lA * G::NZP;
+            cx<q64>* outB = W + fB * G::FS + lB * G::NZP;
+            if (p == 0) {
+                sc.z[(long long)fA * N * N + lA] = kA;
+                sc.z[(long long)fB * N * N + lB] = kB;
+            }
 #pragma unroll
             for (int s = 0; s < NLOW; ++s) {
                 const int m = p + P * s;
                 if (m <= G::KC) {
                     const cx<q64> zm = a[s], zc = sb[sidx(m == 0 ? 0 : N - m)];
-                    cx<double> oa = mk(fx_to(zm.x + zc.x, kA), fx_to(zm.y - zc.y, kA));
-                    cx<double> ob = mk(fx_to(zm.y + zc.y, kB), fx_to(zc.x - zm.x, kB));
-                    if (tinyA) oa = czero<double>();
-                    if (tinyB) ob = czero<double>();
-                    if (bad) oa = ob = mk(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));
-                    outA[m] = oa;
-                    outB[m] = ob;
+                    outA[m] = mk<q64>(zm.x + zc.x, zm.y - zc.y);
+                    outB[m] = mk<q64>(zm.y + zc.y, zc.x - zm.x);
                 }
             }
         }

@@ -5,22 +5,26 @@
 // multiply-add, so an FP64 butterfly costs about 64 issue slots per instruction.
 // A transform's own values need no floating exponent: every intermediate value of
 // a DFT is a sum of inputs times numbers of modulus <= 1, so it is bounded by the
-// line's L1 norm. Each line is therefore scaled by the power of two that puts its
-// L1 norm just below 2^61, converted to 64-bit integers, transformed with exact
-// 64-bit additions and 64x61-bit twiddle products (both parts of the product that
-// reach the result's last bit), and converted back with one rounding. No stage
-// needs a shift and nothing can overflow. The absolute error is about one unit of
-// 2^-61 of the L1 norm per input and per twiddle product, below the rounding errors
-// of the FP64 butterflies it replaces (measured against 64-bit library transforms
-// in tests/test_fx_fft.py).
+// line's L1 norm. Each line is therefore scaled by the power of two that keeps its
+// L1 norm below 2^61, held in 64-bit integers and transformed with exact 64-bit
+// additions and 64x61-bit twiddle products (both parts of the product that reach the
+// result's last bit). No stage needs a shift and nothing can overflow. The absolute
+// error is about one unit of 2^-61 of the L1 norm per input and per twiddle product,
+// below the rounding errors of the FP64 butterflies it replaces (measured against
+// 64-bit library transforms in tests/test_fx_fft.py).
+//
+// Between the passes the fields stay integers, each line with its scale k (value =
+// integer 2^-k) in a table beside them (FxScales); the next pass brings a line's
+// elements to a common scale. Doubles are read and written on the sphere's modes only
+// (the x passes), and the integers' range does not end at FP64's exponents.
 //
 // Measured on a GB300 against FP64 butterflies (one RK4 step): 128^3 3.55 -> 0.78 ms, 256^3
 // 28.3 -> 5.6 ms, 512^3 250 -> 54 ms; the nonlinear term's error against a 113-bit
 // evaluation at 16^3 .. 48^3 falls from 3.1e-16 .. 9.9e-16 to 1.5e-16 .. 2.9e-16.
 //
-// Lines that hold a NaN or Inf return NaN throughout, as any transform of them
-// does; lines whose L1 norm is below 2^-900 (values under about 1e-274) are taken
-// as zero.
+// Lines that hold a NaN or Inf carry the scale kFxBad and end as NaN throughout, as any
+// transform of them does; lines of doubles whose L1 norm is below 2^-900 (values under
+// about 1e-274) are taken as zero, scale kFxZero.
 #pragma once
 #include "fft_engine.cuh"
 
@@ -150,31 +154,29 @@ template <> struct TwOf<cx<q64>> {
 };
 
 // ---------------------------------------------------------------------------
-// Scale of a line. Each thread adds the magnitudes of its values as FP32 numbers cut
-// from the high words, in units set by its largest exponent (FP64's range does not fit
-// FP32's); the threads of a line combine their sums.
+// Scale of a line. Each thread bounds the sum of its magnitudes in units set by its
+// largest value; the threads of a line combine their sums.
 // ---------------------------------------------------------------------------
+constexpr int kFxZero = 30000, kFxBad = -30000;
 struct FxBound {
-    float sum;   // sum of magnitudes / 2^(lo - 896), low by under 2^-19 of itself
-    int lo;      // exponent field that the sum's unit belongs to
+    float sum;   // the magnitudes sum to sum 2^e, low by under 2^-19 of itself
+    int e;
 };
-struct FxScale {
-    int k;       // values times 2^k are the integers
-    bool bad;    // a NaN or Inf in the line
-};
-constexpr int kFxSpan = 190;   // the largest exponent field is lo + kFxSpan (kept below 254: room for sums)
+// Doubles: FP32 numbers cut from the high words with the exponent rebased on the multiply
+// pipe (largest field base + kFxSpan: room for sums); smaller values count as zero.
+constexpr int kFxSpan = 190;
 template <int E>
 __device__ __forceinline__ FxBound fx_bound(const cx<double> (&v)[E]) {
     unsigned top = 0u;
 #pragma unroll
     for (int s = 0; s < E; ++s)
         top = max(top, max((unsigned)__double2hiint(v[s].x) & 0x7fffffffu, (unsigned)__double2hiint(v[s].y) & 0x7fffffffu));
-    FxBound b{0.f, max((int)(top >> 20) - kFxSpan, 0)};
-    const unsigned low = (unsigned)b.lo << 20;
-    const int base = (int)(0u - ((unsigned)b.lo << 23));
+    const int lo = max((int)(top >> 20) - kFxSpan, 0);
+    const unsigned low = (unsigned)lo << 20;
+    const int base = (int)(0u - ((unsigned)lo << 23));
+    FxBound b{0.f, top >= 0x7ff00000u ? -kFxBad : lo - 896};
 #pragma unroll
     for (int s = 0; s < E; ++s) {
-        // the exponent rebased on the multiply pipe; values below the unit's range count as zero
         int x, y;
         asm("mad.lo.s32 %0, %1, 8, %2;" : "=r"(x) : "r"((int)max((unsigned)__double2hiint(v[s].x) & 0x7fffffffu, low)), "r"(base));
         asm("mad.lo.s32 %0, %1, 8, %2;" : "=r"(y) : "r"((int)max((unsigned)__double2hiint(v[s].y) & 0x7fffffffu, low)), "r"(base));
@@ -183,113 +185,105 @@ __device__ __forceinline__ FxBound fx_bound(const cx<double> (&v)[E]) {
     }
     return b;
 }
+// Integers (|a| <= 2^61) with their scales: sums of the high words' upper bits, aligned to
+// the thread's smallest scale, in units of 2^38; at most 2^28 for 16 elements.
+template <int E>
+__device__ __forceinline__ FxBound fx_bound(const cx<q64> (&a)[E], const int (&k)[E]) {
+    int km = kFxZero;
+#pragma unroll
+    for (int s = 0; s < E; ++s) km = min(km, k[s]);
+    unsigned sum = 2 * E;   // cut parts
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+        const int sh = min(6 + k[s] - km, 31);
+        sum += ((unsigned)abs((int)(a[s].x >> 32)) >> sh) + ((unsigned)abs((int)(a[s].y >> 32)) >> sh);
+    }
+    return FxBound{(float)sum, 38 - km};
+}
 __device__ __forceinline__ FxBound fx_join(FxBound a, FxBound b) {
-    const int lo = max(a.lo, b.lo);
-    const float fa = __int_as_float(max(127 + a.lo - lo, 0) << 23), fb = __int_as_float(max(127 + b.lo - lo, 0) << 23);
-    return FxBound{a.sum * fa + b.sum * fb, lo};
+    const int e = max(a.e, b.e);
+    const float fa = __int_as_float(max(127 + a.e - e, 0) << 23), fb = __int_as_float(max(127 + b.e - e, 0) << 23);
+    return FxBound{a.sum * fa + b.sum * fb, e};
 }
-// floor(log2(L1 norm)) or above; -4096: nothing to transform; over 1000: NaN, Inf or out of range
-__device__ __forceinline__ int fx_exponent(FxBound b) {
-    const float f = b.sum * 1.0001f;
-    if (b.lo >= 2047 - kFxSpan) return 4096;
-    const int e = (int)(__float_as_uint(f) >> 23) - 127 + b.lo - 896;
-    return f < 1e-30f || e < -900 ? -4096 : e;
-}
-__device__ __forceinline__ FxScale fx_scale(int e) {
-    return FxScale{e == -4096 ? -4096 : 60 - e, e > 1000};   // |values| 2^k sum to less than 2^61
-}
-// v 2^k as an integer, cut towards zero
-__device__ __forceinline__ q64 fx_from(double v, int k) {
-    const int hi = __double2hiint(v), lo = __double2loint(v);
-    const int sh = min(1083 - k - (int)(((unsigned)hi << 1) >> 21), 63);   // >= 0: |v| 2^k < 2^61
-    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    const q64 r = (q64)((((unsigned long long)mh << 32 | (unsigned)lo) << 8) >> sh);
-    const q64 sgn = hi >> 31;
-    return (r ^ sgn) - sgn;
-}
-// i 2^-k, rounded to nearest: the conversion on the FP64 pipe (idle in a transform), the
-// scale as an exponent addition
-__device__ __forceinline__ double fx_to(q64 i, int k) {
-    const double d = __ll2double_rn(i);
-    const int hi = __double2hiint(d);
-    return __hiloint2double(hi ? hi - (k << 20) : 0, __double2loint(d));
-}
-
 // combine the bounds of the lanes of a warp that differ in the bits of LO..HI-1
 template <int LO, int HI>
 __device__ __forceinline__ void fx_warp_bound(FxBound& b, unsigned mask) {
 #pragma unroll
     for (int o = LO; o < HI; o <<= 1)
-        b = fx_join(b, FxBound{__shfl_xor_sync(mask, b.sum, o), __shfl_xor_sync(mask, b.lo, o)});
+        b = fx_join(b, FxBound{__shfl_xor_sync(mask, b.sum, o), __shfl_xor_sync(mask, b.e, o)});
 }
-
-// ---------------------------------------------------------------------------
-// A line transform of the passes, v: the thread's E elements (see fft_stages).
-// STRIDED passes: the block's NT threads hold TT lines, thread = p TT + t. Line
-// passes (TT = 1): P consecutive threads hold a line. `tw` is the engine's table.
-// FP32 lines run in floating point. The FP64 result is scaled by 2^-kadd; its slots
-// outside the kept band are taken as zero in an inverse transform and left as they
-// were by a forward one.
-// ---------------------------------------------------------------------------
-template <class PL, bool INV, bool PK, int TT, int NT, typename SIdx, typename Sync, int E>
-__device__ __forceinline__ void line_fft(cx<float> (&v)[E], cx<float>* sbuf, int p, const cx<float>* __restrict__ tw,
-                                         SIdx sidx, Sync sync) {
-    if constexpr (INV) PL::template inv<PK>(v, sbuf, p, tw, sidx, sync);
-    else PL::template fwd<PK>(v, sbuf, p, tw, sidx, sync);
-}
-// slot s of every thread lies outside the kept band |k| <= KC = N / 3: a quarter of the
-// slots of 16, neither converted nor added (256^3 y passes 0.272 + 0.142 -> 0.255 + 0.132 ms)
-template <class PL> constexpr bool fx_outside(int s) {
-    return PL::P * s > PL::N / 3 && PL::P * s + PL::P - 1 < PL::N - PL::N / 3;
-}
-template <class PL, bool INV, bool PK, int TT, int NT, typename SIdx, typename Sync, int E>
-__device__ __forceinline__ void line_fft(cx<double> (&v)[E], cx<double>* sbuf, int p,
-                                         const cx<double>* __restrict__ tw, SIdx sidx, Sync sync, int kadd = 0) {
-    constexpr int P = PL::P;
-    FxBound bd = fx_bound(v);
+// The bound of a line of a strided tile: NT threads of the block hold tiles of TT lines, P
+// threads each, thread = (tile P + p) TT + t.
+template <int P, int TT, int NT, typename Sync>
+__device__ __forceinline__ FxBound fx_line_bound(FxBound b, Sync sync) {
     if constexpr (P > 1) {
         // the lanes of this warp (the last warp of a small block may be short)
         const unsigned mask =
             NT % 32 == 0 || (int)(threadIdx.x | 31) < NT ? 0xffffffffu : (1u << (NT % 32 ? NT % 32 : 31)) - 1u;
-        constexpr int span = P * TT < 32 ? P * TT : 32;   // lanes that hold parts of one line's tile
-        fx_warp_bound<TT, span>(bd, mask);
+        constexpr int span = P * TT < 32 ? P * TT : 32;   // lanes that hold parts of one tile
+        fx_warp_bound<TT, span>(b, mask);
         if constexpr (P * TT > 32) {
             // several warps per tile: one entry per warp and line
             constexpr int NW = P * TT / 32;
             __shared__ FxBound part[NT / 32][TT];
             const int w = threadIdx.x / 32, t = threadIdx.x % TT;
-            if ((threadIdx.x & 31) < TT) part[w][t] = bd;
+            if ((threadIdx.x & 31) < TT) part[w][t] = b;
             sync();
             const int w0 = w / NW * NW;
-            bd = part[w0][t];
+            b = part[w0][t];
 #pragma unroll
-            for (int q = 1; q < NW; ++q) bd = fx_join(bd, part[w0 + q][t]);
+            for (int q = 1; q < NW; ++q) b = fx_join(b, part[w0 + q][t]);
         }
     }
-    const FxScale sc = fx_scale(fx_exponent(bd));
-    cx<q64> a[E];
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-        a[s] = mk<q64>(0, 0);
-        if (INV && fx_outside<PL>(s)) continue;
-        // the inverse transform is the forward one with real and imaginary parts exchanged
-        const q64 x = fx_from(v[s].x, sc.k), y = fx_from(v[s].y, sc.k);
-        a[s] = INV ? mk<q64>(y, x) : mk<q64>(x, y);
-    }
-    PL::template fwd<false>(a, reinterpret_cast<cx<q64>*>(sbuf), p, reinterpret_cast<const int4*>(tw), sidx, sync);
-    // a line taken as zero keeps its zeros
-    const int k = (sc.k == -4096 ? 0 : sc.k) + kadd;
-#pragma unroll
-    for (int s = 0; s < E; ++s) {
-        if (!INV && fx_outside<PL>(s)) continue;
-        const double x = fx_to(a[s].x, k), y = fx_to(a[s].y, k);
-        v[s] = INV ? mk(y, x) : mk(x, y);
-    }
-    if (sc.bad) {
-        const double nan = __hiloint2double(0x7ff80000, 0);
-#pragma unroll
-        for (int s = 0; s < E; ++s) v[s] = mk(nan, nan);
-    }
+    return b;
+}
+// The largest scale at which a line of this bound sums to less than 2^(61 - spare), kFxZero
+// or kFxBad; doubles below 2^flush count as zero.
+__device__ __forceinline__ int fx_scale(FxBound b, int spare, int flush) {
+    if (b.e >= -kFxBad - 1000) return kFxBad;
+    const float f = b.sum * 1.0001f;
+    const int e = (int)(__float_as_uint(f) >> 23) - 127 + b.e;
+    return f < 1e-30f || e < flush ? kFxZero : 60 - spare - e;
+}
+constexpr int kFxFlush = -900, kFxNoFlush = -20000;
+// and for integers: no finer than the finest common scale of the elements
+__device__ __forceinline__ int fx_scale_of(FxBound b, int spare) {
+    const int k = fx_scale(b, spare, kFxNoFlush);
+    return k == kFxBad || k == kFxZero ? k : min(k, 38 - b.e);
+}
+// v 2^k as an integer, cut towards zero (|v| 2^k < 2^61)
+__device__ __forceinline__ q64 fx_from(double v, int k) {
+    const int hi = __double2hiint(v), lo = __double2loint(v);
+    const int sh = min(max(1083 - k - (int)(((unsigned)hi << 1) >> 21), 0), 63);
+    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    const q64 r = (q64)((((unsigned long long)mh << 32 | (unsigned)lo) << 8) >> sh);
+    const q64 sgn = hi >> 31;
+    return (r ^ sgn) - sgn;
+}
+// an integer at scale k0 to the line's scale k <= k0, rounded to nearest
+__device__ __forceinline__ cx<q64> fx_align(cx<q64> a, int k0, int k) {
+    const int sh = min(max(k0 - k, 0), 63);
+    const q64 half = (q64)((1ull << sh) >> 1);
+    return mk<q64>((a.x + half) >> sh, (a.y + half) >> sh);
+}
+// i 2^-k, rounded to nearest: the conversion on the FP64 pipe, the scale as an exponent
+// addition (-1020 <= -k, |i| < 2^62)
+__device__ __forceinline__ double fx_to(q64 i, int k) {
+    const double d = __ll2double_rn(i);
+    const int hi = __double2hiint(d);
+    return __hiloint2double(hi ? hi - (k << 20) : 0, __double2loint(d));
+}
+// the same over all scales: zero below FP64's range, NaN above it and for bad lines
+__device__ __forceinline__ cx<double> fx_to_any(cx<q64> a, int k) {
+    if (k > 1020) return czero<double>();
+    if (k < -900) return mk(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));
+    return mk(fx_to(a.x, k), fx_to(a.y, k));
+}
+// slot s of every thread lies outside the kept band |k| <= KC = N / 3: a quarter of the
+// slots of 16, neither loaded nor added by an inverse transform, nor stored by a forward
+// one (256^3 y passes 0.272 + 0.142 -> 0.255 + 0.132 ms)
+template <class PL> constexpr bool fx_outside(int s) {
+    return PL::P * s > PL::N / 3 && PL::P * s + PL::P - 1 < PL::N - PL::N / 3;
 }
 
 }  // namespace ns3d

@@ -101,6 +101,10 @@ class Impl final : public Base {
     cx<T>* UTm(int m) const { return UT_ + (size_t)m * 3 * G::FS; }
     cx<T>* ACCm(int m) const { return ACC_ + (size_t)m * 3 * G::FS; }
     cx<T>* Wm(int m) const { return W_ + (size_t)m * 6 * G::FS; }
+    // FP64 engines: W as integers, its lines' scales, the integer twiddles (fx_passes.cuh)
+    cx<q64>* Wq(int m) const { return reinterpret_cast<cx<q64>*>(Wm(m)); }
+    int* scales(int m) const { return scales_ + (size_t)m * fx_scales_ints<N>(); }
+    const int4* twq() const { return reinterpret_cast<const int4*>(tw_); }
     cx<T>* tabm(int m) const { return tab_ + (size_t)m * (G::KC2 + 1); }
     StepDev* sdm(int m) const { return sd_ + m; }
 
@@ -109,7 +113,7 @@ class Impl final : public Base {
         for (void* q : {(void*)U_, (void*)UT_, (void*)ACC_, (void*)W_, (void*)tw_, (void*)tab_, (void*)part_,
                         (void*)mout_, (void*)stage_, (void*)real_, (void*)sd_, (void*)TAU_, (void*)F_,
                         (void*)tau_real_, (void*)sgs_part_, (void*)K_, (void*)dpart_, (void*)plan_out_.ranges, (void*)plan_in_.ranges,
-                        (void*)zg_b_, (void*)zg_P_, (void*)xt_items_, (void*)aux_})
+                        (void*)zg_b_, (void*)zg_P_, (void*)xt_items_, (void*)aux_, (void*)scales_})
             if (q) cudaFree(q);
         if (sd_host_) cudaFreeHost(sd_host_);
         if (mout_host_) cudaFreeHost(mout_host_);
@@ -181,12 +185,20 @@ class Impl final : public Base {
         } else {
             NS3D_CK(cudaFuncSetAttribute(k_xinv<T, N, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_xi()));
         }
-        NS3D_CK(cudaFuncSetAttribute(k_ypass<T, N, true, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_a()));
-        NS3D_CK(cudaFuncSetAttribute(k_ypass<T, N, false, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_af()));
-        if constexpr (sizeof(T) == 8)
-            NS3D_CK(cudaFuncSetAttribute(k_zfx<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, zfx_smem<N>()));
-        else
+        if constexpr (sizeof(T) == 8) {
+            NS3D_CK(cudaMalloc(&scales_, sizeof(int) * fx_scales_ints<N>() * M_));
+            NS3D_CK(cudaFuncSetAttribute(k_ypass_fx<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_a()));
+            NS3D_CK(cudaFuncSetAttribute(k_ypass_fx<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_af()));
+            NS3D_CK(cudaFuncSetAttribute(k_zfx<N, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, zfx_smem<N>()));
+            NS3D_CK(cudaFuncSetAttribute(k_zfx<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, zfx_smem<N>()));
+            NS3D_CK(cudaFuncSetAttribute(k_zfx<N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, zfx_smem<N>()));
+        } else {
+            NS3D_CK(cudaFuncSetAttribute(k_ypass<T, N, true, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_a()));
+            NS3D_CK(cudaFuncSetAttribute(k_ypass<T, N, false, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_af()));
             NS3D_CK(cudaFuncSetAttribute(k_zpass<T, N, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_z()));
+            NS3D_CK(cudaFuncSetAttribute(k_zpass<T, N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_z()));
+            NS3D_CK(cudaFuncSetAttribute(k_zpass<T, N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_z()));
+        }
         if constexpr (zline_ok<T, N>()) {
             NS3D_CK(cudaFuncSetAttribute(k_zline<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_zl()));
             int per_sm = 0, nsm = 0, dev = 0;
@@ -195,8 +207,6 @@ class Impl final : public Base {
             NS3D_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_zline<T, N>, ZLINE_WARPS * 32, smem_zl()));
             zline_ctas_ = (per_sm > 0 ? per_sm : 1) * nsm;
         }
-        NS3D_CK(cudaFuncSetAttribute(k_zpass<T, N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_z()));
-        NS3D_CK(cudaFuncSetAttribute(k_zpass<T, N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_z()));
         if constexpr (zgemm_ok<T, N>()) {
             // z-pass form 2: DFT matrices (built once, on the host), the product workspace
             using Z = ZGeo<N>;
@@ -300,12 +310,15 @@ class Impl final : public Base {
         }
         const cx<T>* src = in + (size_t)m0 * 3 * G::FS;
         if constexpr (sizeof(T) == 8)
-            pass(k_xinv_fx<N>, dim3(NTX, G::NKY, 6 * cnt), fxinv_threads<N>(), fxinv_smem<N>(), s_)(src, Wm(m0), tw_, aux_);
+            pass(k_xinv_fx<N>, dim3(NTX, G::NKY, 6 * cnt), fxinv_threads<N>(), fxinv_smem<N>(), s_)(src, Wq(m0), scales(m0), twq(), aux_);
         else
             pass(k_xinv<T, N, V>, dim3(NTX, G::NKY, cnt), TX * PX::P, smem_xi(), s_)(src, Wm(m0), tw_);
     }
     void p2(int m0, int cnt) {
-        pass(k_ypass<T, N, true, V>, dim3(NTA, N, 6 * cnt), TA * PY::P, smem_a(), s_)(Wm(m0), tw_);
+        if constexpr (sizeof(T) == 8)
+            pass(k_ypass_fx<N, true>, dim3(NTA, N, 6 * cnt), fxy_threads<N>(), smem_a(), s_)(Wq(m0), scales(m0), twq());
+        else
+            pass(k_ypass<T, N, true, V>, dim3(NTA, N, 6 * cnt), TA * PY::P, smem_a(), s_)(Wm(m0), tw_);
     }
     static constexpr size_t smem_zl() { return zline_smem<T, N>(); }
     void p3(int want_umax, int m0, int cnt) {
@@ -335,10 +348,28 @@ class Impl final : public Base {
             }
         }
         if constexpr (sizeof(T) == 8)
-            pass(k_zfx<N>, dim3((unsigned)((long long)N * N / 2 / zfx_pairs<N>()), cnt), zfx_threads<N>(), zfx_smem<N>(), s_)(
-                Wm(m0), tw_, sdm(m0), want_umax);
+            zfx<0>(nullptr, sdm(m0), want_umax, m0, cnt);
         else
             pass(k_zpass<T, N, 0>, dim3((unsigned)((long long)N * N / 2 / ZP), cnt), 3 * PA::P * ZP, smem_z(), s_)(Wm(m0), tw_, nullptr, sdm(m0), want_umax);
+    }
+    // the selected member's W (P2's output) to real_ [6][N][N][N], and real_ [3][N][N][N] to W
+    void c2r() {
+        if constexpr (sizeof(T) == 8) zfx<1>(real_, nullptr, 0, m_, 1);
+        else
+            pass(k_zpass<T, N, 1>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
+                Wm(m_), tw_, real_, nullptr, 0);
+    }
+    void r2c() {
+        if constexpr (sizeof(T) == 8) zfx<2>(real_, nullptr, 0, m_, 1);
+        else
+            pass(k_zpass<T, N, 2>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
+                Wm(m_), tw_, real_, nullptr, 0);
+    }
+    template <int MODE>
+    void zfx(T* real, StepDev* sd, int want_umax, int m0, int cnt) {
+        if constexpr (sizeof(T) == 8)
+            pass(k_zfx<N, MODE>, dim3((unsigned)((long long)N * N / 2 / zfx_pairs<N>()), cnt), zfx_threads<N>(),
+                 zfx_smem<N>(), s_)(Wq(m0), scales(m0), twq(), real, sd, want_umax);
     }
     void set_zform(int z) override {
         const int zn = (zline_ok<T, N>() && z == 0) ? 0 : (zgemm_ok<T, N>() && z == 2) ? 2 : 1;
@@ -351,7 +382,10 @@ class Impl final : public Base {
     int zform() const override { return zform_; }
     int variant() const override { return V; }
     void p4(int m0, int cnt) {
-        pass(k_ypass<T, N, false, V>, dim3(NTAF, N, 3 * cnt), TAF * PYF::P, smem_af(), s_)(Wm(m0), tw_);
+        if constexpr (sizeof(T) == 8)
+            pass(k_ypass_fx<N, false>, dim3(NTAF, N, 3 * cnt), fxy_threads<N>(), smem_af(), s_)(Wq(m0), scales(m0), twq());
+        else
+            pass(k_ypass<T, N, false, V>, dim3(NTAF, N, 3 * cnt), TAF * PYF::P, smem_af(), s_)(Wm(m0), tw_);
     }
     template <int INTEG, int MODE>
     void p5x(int m0, int cnt, cx<T>* out) {
@@ -359,7 +393,7 @@ class Impl final : public Base {
         const dim3 grid(NTXF, G::NKY, cnt);
         if constexpr (sizeof(T) == 8)
             pass(k_xfwd_fx<N, INTEG, MODE>, grid, fxfwd_threads<N>(), fxfwd_smem<N>(), s_)(
-                Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0), aux_, nullptr, nullptr, RkStage{});
+                Wq(m0), scales(m0), Um(m0), UTm(m0), acc, twq(), sdm(m0), tabm(m0), aux_, nullptr, nullptr, RkStage{});
         else
             pass(k_xfwd<T, N, INTEG, MODE, V>, grid, TXF * PX::P, smem_x(), s_)(
                 Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0), (les_ && MODE <= X_STAGE4) ? F_ : nullptr,
@@ -372,7 +406,8 @@ class Impl final : public Base {
         double* dpart = dpart_ + (size_t)m0 * 3 * NTXF * G::NKY;
         if constexpr (sizeof(T) == 8)
             pass(k_xfwd_fx<N, INT_TAB, X_STAGE1>, grid, fxfwd_threads<N>(), fxfwd_smem<N>(), s_)(
-                Wm(m0), Um(m0), UTm(m0), ACCm(m0), tw_, sdm(m0), tabm(m0), aux_, K, dpart, rk_stage(s, dp5()));
+                Wq(m0), scales(m0), Um(m0), UTm(m0), ACCm(m0), twq(), sdm(m0), tabm(m0), aux_, K, dpart,
+                rk_stage(s, dp5()));
         else
             pass(k_xfwd<T, N, INT_TAB, X_STAGE1, V>, grid, TXF * PX::P, smem_x(), s_)(
                 Wm(m0), Um(m0), UTm(m0), ACCm(m0), tw_, sdm(m0), tabm(m0), les_ ? F_ : nullptr, K, dpart,
@@ -851,8 +886,7 @@ class Impl final : public Base {
         ns3d_status st = ensure_real();
         if (st != NS3D_OK) return st;
         k_fill_real<T, N><<<grid_for((long long)N * N * N), 256, 0, s_>>>(real_, kind);
-        pass(k_zpass<T, N, 2>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
-            Wm(m_), tw_, real_, nullptr, 0);
+        r2c();
         p4(m_, 1);
         p5<X_PLAIN>(m_, 1, U_);
         NS3D_CK(cudaGetLastError());
@@ -906,8 +940,7 @@ class Impl final : public Base {
         if (st == NS3D_OK) st = ensure_stage();
         if (st != NS3D_OK) return st;
         p1(U_, m_, 1); p2(m_, 1);
-        pass(k_zpass<T, N, 1>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
-            Wm(m_), tw_, real_, nullptr, 0);
+        c2r();
         // a reference real array has the bytes of a Fourier one: both pass through the staging buffer
         const size_t rb = sizeof(double) * 3 * (size_t)N * N * (N + 2);
         static_assert(24LL * N * N * (N + 2) == kRefBytes, "");
@@ -984,8 +1017,7 @@ class Impl final : public Base {
         ns3d_status st = ensure_real();
         if (st != NS3D_OK) return st;
         p1(U_, m_, 1); p2(m_, 1);
-        pass(k_zpass<T, N, 1>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
-            Wm(m_), tw_, real_, nullptr, 0);
+        c2r();
         double *part = nullptr, *red = nullptr;
         unsigned long long* cnt = nullptr;
         cudaError_t e = cudaMalloc(&part, sizeof(double) * (kIncrParts * 4 + 8));
@@ -1129,8 +1161,7 @@ class Impl final : public Base {
         *st = ensure_real();
         if (*st != NS3D_OK) return nullptr;
         p1(U_, m_, 1); p2(m_, 1);
-        pass(k_zpass<T, N, 1>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
-            Wm(m_), tw_, real_, nullptr, 0);
+        c2r();
         *st = cudaGetLastError() == cudaSuccess ? NS3D_OK : NS3D_ERR_CUDA;
         return reinterpret_cast<const float*>(real_);
     }
@@ -1142,8 +1173,7 @@ class Impl final : public Base {
         NS3D_CK(cudaMemcpyAsync(stage_, u, sizeof(double) * 3 * (size_t)N * N * (N + 2), cudaMemcpyHostToDevice, s_));
         k_real_pack<T, N><<<grid_for((long long)N * N * N), 256, 0, s_>>>(reinterpret_cast<const double*>(stage_),
                                                                          real_);
-        pass(k_zpass<T, N, 2>, (unsigned)((long long)N * N / 2 / ZP), 3 * PA::P * ZP, smem_z(), s_)(
-            Wm(m_), tw_, real_, nullptr, 0);
+        r2c();
         p4(m_, 1);
         p5<X_PLAIN>(m_, 1, U_);
         NS3D_CK(cudaGetLastError());
@@ -1178,6 +1208,7 @@ class Impl final : public Base {
     CUtensorMap xmap_[2];          // P1 tensor-tile form: U and UT as [3 M][N kx][N ky][2 NZP] FP32
     CUtensorMap wmap_;             // and W as [6 M][N x][N ky][2 NZP] FP32 (its outputs)
     double* aux_ = nullptr;        // FP64 x passes: 1/k2 and the x wavenumbers
+    int* scales_ = nullptr;        // FP64: scales of the lines of W
     int xt_ctas_ = 1;
     int* xt_items_ = nullptr;      // P1 tensor-tile form: compact list of the x tiles inside the circle
     int xt_nvalid_ = 0;

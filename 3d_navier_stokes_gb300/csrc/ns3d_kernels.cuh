@@ -303,8 +303,8 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         load(0, X);
         load(1, Y);
         ikx(Y, B);
-        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
-        line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
+        PL::inv(B, sbuf, p, tw, sidx, sync);
+        PL::inv(X, sbuf, p, tw, sidx, sync);
         store(0, X);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = B[s] - mul_i(X[s]) * fky;
@@ -314,14 +314,14 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
             staged(2, Z);
             ikx(Z, B);
         }
-        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
+        PL::inv(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fkz - B[s];
         store(4, B);
-        line_fft<PL, true, false, TT, NT>(Y, sbuf, p, tw, sidx, sync);
+        PL::inv(Y, sbuf, p, tw, sidx, sync);
         store(1, Y);
         staged(2, X);   // uz
-        line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
+        PL::inv(X, sbuf, p, tw, sidx, sync);
         store(2, X);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fky - mul_i(Y[s]) * fkz;
@@ -335,20 +335,20 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         load(1, Y);
         load(2, Z);
         ikx(Y, B);
-        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
-        line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
+        PL::inv(B, sbuf, p, tw, sidx, sync);
+        PL::inv(X, sbuf, p, tw, sidx, sync);
         store(0, X);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = B[s] - mul_i(X[s]) * fky;
         store(5, B);
         ikx(Z, B);
-        line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
+        PL::inv(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fkz - B[s];
         store(4, B);
-        line_fft<PL, true, false, TT, NT>(Y, sbuf, p, tw, sidx, sync);
+        PL::inv(Y, sbuf, p, tw, sidx, sync);
         store(1, Y);
-        line_fft<PL, true, false, TT, NT>(Z, sbuf, p, tw, sidx, sync);
+        PL::inv(Z, sbuf, p, tw, sidx, sync);
         store(2, Z);
 #pragma unroll
         for (int s = 0; s < E; ++s) B[s] = mul_i(Z[s]) * fky - mul_i(Y[s]) * fkz;
@@ -358,7 +358,7 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
     cx<T> X[E], B[E];
     // ux
     load(0, X);
-    line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
+    PL::inv(X, sbuf, p, tw, sidx, sync);
     store(0, X);
     // wz = T(i kx uy) - i ky T(ux)
     {
@@ -366,7 +366,7 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         staged(1, Y);
         ikx(Y, B);
     }
-    line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
+    PL::inv(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
     for (int s = 0; s < E; ++s) B[s] = B[s] - mul_i(X[s]) * fky;
     store(5, B);
@@ -376,16 +376,16 @@ k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restri
         staged(2, Z);
         ikx(Z, B);
     }
-    line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
+    PL::inv(B, sbuf, p, tw, sidx, sync);
 #pragma unroll
     for (int s = 0; s < E; ++s) B[s] = mul_i(X[s]) * fkz - B[s];
     store(4, B);
     // uy, uz, then wx = i ky T(uz) - i kz T(uy)
     staged(1, X);
-    line_fft<PL, true, false, TT, NT>(X, sbuf, p, tw, sidx, sync);
+    PL::inv(X, sbuf, p, tw, sidx, sync);
     store(1, X);
     staged(2, B);
-    line_fft<PL, true, false, TT, NT>(B, sbuf, p, tw, sidx, sync);
+    PL::inv(B, sbuf, p, tw, sidx, sync);
     store(2, B);
 #pragma unroll
     for (int s = 0; s < E; ++s) B[s] = mul_i(B[s]) * fky - mul_i(X[s]) * fkz;
@@ -640,11 +640,10 @@ k_xinv_tma(const __grid_constant__ CUtensorMap map, int c0, const __grid_constan
 // Forward: inputs every y, outputs only where ky^2 + kz^2 <= KC^2.
 // ---------------------------------------------------------------------------
 // CTAs per SM the y pass is compiled for: 1024 threads per SM (64 registers per
-// thread), 512 (128 registers) for plans of more than 16 elements per thread and
-// for FP64 (its 64-bit integer elements take twice the registers)
+// thread), 512 (128 registers) for plans of more than 16 elements per thread
 template <typename T, int N, int V, bool INV> constexpr int ypass_minb() {
     constexpr int nt = tile_a<T, N, V, INV>() * YPlan<T, N, INV>::A::P;
-    constexpr int per_sm = YPlan<T, N, INV>::A::E > 16 || sizeof(T) == 8 ? 512 : 1024;
+    constexpr int per_sm = YPlan<T, N, INV>::A::E > 16 ? 512 : 1024;
     return per_sm / nt > 0 ? per_sm / nt : 1;
 }
 template <typename T, int N, bool INV, int V = 0>
@@ -676,7 +675,8 @@ k_ypass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw) {
         if (INV) in = in && (ky * ky <= rem) && !(P * s > G::KC && P * s + P - 1 < N - G::KC);
         v[s] = in ? base[(long long)jj * G::NZP] : czero<T>();
     }
-    line_fft<PL, INV, true, TT, TT * P>(v, sbuf, p, tw, sidx, sync);
+    if (INV) PL::template inv<true>(v, sbuf, p, tw, sidx, sync);
+    else PL::template fwd<true>(v, sbuf, p, tw, sidx, sync);
     if (colok) {
 #pragma unroll
         for (int s = 0; s < E; ++s) {
@@ -759,7 +759,7 @@ k_zpass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, T* __restrict__ rea
                 }
                 v[s] = z;
             }
-            line_fft<PL, true, false, 1, 3 * P * ZP>(v, sb, p, tw, sidx, sync);
+            PL::inv(v, sb, p, tw, sidx, sync);
             T* ra = Rl + (L * 6 + 2 * g) * N;
             T* rb = ra + N;
 #pragma unroll
@@ -826,7 +826,7 @@ k_zpass(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, T* __restrict__ rea
         cx<T> v[E];
 #pragma unroll
         for (int s = 0; s < E; ++s) v[s] = mk(ra[p + P * s], rb[p + P * s]);
-        line_fft<PL, false, false, 1, 3 * P * ZP>(v, sb, p, tw, sidx, sync);
+        PL::fwd(v, sb, p, tw, sidx, sync);
 #pragma unroll
         for (int s = 0; s < E; ++s) sb[sidx(p + P * s)] = v[s];
         __syncthreads();
@@ -1369,7 +1369,7 @@ k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ U
     }
     xfwd_prefetch_state<T, N, INTEG, MODE, E, P, TT>(U, ACC, K, rs, p, t, ky, kz0, j);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) line_fft<PL, false, false, TT, TT * P>(F[c], sbuf, p, tw, sidx, sync);
+    for (int c = 0; c < 3; ++c) PL::fwd(F[c], sbuf, p, tw, sidx, sync);
     if (INTEG != INT_TAB && !colok) return;
 
     T h = T(0);
