@@ -238,8 +238,28 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
     }
     const long long xs = (long long)N * G::NZP;
     C* sbuf = buf + (size_t)g * N * TT;
+    // the stage algebra's modes of this thread: rows r0 + it RPI, it < NIT, of the band's 2 KC + 1;
+    // their state is loaded CH rows at a time, before the transform where that is all of them
+    constexpr int RPI = NT / TT, NIT = (2 * G::KC + RPI) / RPI, CH = NIT < 2 ? 1 : 2;
+    constexpr bool needU = MODE <= X_STAGE4 && !(INTEG == INT_IFRK4 && MODE == X_STAGE4);
+    constexpr bool needA = MODE <= X_STAGE4 && MODE != X_STAGE1 && INTEG != INT_TAB;
+    const int r0 = threadIdx.x / TT, kz = kz0 + t, kp2 = ky * ky + kz * kz;
+    const double fkz = kz;
+    C us[CH][3], as[CH][3];
+    auto load_state = [&](int it, C (&u)[3], C (&a)[3]) {
+        const int r = r0 + it * RPI, kx = r - G::KC;
+        if (r > 2 * G::KC || kz > G::KC || kx * kx + kp2 > G::KC2) return;
+        const long long q = (long long)(kx < 0 ? kx + N : kx) * xs + (long long)j * G::NZP + kz;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (needU) u[c] = U[c * G::FS + q];
+            if (needA) a[c] = ACC[c * G::FS + q];
+        }
+    };
+    if (NIT <= CH)
+#pragma unroll
+        for (int q = 0; q < CH; ++q) load_state(q, us[q], as[q]);
     {
-        const int kz = kz0 + t;
         const bool colok = kz <= G::KC && ky * ky + kz * kz <= G::KC2;
         const cx<q64>* src = W + g * G::FS + (long long)j * G::NZP + kz;
         const int* kin = fx_scales<N>(scales, blockIdx.z).w + (long long)g * N * G::NZP + kz;
@@ -272,14 +292,17 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
     const double h = MODE <= X_STAGE4 ? sd->dt : 0.0;
     const double h2 = 0.5 * h, h3 = h * (1.0 / 3.0), h6 = h * (1.0 / 6.0);
     double es[3] = {0.0, 0.0, 0.0};   // DP5CN error partial sums
-    // rows |kx| <= KC of the tile, NT / TT rows at a time (NT is a multiple of TT)
-    const int kz = kz0 + t, kp2 = ky * ky + kz * kz;
-    const double fkz = kz;
-#pragma unroll 2
-    for (int r = threadIdx.x / TT; r < 2 * G::KC + 1; r += NT / TT) {
+#pragma unroll 1
+    for (int it0 = 0; it0 < NIT; it0 += CH) {
+      if (NIT > CH)
+#pragma unroll
+        for (int q = 0; q < CH; ++q) load_state(it0 + q, us[q], as[q]);
+#pragma unroll
+      for (int ch = 0; ch < CH; ++ch) {
+        const int r = r0 + (it0 + ch) * RPI;
         const int kx = r - G::KC, i = kx < 0 ? kx + N : kx;
         const int k2 = kx * kx + kp2;
-        if (kz > G::KC || k2 > G::KC2) continue;
+        if (r > 2 * G::KC || kz > G::KC || k2 > G::KC2) continue;
         const long long idx = (long long)i * xs + (long long)j * G::NZP + kz;
         C n[3];
 #pragma unroll
@@ -312,7 +335,7 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
                     }
                 }
                 if (rs.store >= 0) K[(long long)rs.store * 3 * G::FS + q] = n[c];
-                const C u = U[q];
+                const C u = us[ch][c];
                 if (rs.kind == 0) {
                     UT[q] = u + acc * h;
                 } else if (rs.kind == 1) {
@@ -334,14 +357,14 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
             for (int c = 0; c < 3; ++c) {
                 const long long q = c * G::FS + idx;
                 if (MODE == X_STAGE1) {
-                    const C u = U[q];
+                    const C u = us[ch][c];
                     UT[q] = (u + n[c] * h2) * Eh;
                     ACC[q] = (u + n[c] * h6) * Ef;
                 } else if (MODE == X_STAGE4) {
-                    U[q] = ACC[q] + n[c] * h6;
+                    U[q] = as[ch][c] + n[c] * h6;
                 } else {
-                    UT[q] = U[q] * (MODE == X_STAGE2 ? Eh : Ef) + n[c] * cu;
-                    ACC[q] = ACC[q] + n[c] * ca;
+                    UT[q] = us[ch][c] * (MODE == X_STAGE2 ? Eh : Ef) + n[c] * cu;
+                    ACC[q] = as[ch][c] + n[c] * ca;
                 }
             }
         } else {
@@ -350,13 +373,14 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
                 const long long q = c * G::FS + idx;
                 if (MODE == X_STAGE4) {
                     const C ab = ldg(&tab[k2]);
-                    U[q] = U[q] * ab.x + (ACC[q] + n[c] * (1.0 / 6.0)) * ab.y;
+                    U[q] = us[ch][c] * ab.x + (as[ch][c] + n[c] * (1.0 / 6.0)) * ab.y;
                 } else {
-                    UT[q] = U[q] + n[c] * (MODE == X_STAGE3 ? h : h2);
-                    ACC[q] = MODE == X_STAGE1 ? n[c] * (1.0 / 6.0) : ACC[q] + n[c] * (1.0 / 3.0);
+                    UT[q] = us[ch][c] + n[c] * (MODE == X_STAGE3 ? h : h2);
+                    ACC[q] = MODE == X_STAGE1 ? n[c] * (1.0 / 6.0) : as[ch][c] + n[c] * (1.0 / 3.0);
                 }
             }
         }
+      }
     }
     if constexpr (INTEG == INT_TAB) {
         if (rs.kind == 2) dp_block_sum<NT>(es, dpart);
