@@ -282,7 +282,7 @@ class Impl final : public Base {
     void set_xfwd_attr() {
         if constexpr (sizeof(T) == 8)
             cudaFuncSetAttribute(k_xfwd_fx<N, INTEG, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, fxfwd_smem<N>());
-        else
+        else if constexpr (N > kXfwdPreMax)   // below, the default limit does
             cudaFuncSetAttribute(k_xfwd<T, N, INTEG, MODE, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_x());
     }
     template <int INTEG>
@@ -394,10 +394,17 @@ class Impl final : public Base {
         if constexpr (sizeof(T) == 8)
             pass(k_xfwd_fx<N, INTEG, MODE>, grid, fxfwd_threads<N>(), fxfwd_smem<N>(), s_)(
                 Wq(m0), scales(m0), Um(m0), UTm(m0), acc, twq(), sdm(m0), tabm(m0), aux_, nullptr, nullptr, RkStage{});
-        else
-            pass(k_xfwd<T, N, INTEG, MODE, V>, grid, TXF * PX::P, smem_x(), s_)(
-                Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0), (les_ && MODE <= X_STAGE4) ? F_ : nullptr,
-                nullptr, nullptr, RkStage{});
+        else {
+            auto run = [&](auto kernel) {
+                pass(kernel, grid, TXF * PX::P, smem_x(), s_)(
+                    Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0), (les_ && MODE <= X_STAGE4) ? F_ : nullptr,
+                    nullptr, nullptr, RkStage{});
+            };
+            if constexpr (MODE <= X_STAGE4 && N <= kXfwdPreMax) {
+                if (xfwd_pre<N>(cnt)) return run(k_xfwd<T, N, INTEG, MODE, V, true>);
+            }
+            if constexpr (!(MODE <= X_STAGE4 && xfwd_pre<N>(1 << 30))) run(k_xfwd<T, N, INTEG, MODE, V>);
+        }
     }
     // RK5-family stage epilogue s (0-based) of members [m0, m0 + cnt)
     void p5tab(int s, int m0, int cnt) {

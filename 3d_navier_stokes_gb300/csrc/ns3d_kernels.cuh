@@ -1175,9 +1175,39 @@ __device__ __forceinline__ void xfwd_prefetch_state(const cx<T>* U, const cx<T>*
 // p + P s of the column (ky, kz) inside the sphere: the Leray projection of every
 // mode first, then, in chunks of up to 8 modes and per component, the chunk's
 // state loads before their updates, so that a chunk's loads (per array) are in
-// flight at once.
+// flight at once. With PRE the state of all modes was loaded before the transforms
+// (xfwd_load_state): on a small grid the pass is a chain of latencies, and the
+// registers are free (xfwd_pre).
+// Where the pass loads its state before the transforms: up to 64 points always, up to 128 with
+// at most four members. One RK4 step: 32^3 63.5 -> 57.3 us, 48^3 91 -> 76 us, 64^3 71.7 ->
+// 65.5 us, 96^3 159 -> 147 us, 128^3 203 -> 195 us (188 -> 184 us in variant 2); eight members
+// of 48^3 156 -> 141 us, of 96^3 778 -> 786 us, four 381 -> 380 us. 192^3 705 -> 702 us, 256^3
+// 1357 -> 1411 us.
+constexpr int kXfwdPreMax = 128;
+template <int N> constexpr bool xfwd_pre(int members) { return N <= 64 || (N <= kXfwdPreMax && members <= 4); }
+template <int INTEG, int MODE> constexpr bool xfwd_need_u() { return !(INTEG == INT_IFRK4 && MODE == X_STAGE4); }
+template <int INTEG, int MODE> constexpr bool xfwd_need_a() { return MODE != X_STAGE1; }
 template <typename T, int N, int INTEG, int MODE, int E, int P>
-__device__ __forceinline__ void xfwd_rk4_epilogue(cx<T> (&F)[3][E], int p, int ky, int kz, long long off,
+__device__ __forceinline__ void xfwd_load_state(cx<T> (&u)[3][E], cx<T> (&a)[3][E], int p, bool colok, int rem,
+                                                long long off, const cx<T>* __restrict__ U,
+                                                const cx<T>* __restrict__ ACC) {
+    using G = Geo<N>;
+    const long long xs = (long long)N * G::NZP;
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+        const int kx = kof<N>(p + P * s);
+        const bool in = colok && kx * kx <= rem;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const long long q = c * G::FS + (long long)(p + P * s) * xs + off;
+            u[c][s] = a[c][s] = czero<T>();
+            if (xfwd_need_u<INTEG, MODE>() && in) u[c][s] = U[q];
+            if (xfwd_need_a<INTEG, MODE>() && in) a[c][s] = ACC[q];
+        }
+    }
+}
+template <bool PRE, typename T, int N, int INTEG, int MODE, int E, int P, int EP>
+__device__ __forceinline__ void xfwd_rk4_epilogue(cx<T> (&F)[3][E], const cx<T> (&pu)[3][EP], const cx<T> (&pa)[3][EP], int p, int ky, int kz, long long off,
                                                   cx<T>* __restrict__ U, cx<T>* __restrict__ UT,
                                                   cx<T>* __restrict__ ACC, const cx<T>* __restrict__ tab,
                                                   const StepDev* __restrict__ sd, const cx<T>* __restrict__ sgs, T h) {
@@ -1218,8 +1248,7 @@ __device__ __forceinline__ void xfwd_rk4_epilogue(cx<T> (&F)[3][E], int p, int k
         k2s[s] = k2;
     }
     constexpr bool kIF = INTEG == INT_IFRK4;
-    constexpr bool needU = !(kIF && MODE == X_STAGE4);
-    constexpr bool needA = kIF ? (MODE != X_STAGE1) : (MODE != X_STAGE1);
+    constexpr bool needU = xfwd_need_u<INTEG, MODE>() && !PRE, needA = xfwd_need_a<INTEG, MODE>() && !PRE;
 #pragma unroll
     for (int s0 = 0; s0 < E; s0 += CH) {
       if (!((valid >> s0) & ((1u << CH) - 1u))) continue;
@@ -1231,8 +1260,8 @@ __device__ __forceinline__ void xfwd_rk4_epilogue(cx<T> (&F)[3][E], int p, int k
         cx<T> u[CH], a[CH];
 #pragma unroll
         for (int s = 0; s < CH; ++s) {
-            u[s] = czero<T>();
-            a[s] = czero<T>();
+            u[s] = PRE ? pu[c][PRE ? s0 + s : 0] : czero<T>();
+            a[s] = PRE ? pa[c][PRE ? s0 + s : 0] : czero<T>();
             if (!((valid >> (s0 + s)) & 1u)) continue;
             const long long q = c * G::FS + (long long)(p + P * (s0 + s)) * xs + off;
             if (needU) u[s] = U[q];
@@ -1309,7 +1338,7 @@ __device__ __forceinline__ void dp_block_sum(const double (&es)[3], double* __re
 // T. INTEG = INT_TAB runs the RkStage epilogue of the RK5 family; its DP5CN
 // error partial sums go to dpart[member][block][3] in a fixed order.
 // ---------------------------------------------------------------------------
-template <typename T, int N, int INTEG, int MODE, int V = 0>
+template <typename T, int N, int INTEG, int MODE, int V = 0, bool PRE = false>
 __global__ void __launch_bounds__(tile_x<T, N, V, true>() * PlansV<N, V>::X::P, TileVar<V>::MINB)
 k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ UT,
        cx<T>* __restrict__ ACC, const cx<T>* __restrict__ tw, const StepDev* __restrict__ sd,
@@ -1367,16 +1396,20 @@ k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ U
 #pragma unroll
         for (int s = 0; s < E; ++s) F[c][s] = colok ? src[(long long)(p + P * s) * xs] : czero<T>();
     }
-    xfwd_prefetch_state<T, N, INTEG, MODE, E, P, TT>(U, ACC, K, rs, p, t, ky, kz0, j);
+    const int rem = G::KC2 - ky * ky - kz * kz;
+    constexpr bool kBatch = (INTEG == INT_IFRK4 || INTEG == INT_RK4CN) && MODE <= X_STAGE4 && TileVar<V>::BATCH;
+    constexpr bool kPre = kBatch && PRE;
+    cx<T> pu[3][kPre ? E : 1], pa[3][kPre ? E : 1];
+    if constexpr (kPre) xfwd_load_state<T, N, INTEG, MODE, E, P>(pu, pa, p, colok, rem, off, U, ACC);
+    else xfwd_prefetch_state<T, N, INTEG, MODE, E, P, TT>(U, ACC, K, rs, p, t, ky, kz0, j);
 #pragma unroll
     for (int c = 0; c < 3; ++c) PL::fwd(F[c], sbuf, p, tw, sidx, sync);
     if (INTEG != INT_TAB && !colok) return;
 
     T h = T(0);
     if (MODE <= X_STAGE4) h = T(sd->dt);
-    const int rem = G::KC2 - ky * ky - kz * kz;
-    if constexpr ((INTEG == INT_IFRK4 || INTEG == INT_RK4CN) && MODE <= X_STAGE4 && TileVar<V>::BATCH) {
-        xfwd_rk4_epilogue<T, N, INTEG, MODE, E, P>(F, p, ky, kz, off, U, UT, ACC, tab, sd, sgs, h);
+    if constexpr (kBatch) {
+        xfwd_rk4_epilogue<kPre, T, N, INTEG, MODE, E, P>(F, pu, pa, p, ky, kz, off, U, UT, ACC, tab, sd, sgs, h);
         return;
     }
     double es[3] = {0.0, 0.0, 0.0};   // DP5CN error partial sums
