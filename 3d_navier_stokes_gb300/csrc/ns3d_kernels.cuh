@@ -148,20 +148,23 @@ struct SyncBlock {
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
 // Exchange slot of element m of pencil t: [m'][TT] with the row m' = m XOR
-// ((m / R1) mod G), G = 32 / TT pencil groups per warp (G < R1, power-of-two
-// R1; identity otherwise). The first stage's writes of a warp's G groups go
+// ((m / R1) mod G), G = 32 / TT pencil groups per warp (mod 2 where G does not divide
+// R1; identity for odd R1 and G > R1). The first stage's writes of a warp's G groups go
 // to rows R1 apart (R1 * TT complex, a multiple of 128 bytes) and would share
 // one bank range; the XOR spreads them over the banks. The reads of
 // consecutive rows stay consecutive (a permutation inside each aligned block
-// of R1 rows), so neither side has bank conflicts.
+// of R1 rows), so neither side has bank conflicts. (Radix 12, 96^3 inverse y pass:
+// 10.2 -> 9.6 us.)
 template <int TT, int R1 = 1>
 struct StridedIdx {
     static constexpr int G = TT < 16 ? 32 / TT : 1;
-    static constexpr bool kSwz = G > 1 && (R1 & (R1 - 1)) == 0 && R1 >= G;
+    static constexpr bool kPow2 = (R1 & (R1 - 1)) == 0;
+    static constexpr bool kSwz = G > 1 && (kPow2 ? R1 >= G : SWZ && R1 % 2 == 0);
+    static constexpr int kMask = kPow2 || R1 % G == 0 ? G - 1 : 1;
     static constexpr int kShift = (R1 >= 16) ? 4 : (R1 >= 8) ? 3 : (R1 >= 4) ? 2 : (R1 >= 2) ? 1 : 0;
     int t;
     __device__ __forceinline__ int operator()(int m) const {
-        if constexpr (kSwz) m ^= (m >> kShift) & (G - 1);
+        if constexpr (kSwz) m ^= (kPow2 ? m >> kShift : m / R1) & kMask;
         return m * TT + t;
     }
 };
@@ -885,6 +888,37 @@ constexpr int ZLINE_WARPS = 4;
 // (8 x 8 x 3: 0.083 -> 0.095 ms) or 96 points (eight members, 8 x 12: 0.091 -> 0.141 ms).
 template <int N> struct ZPlan { using A = typename Plans<N>::A; };
 template <> struct ZPlan<384> { using A = Plan<384, 24, 8, 8, 6>; };
+// Shared-memory layout of a warp's line groups, 8-byte elements, 16 lanes (one wavefront)
+// at a time. The exchange slot of element m is m + (m >> A) B or m XOR ((m >> A) & MASK),
+// one line LP slots after the other; the input rows of a line are LS elements apart. The
+// values are those with the fewest bank conflicts over a plan's stage writes and reads
+// (counted; 1.0 is none): with one pad slot per 16 and unpadded lines 24 .. 96 points had
+// 1.6 - 2.0 wavefronts per access and 192 points 1.7 (96 points, eight members: LSU pipe
+// 84 % busy), now 1.04 - 1.08 and 1.27. Per launch: 96 points, eight members 0.0905 ->
+// 0.0711 ms, 48 points 0.0186 -> 0.0155 ms, 192 points 0.083 -> 0.071 ms, 512 points 1.166
+// -> 1.137 ms. The XOR forms count 1.04 at 96, 192 and 384 points too, but their address
+// arithmetic costs more there (0.087, 0.086 and 0.87 ms).
+template <int A, int B> struct PadIdx {
+    __device__ __forceinline__ int operator()(int m) const { return m + (m >> A) * B; }
+};
+template <int A, int MASK> struct XorIdx {
+    __device__ __forceinline__ int operator()(int m) const { return m ^ ((m >> A) & MASK); }
+};
+// default: one pad slot per 16; single-lane lines an odd number of slots apart
+template <int N> struct ZLay { using Idx = PadIdx<4, 1>; static constexpr int LP = N <= 16 ? zpad<N>() | 1 : zpad<N>(); };
+template <> struct ZLay<24> { using Idx = PadIdx<2, 1>; static constexpr int LP = 30; };
+template <> struct ZLay<32> { using Idx = PadIdx<2, 1>; static constexpr int LP = 44; };
+template <> struct ZLay<48> { using Idx = PadIdx<2, 1>; static constexpr int LP = 60; };
+template <> struct ZLay<64> { using Idx = PadIdx<3, 1>; static constexpr int LP = 72; };
+template <> struct ZLay<96> { using Idx = PadIdx<3, 1>; static constexpr int LP = 120; };
+template <> struct ZLay<192> { using Idx = PadIdx<4, 3>; static constexpr int LP = 228; };
+template <> struct ZLay<512> { using Idx = XorIdx<3, 15>; static constexpr int LP = 512; };
+template <int N> constexpr int zline_lp() { return ZLay<N>::LP; }
+// the lines of a wavefront P elements apart in the banks (an even number: bulk copies)
+template <int N> constexpr int zline_ls() {
+    constexpr int P = ZPlan<N>::A::P;
+    return 6 * Geo<N>::NZP + (P < 16 ? (P < 2 ? 2 : P) : 0);
+}
 template <int N> constexpr int zline_gw() { return ZPlan<N>::A::P > 32 ? ZPlan<N>::A::P / 32 : 1; }
 template <int N> constexpr int zline_gpw() { return ZPlan<N>::A::P <= 32 ? 32 / ZPlan<N>::A::P : 1; }
 // the real Nz line as a half-length complex transform (a plan of N/2 points on the
@@ -913,13 +947,13 @@ constexpr bool zline_ok() {
 template <int N> constexpr bool zline_xbuf_in_stage() { return zline_gpw<N>() > 1; }
 template <int N> constexpr int zline_minb() { return zline_xbuf_in_stage<N>() && ZPlan<N>::A::E <= 16 ? 3 : 2; }
 template <int N> constexpr int zline_stage_elems() {
-    constexpr int a = zline_gpw<N>() * 6 * Geo<N>::NZP, b = zline_gpw<N>() * zpad<N>();
+    constexpr int a = zline_gpw<N>() * zline_ls<N>(), b = zline_gpw<N>() * zline_lp<N>();
     return ((zline_xbuf_in_stage<N>() && b > a ? b : a) + 15) / 16 * 16;
 }
 // complex elements of shared memory per line group: two stage buffers (+ the exchange buffers)
 template <typename T, int N> constexpr int zline_group_elems() {
     return 2 * zline_stage_elems<N>() +
-           (zline_xbuf_in_stage<N>() ? 0 : (zline_gpw<N>() * zpad<N>() + 15) / 16 * 16);
+           (zline_xbuf_in_stage<N>() ? 0 : (zline_gpw<N>() * zline_lp<N>() + 15) / 16 * 16);
 }
 // line groups per CTA
 template <int N> constexpr int zline_groups() { return ZLINE_WARPS / zline_gw<N>(); }
@@ -958,7 +992,7 @@ k_zline(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, StepDev* __restrict
     uint64_t* bars_all = reinterpret_cast<uint64_t*>(smem_raw + sizeof(cx<T>) * (size_t)NGRP * zline_group_elems<T, N>());
     uint64_t* bars = bars_all + 2 * grp;
     int* votes = reinterpret_cast<int*>(bars_all + 2 * NGRP) + grp * GW;   // one word per warp of the group
-    PaddedIdx sidx;
+    typename ZLay<N>::Idx sidx;
     using Sync = typename std::conditional<(GW > 1), SyncGroup, SyncWarp>::type;
     Sync sync{};
     if constexpr (GW > 1) sync = Sync{1 + grp, GT};
@@ -976,7 +1010,7 @@ k_zline(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, StepDev* __restrict
             const long long m = g / NG, gl = g % NG;
             for (int l = 0; l < GPW; ++l)
                 for (int f = 0; f < 6; ++f)
-                    bulk_g2s(stage[s] + (l * 6 + f) * NZP, W + (m * 6 + f) * G::FS + (gl * GPW + l) * NZP,
+                    bulk_g2s(stage[s] + l * zline_ls<N>() + f * NZP, W + (m * 6 + f) * G::FS + (gl * GPW + l) * NZP,
                              LINE_BYTES, &bars[s]);
         }
     };
@@ -1026,10 +1060,10 @@ k_zline(cx<T>* __restrict__ W, const cx<T>* __restrict__ tw, StepDev* __restrict
             cur = mem;
         }
         cx<T>* Wm = W + mem * 6 * G::FS;
-        const cx<T>* in = stage[s] + gi * 6 * NZP;
+        const cx<T>* in = stage[s] + gi * zline_ls<N>();
         const long long line = (g % NG) * GPW + gi;
         // exchange buffer of this group (in the stage buffer once its lines are in registers)
-        cx<T>* sb = (zline_xbuf_in_stage<N>() ? stage[s] : wbase + 2 * SE) + gi * zpad<N>();
+        cx<T>* sb = (zline_xbuf_in_stage<N>() ? stage[s] : wbase + 2 * SE) + gi * zline_lp<N>();
 
         auto load_pair = [&](int f, cx<T>(&v)[E]) {
             const cx<T>* A = in + f * NZP;
