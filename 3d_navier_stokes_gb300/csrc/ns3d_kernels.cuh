@@ -159,7 +159,7 @@ template <int TT, int R1 = 1>
 struct StridedIdx {
     static constexpr int G = TT < 16 ? 32 / TT : 1;
     static constexpr bool kPow2 = (R1 & (R1 - 1)) == 0;
-    static constexpr bool kSwz = G > 1 && (kPow2 ? R1 >= G : SWZ && R1 % 2 == 0);
+    static constexpr bool kSwz = G > 1 && (kPow2 ? R1 >= G : R1 % 2 == 0);
     static constexpr int kMask = kPow2 || R1 % G == 0 ? G - 1 : 1;
     static constexpr int kShift = (R1 >= 16) ? 4 : (R1 >= 8) ? 3 : (R1 >= 4) ? 2 : (R1 >= 2) ? 1 : 0;
     int t;
