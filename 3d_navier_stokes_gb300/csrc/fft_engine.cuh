@@ -325,6 +325,7 @@ struct Plan {
     static constexpr int P = N_ / E_;
     static constexpr int nstages = sizeof...(Rs);
     static constexpr int R1 = FirstOf<Rs...>::value;   // radix of the first stage
+    static_assert((Rs * ... * 1) == N_ && N_ % E_ == 0, "the radices' product is the length");
     // PK: FP32x2 additions in the butterflies (see vadd); TS: twiddle table of a
     // TS times longer transform
     template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync>

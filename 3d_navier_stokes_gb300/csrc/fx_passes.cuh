@@ -22,13 +22,12 @@ template <int N> __device__ __forceinline__ FxScales fx_scales(int* base, long l
 }
 
 // ---------------------------------------------------------------------------
-// x passes: the z lines' plan (16 elements per thread where N allows, one or two
-// exchanges), fx_tile pencils per CTA. `aux` holds 1/k2 for k2 <= KC^2 (0 at 0) and
+// x passes, on FxPlan<N>::X, fx_tile pencils per CTA. `aux` holds 1/k2 for k2 <= KC^2 (0 at 0) and
 // then the N wavenumbers of the x rows, so that no mode pays an FP64 division or
 // conversion.
 // ---------------------------------------------------------------------------
-template <int N> constexpr int fxinv_threads() { return fx_tile<N>() * Plans<N>::A::P; }
-template <int N> constexpr int fxfwd_threads() { return 3 * fx_tile<N, true>() * Plans<N>::A::P; }
+template <int N> constexpr int fxinv_threads() { return fx_tile<N>() * FxPlan<N>::X::P; }
+template <int N> constexpr int fxfwd_threads() { return 3 * fx_tile<N, true>() * FxPlan<N>::X::P; }
 constexpr int fx_log2(int n) { return n <= 1 ? 0 : 1 + fx_log2(n / 2); }
 constexpr int fx_ctas(int per_sm, int threads) { return per_sm / threads < 1 ? 1 : per_sm / threads; }
 // CTAs per SM the passes are compiled for. Inverse: 640 threads (96 registers) from 16
@@ -36,7 +35,7 @@ constexpr int fx_ctas(int per_sm, int threads) { return per_sm / threads < 1 ? 1
 // Forward: two CTAs of 384 threads or one of 768 (80 registers, a few spills, but one
 // CTA's transforms under the other's FP64 work: 256^3 0.208 -> 0.166 ms, 512^3 1.96 ->
 // 1.51 ms), 576 threads with smaller CTAs (128^3 0.0395 -> 0.0343 ms, 0.0411 with 768).
-template <int N> constexpr int fxinv_ctas() { return fx_ctas(Plans<N>::A::P >= 16 ? 640 : 512, fxinv_threads<N>()); }
+template <int N> constexpr int fxinv_ctas() { return fx_ctas(FxPlan<N>::X::P >= 16 ? 640 : 512, fxinv_threads<N>()); }
 template <int N> constexpr int fxfwd_ctas() { return fx_ctas(fxfwd_threads<N>() >= 384 ? 768 : 576, fxfwd_threads<N>()); }
 template <int N> constexpr int fxinv_smem() { return N * fx_tile<N>() * 16; }
 template <int N> constexpr int fxfwd_smem() { return 3 * N * fx_tile<N, true>() * 16; }
@@ -56,7 +55,7 @@ k_xinv_fx(const cx<double>* __restrict__ U, cx<q64>* __restrict__ W, int* __rest
     W += dep;
     scales += dep;
     using G = Geo<N>;
-    using PL = typename Plans<N>::A;
+    using PL = typename FxPlan<N>::X;
     constexpr int TT = fx_tile<N>(), E = PL::E, P = PL::P, NT = TT * P;
     constexpr bool kPow2 = (N & (N - 1)) == 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -126,11 +125,11 @@ k_xinv_fx(const cx<double>* __restrict__ U, cx<q64>* __restrict__ W, int* __rest
 
 // P2 / P4: FFT along y in place, grid and masks of k_ypass; the elements of a line come
 // with scales of their own (per ky after P1, per y after P3).
-template <int N> constexpr int fxy_tile() { return Plans<N>::A::P * 8 <= 512 ? 8 : 4; }
-template <int N> constexpr int fxy_threads() { return fxy_tile<N>() * Plans<N>::A::P; }
+template <int N> constexpr int fxy_tile() { return FxPlan<N>::A::P * 8 <= 512 ? 8 : 4; }
+template <int N> constexpr int fxy_threads() { return fxy_tile<N>() * FxPlan<N>::A::P; }
 // 512 threads per SM (128 registers); 640 with at most 12 elements per thread (192^3 0.118 ->
 // 0.114 ms; 256^3, 16 elements: 0.201 against 0.207 ms)
-template <int N> constexpr int fxy_ctas() { return fx_ctas(Plans<N>::A::E <= 12 ? 640 : 512, fxy_threads<N>()); }
+template <int N> constexpr int fxy_ctas() { return fx_ctas(FxPlan<N>::A::E <= 12 ? 640 : 512, fxy_threads<N>()); }
 template <int N, bool INV>
 __global__ void __launch_bounds__(fxy_threads<N>(), fxy_ctas<N>())
 k_ypass_fx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict__ tw) {
@@ -138,7 +137,7 @@ k_ypass_fx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __rest
     W += dep;
     scales += dep;
     using G = Geo<N>;
-    using PL = typename Plans<N>::A;
+    using PL = typename FxPlan<N>::A;
     constexpr int TT = fxy_tile<N>(), E = PL::E, P = PL::P, NT = TT * P;
     constexpr int NF = INV ? 6 : 3;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -209,7 +208,7 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
     K += dep;
     dpart += dep;
     using G = Geo<N>;
-    using PL = typename Plans<N>::A;
+    using PL = typename FxPlan<N>::X;
     using C = cx<double>;
     constexpr int TT = fx_tile<N, true>(), E = PL::E, P = PL::P, NG = TT * P, NT = 3 * NG;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -403,10 +402,19 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 // issue bound (49 % of slots, instruction fetch the largest stall: CTAs of 192 and 384
 // threads, whose warps run in step, measured 0.64 and 0.73 ms).
 // ---------------------------------------------------------------------------
+// Exchange slots of a line, 16-byte elements, 8 lanes (one wavefront) at a time: m + (m >> A),
+// lines XS slots apart. One pad slot per 16 counts 2.0 - 2.1 wavefronts per access at 8, 24 and
+// 48 points and 1.33 at 64, these 1.2 and 1.0; at 96 and 192 points (1.4 to 1.2) nothing was
+// gained.
+template <int N> struct FxLay { static constexpr int A = 4, XS = zpad<N>(); };
+template <> struct FxLay<8> { static constexpr int A = 2, XS = 12; };
+template <> struct FxLay<24> { static constexpr int A = 4, XS = 28; };
+template <> struct FxLay<48> { static constexpr int A = 2, XS = 60; };
+template <> struct FxLay<64> { static constexpr int A = 3, XS = 72; };
 // line pairs per CTA (>= 96 threads)
-template <int N> constexpr int zfx_pairs() { return (95 + 3 * Plans<N>::A::P) / (3 * Plans<N>::A::P); }
-template <int N> constexpr int zfx_smem() { return zfx_pairs<N>() * 6 * zpad<N>() * 16; }
-template <int N> constexpr int zfx_threads() { return 3 * Plans<N>::A::P * zfx_pairs<N>(); }
+template <int N> constexpr int zfx_pairs() { return (95 + 3 * FxPlan<N>::A::P) / (3 * FxPlan<N>::A::P); }
+template <int N> constexpr int zfx_smem() { return zfx_pairs<N>() * 6 * FxLay<N>::XS * 16; }
+template <int N> constexpr int zfx_threads() { return 3 * FxPlan<N>::A::P * zfx_pairs<N>(); }
 constexpr int zfx_fit(int by_regs, int by_smem) { return by_regs < by_smem ? (by_regs < 1 ? 1 : by_regs) : by_smem; }
 // CTAs per SM: 384 threads (168 registers each) or what the buffers allow
 template <int N> constexpr int zfx_minb() { return zfx_fit(384 / zfx_threads<N>(), 227 * 1024 / (zfx_smem<N>() + 2048)); }
@@ -440,8 +448,8 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
     real += dep;
     sd += dep;
     using G = Geo<N>;
-    using PL = typename Plans<N>::A;
-    constexpr int E = PL::E, P = PL::P, ZP = zfx_pairs<N>(), XS = zpad<N>();
+    using PL = typename FxPlan<N>::A;
+    constexpr int E = PL::E, P = PL::P, ZP = zfx_pairs<N>(), XS = FxLay<N>::XS;
     constexpr int NW = P > 32 ? P / 32 : 1;    // warps per line
     constexpr int NLOW = (G::KC + P) / P;      // slots s that can hold a mode p + P s <= KC
     W += (long long)blockIdx.y * 6 * G::FS;    // ensemble member
@@ -455,7 +463,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
     const int lp = threadIdx.x / (3 * P);
     const long long la = 2 * ((long long)blockIdx.x * ZP + lp);
     const FxScales sc = fx_scales<N>(scales, blockIdx.y);
-    PaddedIdx sidx;
+    PadIdx<FxLay<N>::A, 1> sidx;
     SyncLine<P> sync;
 
     int kA = 0, kB = 0;   // scales of what a group writes

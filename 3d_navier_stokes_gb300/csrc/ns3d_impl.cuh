@@ -295,6 +295,13 @@ class Impl final : public Base {
         set_xfwd_attr<INTEG, X_PLAIN>();
     }
 
+    // run(true) where the FP32 x passes have smaller tiles for launches of cnt members, else run(false)
+    template <class F> static void x_sized(int cnt, F&& run) {
+        if constexpr (x_small<N, V>(1)) {
+            if (x_small<N, V>(cnt)) return run(std::true_type{});
+        }
+        run(std::false_type{});
+    }
     // each launcher covers members [m0, m0 + cnt); `in` points at member 0's arrays
     void p1(const cx<T>* in, int m0, int cnt) {
         if constexpr (xinv_tma_ok<T, N, V>()) {
@@ -312,7 +319,12 @@ class Impl final : public Base {
         if constexpr (sizeof(T) == 8)
             pass(k_xinv_fx<N>, dim3(NTX, G::NKY, 6 * cnt), fxinv_threads<N>(), fxinv_smem<N>(), s_)(src, Wq(m0), scales(m0), twq(), aux_);
         else
-            pass(k_xinv<T, N, V>, dim3(NTX, G::NKY, cnt), TX * PX::P, smem_xi(), s_)(src, Wm(m0), tw_);
+            x_sized(cnt, [&](auto small) {
+                constexpr bool S = small;
+                constexpr int TT = tile_x<T, N, V, false, S>();
+                pass(k_xinv<T, N, V, S>, dim3((G::NZ1 + TT - 1) / TT, G::NKY, cnt), TT * PX::P,
+                     xinv_smem<T, N, V, S>(), s_)(src, Wm(m0), tw_);
+            });
     }
     void p2(int m0, int cnt) {
         if constexpr (sizeof(T) == 8)
@@ -395,15 +407,20 @@ class Impl final : public Base {
             pass(k_xfwd_fx<N, INTEG, MODE>, grid, fxfwd_threads<N>(), fxfwd_smem<N>(), s_)(
                 Wq(m0), scales(m0), Um(m0), UTm(m0), acc, twq(), sdm(m0), tabm(m0), aux_, nullptr, nullptr, RkStage{});
         else {
-            auto run = [&](auto kernel) {
-                pass(kernel, grid, TXF * PX::P, smem_x(), s_)(
-                    Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0), (les_ && MODE <= X_STAGE4) ? F_ : nullptr,
-                    nullptr, nullptr, RkStage{});
+            auto run = [&](auto kernel, int tile) {
+                pass(kernel, dim3((G::NZ1 + tile - 1) / tile, G::NKY, cnt), tile * PX::P,
+                     sizeof(cx<T>) * (size_t)N * tile, s_)(Wm(m0), Um(m0), UTm(m0), acc, tw_, sdm(m0), tabm(m0),
+                                                           (les_ && MODE <= X_STAGE4) ? F_ : nullptr, nullptr, nullptr,
+                                                           RkStage{});
             };
-            if constexpr (MODE <= X_STAGE4 && N <= kXfwdPreMax) {
-                if (xfwd_pre<N>(cnt)) return run(k_xfwd<T, N, INTEG, MODE, V, true>);
+            if constexpr (MODE <= X_STAGE4 && x_small<N, V>(1)) {
+                if (x_small<N, V>(cnt))
+                    return run(k_xfwd<T, N, INTEG, MODE, V, true, true>, tile_x<T, N, V, true, true>());
             }
-            if constexpr (!(MODE <= X_STAGE4 && xfwd_pre<N>(1 << 30))) run(k_xfwd<T, N, INTEG, MODE, V>);
+            if constexpr (MODE <= X_STAGE4 && N <= kXfwdPreMax) {
+                if (xfwd_pre<N>(cnt)) return run(k_xfwd<T, N, INTEG, MODE, V, true>, TXF);
+            }
+            if constexpr (!(MODE <= X_STAGE4 && xfwd_pre<N>(1 << 30))) run(k_xfwd<T, N, INTEG, MODE, V>, TXF);
         }
     }
     // RK5-family stage epilogue s (0-based) of members [m0, m0 + cnt)

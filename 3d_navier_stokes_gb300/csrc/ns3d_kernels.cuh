@@ -52,13 +52,23 @@ struct Geo {
 // wavenumber of storage index i (InitializeSpaceVariables, solver.c:1786-1812)
 template <int N> __device__ __forceinline__ int kof(int i) { return i <= N / 2 ? i : i - N; }
 
+// A: plan of the y and z lines, X: of the x lines (FP32). Grids of up to 64 points are chains
+// of latencies on a part-empty chip, where fewer elements per thread make shorter chains: one
+// RK4 step of 16^3 88 -> 43 us, 24^3 74 -> 53 us, 32^3 55 -> 49 us, 48^3 74 -> 65 us, 64^3 63.5
+// -> 55.3 us (eight members 176 -> 170, 24 members 528 -> 515 us). The y and z lines of 32 ..
+// 64 points keep 8 and 12 elements: with 4, 6 and 4 one member of 32^3 and 48^3 would gain (49
+// -> 45, 63 -> 59 us), eight lose (63 -> 70, 127 -> 168, 64^3 174 -> 248 us), and the plan is
+// the same for all, so that a member of an ensemble equals a single run. Small radices stand
+// first where that costs nothing: their twiddles are exact or few. Error of the right-hand side
+// of white fields against FP64, 16 .. 64 points: 2.12, 3.01, 2.87, 4.07, 4.36e-7 -> 2.03, 2.81,
+// 2.89, 4.05, 4.38e-7. (8 points keep one codelet: 2 x 4 would take 1.25e-7, not 1.14e-7.)
 template <int N> struct Plans;
 template <> struct Plans<8>    { using A = Plan<8, 8, 8>;            using X = A; };
-template <> struct Plans<16>   { using A = Plan<16, 16, 16>;         using X = A; };
-template <> struct Plans<24>   { using A = Plan<24, 12, 12, 2>;      using X = A; };
-template <> struct Plans<32>   { using A = Plan<32, 8, 4, 8>;        using X = A; };
-template <> struct Plans<48>   { using A = Plan<48, 12, 4, 12>;     using X = A; };
-template <> struct Plans<64>   { using A = Plan<64, 8, 8, 8>;        using X = A; };
+template <> struct Plans<16>   { using A = Plan<16, 4, 4, 4>;        using X = A; };
+template <> struct Plans<24>   { using A = Plan<24, 6, 2, 2, 6>;     using X = A; };
+template <> struct Plans<32>   { using A = Plan<32, 8, 4, 8>;        using X = Plan<32, 4, 4, 2, 4>; };
+template <> struct Plans<48>   { using A = Plan<48, 12, 4, 12>;      using X = Plan<48, 6, 2, 2, 2, 6>; };
+template <> struct Plans<64>   { using A = Plan<64, 8, 8, 8>;        using X = Plan<64, 4, 4, 4, 4>; };
 template <> struct Plans<96>   { using A = Plan<96, 12, 4, 4, 6>;    using X = A; };
 template <> struct Plans<128>  { using A = Plan<128, 16, 16, 8>;     using X = Plan<128, 8, 8, 4, 4>; };
 template <> struct Plans<256>  { using A = Plan<256, 16, 16, 16>;    using X = Plan<256, 8, 8, 8, 4>; };
@@ -68,6 +78,21 @@ template <> struct Plans<1024> { using A = Plan<1024, 16, 16, 16, 4>; using X = 
 template <> struct Plans<192>  { using A = Plan<192, 12, 4, 4, 12>;    using X = A; };
 template <> struct Plans<384>  { using A = Plan<384, 12, 4, 4, 4, 6>;  using X = A; };
 template <> struct Plans<768>  { using A = Plan<768, 12, 4, 4, 4, 4, 3>; using X = A; };
+
+// Plans of the FP64 engines' integer transforms (fxfft.cuh), A: y and z lines, X: x lines. Short
+// chains on small grids, as above: one RK4 step of 8^3 78 -> 51 us, 16^3 127 -> 57 us, 24^3 131
+// -> 92 us, 32^3 97 -> 74 us (six members 123 -> 123, sixteen 201 -> 231 us), 48^3 147 -> 125
+// us (sixteen 656 -> 668 us; with 6 elements in the y and z lines too 121 and 831 us), 64^3 131
+// -> 121 us (eight 577 -> 583 us; y and z lines too: 141 us). 96 and 128 points: 6 and 8
+// elements in the x lines gave nothing (375 and 632 us). 512 points: 16 x 8 x 4 has fewer
+// twiddle products than 8 x 8 x 8 (45.9 -> 44.8 ms).
+template <int N> struct FxPlan { using A = typename Plans<N>::A; using X = A; };
+template <> struct FxPlan<8>   { using A = Plan<8, 2, 2, 2, 2>;      using X = A; };
+template <> struct FxPlan<16>  { using A = Plan<16, 2, 2, 2, 2, 2>; using X = A; };
+template <> struct FxPlan<32>  { using A = Plan<32, 4, 4, 2, 4>;    using X = A; };
+template <> struct FxPlan<48>  { using A = Plans<48>::A;            using X = Plan<48, 6, 2, 2, 2, 6>; };
+template <> struct FxPlan<64>  { using A = Plans<64>::A;            using X = Plan<64, 4, 4, 4, 4>; };
+template <> struct FxPlan<512> { using A = Plan<512, 16, 16, 8, 4>; using X = A; };
 
 // Tile width (pencils per CTA along kz) of the strided passes: one 128-byte
 // row segment per pencil row where the thread count allows. Variant V of the
@@ -111,6 +136,7 @@ template <> struct TileVar<6> { static constexpr int A = 16, AF = 16, X = 8, XF 
 // 0.155 -> 0.145-0.148 ms per launch for 24 members; the forward pass measured slower
 // with it (0.058 -> 0.060 ms). The z lines hold three fields per line and keep 12.
 template <typename T, int N, bool INV> struct YPlan { using A = typename Plans<N>::A; };
+template <int N, bool INV> struct YPlan<double, N, INV> { using A = typename FxPlan<N>::A; };
 template <> struct YPlan<float, 96, true> { using A = Plan<96, 24, 12, 8>; };
 // 384 points in FP32: 24 elements and one stage less in both directions (inverse 0.308 ->
 // 0.286, forward 0.143 -> 0.129 ms; even at 192)
@@ -130,14 +156,28 @@ template <typename T, int N, int V = 0, bool INV = true> constexpr int tile_a() 
     return sizeof(T) == 4 ? clip_tile<YPlan<T, N, INV>::A::P, (INV ? TileVar<V>::A : TileVar<V>::AF)>()
                           : (YPlan<T, N, INV>::A::P * 8 <= 512 ? 8 : 4);
 }
-// FP64 x passes (fx_passes.cuh), on the z lines' plan: pencils per CTA. Inverse (one
+// FP64 x passes (fx_passes.cuh): pencils per CTA. Inverse (one
 // field per CTA): 8, or 4 where that makes more than 256 threads. Forward (three groups
 // of threads): 8 up to 384 threads (256^3: 0.212 ms per launch, 0.250 with 4 pencils and
 // two CTAs per SM), else 4.
-template <int N, bool FWD = false> constexpr int fx_tile() { return Plans<N>::A::P * 8 <= (FWD ? 128 : 256) ? 8 : 4; }
-template <typename T, int N, int V = 0, bool FWD = false> constexpr int tile_x() {
+template <int N, bool FWD = false> constexpr int fx_tile() { return FxPlan<N>::X::P * 8 <= (FWD ? 128 : 256) ? 8 : 4; }
+// FP32: at most 128 threads per CTA up to 64 points (64^3, tiles of 16 -> 8 pencils: 61.4 ->
+// 55.3 us per step), 8 pencils with S.
+template <typename T, int N, int V = 0, bool FWD = false, bool S = false> constexpr int tile_x() {
     if constexpr (sizeof(T) == 8) return fx_tile<N, FWD>();
-    else return clip_tile<PlansV<N, V>::X::P, (FWD ? TileVar<V>::XF : TileVar<V>::X)>();
+    else {
+        constexpr int P = PlansV<N, V>::X::P;
+        constexpr int W = clip_tile<P, (FWD ? TileVar<V>::XF : TileVar<V>::X)>();
+        return (S || (N <= 64 && P * W > 128)) && W > 8 ? 8 : W;
+    }
+}
+// Launches of few members with x tiles of 8 pencils instead of 16 (the transforms are the
+// same, so that a member's result does not depend on how many there are): more, smaller CTAs.
+// One RK4 step of 48^3 65.3 -> 63.4 us (four members 86 -> 80, eight 129 -> 121, 24 262 -> 268
+// us), of 96^3 133 -> 129 us (two members 191 -> 188 us), of 128^3 187 -> 184 us (two members
+// 324 -> 328 us).
+template <int N, int V> constexpr bool x_small(int members) {
+    return V == 0 && ((N == 48 && members <= 8) || (N == 96 && members <= 2) || (N == 128 && members == 1));
 }
 // line pairs per CTA of the z pass (>= 96 threads)
 template <int N> constexpr int zpairs() {
@@ -225,19 +265,19 @@ enum { X_STAGE1 = 0, X_STAGE2 = 1, X_STAGE3 = 2, X_STAGE4 = 3, X_RHS = 8, X_PLAI
 // inputs of the vorticity are formed from them, so the five transforms below
 // read each input once.
 // ---------------------------------------------------------------------------
-template <typename T, int N, int V = 0>
+template <typename T, int N, int V = 0, bool S = false>
 constexpr size_t xinv_smem() {
-    return sizeof(cx<T>) * (size_t)N * tile_x<T, N, V>() * (1 + TileVar<V>::STAGE);
+    return sizeof(cx<T>) * (size_t)N * tile_x<T, N, V, false, S>() * (1 + TileVar<V>::STAGE);
 }
-template <typename T, int N, int V = 0>
-__global__ void __launch_bounds__(tile_x<T, N, V>() * PlansV<N, V>::X::P, TileVar<V>::MINB_XI)
+template <typename T, int N, int V = 0, bool S = false>
+__global__ void __launch_bounds__(tile_x<T, N, V, false, S>() * PlansV<N, V>::X::P, TileVar<V>::MINB_XI)
 k_xinv(const cx<T>* __restrict__ U, cx<T>* __restrict__ W, const cx<T>* __restrict__ tw) {
     const long long dep = pdl_begin();
     U += dep;
     W += dep;
     using G = Geo<N>;
     using PL = typename PlansV<N, V>::X;
-    constexpr int TT = tile_x<T, N, V>();
+    constexpr int TT = tile_x<T, N, V, false, S>();
     constexpr int E = PL::E, P = PL::P, NT = TT * P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<T>* sbuf = reinterpret_cast<cx<T>*>(smem_raw);
@@ -1372,8 +1412,8 @@ __device__ __forceinline__ void dp_block_sum(const double (&es)[3], double* __re
 // T. INTEG = INT_TAB runs the RkStage epilogue of the RK5 family; its DP5CN
 // error partial sums go to dpart[member][block][3] in a fixed order.
 // ---------------------------------------------------------------------------
-template <typename T, int N, int INTEG, int MODE, int V = 0, bool PRE = false>
-__global__ void __launch_bounds__(tile_x<T, N, V, true>() * PlansV<N, V>::X::P, TileVar<V>::MINB)
+template <typename T, int N, int INTEG, int MODE, int V = 0, bool PRE = false, bool S = false>
+__global__ void __launch_bounds__(tile_x<T, N, V, true, S>() * PlansV<N, V>::X::P, TileVar<V>::MINB)
 k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ UT,
        cx<T>* __restrict__ ACC, const cx<T>* __restrict__ tw, const StepDev* __restrict__ sd,
        const cx<T>* __restrict__ tab, const cx<T>* __restrict__ sgs, cx<T>* __restrict__ K,
@@ -1390,7 +1430,7 @@ k_xfwd(const cx<T>* __restrict__ W, cx<T>* __restrict__ U, cx<T>* __restrict__ U
     dpart += dep;
     using G = Geo<N>;
     using PL = typename PlansV<N, V>::X;
-    constexpr int TT = tile_x<T, N, V, true>();
+    constexpr int TT = tile_x<T, N, V, true, S>();
     constexpr int E = PL::E, P = PL::P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<T>* sbuf = reinterpret_cast<cx<T>*>(smem_raw);
