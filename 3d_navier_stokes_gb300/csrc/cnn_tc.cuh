@@ -21,9 +21,9 @@
 //   B: [(dx,dy) 9][n group 3 NO/8][kchunk KC][8 (dz, co)][16 B]
 // Activations between layers are BF16 in the blocked layout
 // [x][y][z group][kchunk][8 points][8 channels], so every (x, y) line of the
-// halo block is one contiguous run identical to its place in A: one thread
-// stages a tile with 3 (R+2) cp.async.bulk copies completed on an mbarrier.
-// The copies for tile i+2 are issued as soon as the MMAs of tile i have
+// halo block is one contiguous run identical to its place in A: one warp
+// stages a tile with 3 (R+2) cp.async.bulk copies, one per lane, completed on an
+// mbarrier. The copies for tile i+2 are issued as soon as the MMAs of tile i have
 // released its buffer, and the MMAs of tile i+1 before the epilogue of tile i
 // (tensor memory -> registers, the dz combination through a shared exchange
 // of the dz = -1 and +1 blocks, bias, GELU), which the other warps run while
@@ -131,16 +131,18 @@ __global__ void k_to_blocked(const float* __restrict__ u, float in_scale, uint4*
 // a = GELU(z) blocked and as the wg-A copy (cm) of the weight-gradient kernel;
 // 3 (the input gradient, weights packed transposed and mirrored by
 // k_pack_jobs with transposed = 1, no bias): d = out * GELU'(zbuf) blocked and as the wg-B copies
-// (cm). Warp-specialised, 17 warps: lane 0 of warp 16 (the producer) issues the
-// copies and the MMAs; warps 0..15 (the epilogue) each take tensor-memory lane
+// (cm). Warp-specialised, 18 warps: warp 16 issues the copies, lane 0 of warp 17 the
+// MMAs; warps 0..15 (the epilogue) each take tensor-memory lane
 // quarter w % 4 and output channels [8 (w / 4), 8 (w / 4) + 8). Handoffs run on
 // mbarriers only: full[b] (the copies of A buffer b landed), done[b] (the MMAs
 // into accumulator b completed, also freeing A buffer b), aempty[b] (the 16
 // epilogue warps have read accumulator b); the epilogue warps synchronise among
-// themselves on a named barrier, so the producer keeps the MMAs of tile i + 1
-// running while tile i's epilogue runs.
+// themselves on a named barrier, so that the MMAs of tile i + 1 run while tile i's
+// epilogue does. 64^3, 32 -> 32 channels: 41.0 -> 24.6 us, the 6-channel output layer 33.5 ->
+// 16.5 us, against one thread that formed the descriptors in a loop and issued MMAs and copies
+// in turn; now bound by the epilogue's instructions (GELU, the dz exchange).
 constexpr int kConvWarps = 16;                        // epilogue warps
-constexpr int kConvThreads = 32 * (kConvWarps + 1);   // and the producer warp
+constexpr int kConvThreads = 32 * (kConvWarps + 2);   // and the copy and MMA warps
 constexpr int kTcThreads = 256;                       // the weight-gradient kernel
 
 // the epilogue warps' named barrier 1 (512 threads), and the same with an AND
@@ -202,73 +204,67 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
     const uint32_t tmem = *holder;
 
     if (warp == kConvWarps) {
-        // ------------------------------------------------------------ producer
-        if (lane == 0) {
-            const uint32_t sA_u = smem_u32(sA), sB_u = smem_u32(sB);
-            uint32_t ph_full = 0u, ph_done = 0u, ph_empty = 0u;   // bit b: parity of the next completion
-            uint32_t pend_copy = 0u, pend_mma = 0u;               // bit b: in flight
+        // ------------------------------------------------------------ copies
+        // the halo block of tile i into buffer i & 1 once tile i - 2's MMAs, which read it, are
+        // done: 3 (R+2) line copies, one per lane
+        static_assert(3 * rows <= 32, "a lane per line");
+        const int xp = lane / rows, yr = lane % rows;
+        int i = 0;
+#pragma unroll 1
+        for (; i < nmine; ++i) {
+            const int b = i & 1;
             bool ok = true;
-            // the halo block of tile t into buffer b: 3 (R+2) line copies
-            auto load = [&](int t, int b) {
-                const int x = t / tiles_per_x, y0 = (t % tiles_per_x) * R;
-                mbar_arrive_expect_tx(&full[b], a_bytes);
+            if (i >= 2 && lane == 0) ok = mbar_wait(&done[b], (uint32_t)((i >> 1) - 1) & 1u);
+            if (!__shfl_sync(0xffffffffu, (int)ok, 0)) {
+                if (lane == 0) atomicExch(status, kStatusTimeout);
+                break;
+            }
+            const int t = first + i * stride;
+            const int x = t / tiles_per_x, y0 = (t % tiles_per_x) * R;
+            if (lane == 0) mbar_arrive_expect_tx(&full[b], a_bytes);
+            __syncwarp();
+            if (lane < 3 * rows) {
+                const int gx = (x + xp - 1) & (D - 1), gy = (y0 + yr - 1) & (D - 1);
+                bulk_g2s(sA + b * a_bytes + lane * line_bytes, in + (((long long)gx << LOGD) + gy) * (D * KC), line_bytes,
+                         &full[b]);
+            }
+        }
+        // the copies still in flight land before the CTA exits
+        if (lane == 0)
+            for (int q = i > 2 ? i - 2 : 0; q < i; ++q) (void)mbar_wait(&full[q & 1], (uint32_t)(q >> 1) & 1u);
+    } else if (warp == kConvWarps + 1) {
+        // ------------------------------------------------------------ MMAs
+        if (lane == 0) {
+            const uint64_t dA = smem_desc(smem_u32(sA), 128, KC * 128), dB = smem_desc(smem_u32(sB), 128, KC * 128);
+            int i = 0;
 #pragma unroll 1
-                for (int l = 0; l < 3 * rows; ++l) {
-                    const int xp = l / rows, yr = l % rows;
-                    const int gx = (x + xp - 1) & (D - 1), gy = (y0 + yr - 1) & (D - 1);
-                    bulk_g2s(sA + b * a_bytes + l * line_bytes, in + (((long long)gx << LOGD) + gy) * (D * KC),
-                             line_bytes, &full[b]);
-                }
-                pend_copy |= 1u << b;
-            };
-            if (nmine > 0) load(first, 0);
-            if (nmine > 1) load(first + stride, 1);
-#pragma unroll 1
-            for (int i = 0; i < nmine; ++i) {
+            for (; i < nmine; ++i) {
                 const int b = i & 1;
-                ok = mbar_wait(&full[b], (ph_full >> b) & 1u);
-                if (!ok) break;
-                ph_full ^= 1u << b;
-                pend_copy &= ~(1u << b);
-                if (i >= 2) {   // the epilogue of tile i - 2 has read accumulator b
-                    ok = mbar_wait(&aempty[b], (ph_empty >> b) & 1u);
-                    if (!ok) break;
-                    ph_empty ^= 1u << b;
+                bool ok = mbar_wait(&full[b], (uint32_t)(i >> 1) & 1u);
+                // the epilogue of tile i - 2 has read accumulator b
+                if (ok && i >= 2) ok = mbar_wait(&aempty[b], (uint32_t)((i >> 1) - 1) & 1u);
+                if (!ok) {
+                    atomicExch(status, kStatusTimeout);
+                    break;
                 }
                 tc_fence_after();
-                const uint32_t a_base = sA_u + b * a_bytes, d = tmem + 128u * b;
-                uint32_t acc = 0;
-#pragma unroll 1
+                const uint64_t a0 = dA + b * (a_bytes >> 4);
+                const uint32_t d = tmem + 128u * b;
+                // unrolled: the operands of an MMA are constants away from the tile's, which one
+                // thread issues as fast as they execute (with the descriptors formed in a loop, 90 -
+                // 140 clocks each, whatever N)
+#pragma unroll
                 for (int t9 = 0; t9 < 9; ++t9) {
                     const int dx = t9 / 3, dy = t9 % 3;   // offsets + 1
-                    const uint32_t a0 = a_base + ((dx * rows + dy) * ZG) * KC * 128;
-                    const uint32_t b0 = sB_u + (uint32_t)(t9 * (NB / 8) * KC) * 128;
 #pragma unroll
-                    for (int ks = 0; ks < KC / 2; ++ks) {
-                        mma_bf16(d, smem_desc(a0 + ks * 256, 128, KC * 128), smem_desc(b0 + ks * 256, 128, KC * 128),
-                                 idesc, acc);
-                        acc = 1;
-                    }
+                    for (int ks = 0; ks < KC / 2; ++ks)
+                        mma_bf16(d, a0 + (((dx * rows + dy) * ZG * KC * 128 + ks * 256) >> 4),
+                                 dB + ((t9 * (NB / 8) * KC * 128 + ks * 256) >> 4), idesc, t9 + ks > 0);
                 }
                 mma_commit(&done[b]);
-                pend_mma |= 1u << b;
-                // those MMAs read A buffer b: refill it with tile i + 2 once they are done
-                // (refilling the other buffer with tile i + 1 right after issuing these
-                // instead measured slower: its copies then land too late)
-                if (i + 2 < nmine) {
-                    ok = mbar_wait(&done[b], (ph_done >> b) & 1u);
-                    if (!ok) break;
-                    ph_done ^= 1u << b;
-                    pend_mma &= ~(1u << b);
-                    load(first + (i + 2) * stride, b);
-                }
             }
-            if (!ok) atomicExch(status, kStatusTimeout);
-            // the copies and MMAs still in flight complete before the CTA exits
-            for (int b = 0; b < 2; ++b) {
-                if (pend_copy & (1u << b)) (void)mbar_wait(&full[b], (ph_full >> b) & 1u);
-                if (pend_mma & (1u << b)) (void)mbar_wait(&done[b], (ph_done >> b) & 1u);
-            }
+            // the MMAs still in flight complete before the CTA exits
+            for (int q = i > 2 ? i - 2 : 0; q < i; ++q) (void)mbar_wait(&done[q & 1], (uint32_t)(q >> 1) & 1u);
         }
     } else {
         // ------------------------------------------------------------ epilogue warps
@@ -494,8 +490,10 @@ __host__ __device__ constexpr uint32_t tc_chunk(int r, int k8, int K) {
 // the wg-A copy, one bulk copy each, placed so that the 8-row groups of a tap
 // group are SBO = 16 D bytes apart; B is the wg-B line, one bulk copy. A
 // padding row of the last tap group holds ones, so its j = 1 columns sum to
-// the bias gradient sum_p d[co][p]. Persistent CTAs walk the D^2 lines; thread
-// 0 keeps NST stages of copies in flight and issues the MMAs (bounded waits);
+// the bias gradient sum_p d[co][p]. Persistent CTAs walk the D^2 lines; warp 1
+// keeps NST stages of copies in flight, a copy per lane, and thread 0 issues the MMAs
+// (bounded waits). 64^3: 32 x 32 channels 49.5 -> 26.7 us, 32 x 6 44 -> 20.6 us, 3 x 32 32 ->
+// 20.6 us against one thread for both; bound by the copies out of L2 (200 MB at 32 x 32).
 // each CTA writes its FP32 partial sums [group][128][3 NB] to part, reduced in
 // a fixed order by k_wgrad_reduce.
 template <int CI, int NB, int LOGD>
@@ -540,13 +538,10 @@ k_wgrad_tc(const uint4* __restrict__ a, const uint4* __restrict__ d, float* __re
     uint32_t* holder = reinterpret_cast<uint32_t*>(done + NST);
     __shared__ int s_ok;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // zero every stage (the tap slots past the ninth stay zero), then the ones row
-    for (uint32_t q = tid; q < NST * WG::STAGE / 16; q += kTcThreads)
-        reinterpret_cast<uint4*>(smem)[q] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
+    // the ones row of every stage (the other rows past the ninth tap hold anything: theirs are discarded)
     for (int q = tid; q < NST * D; q += kTcThreads) {
         unsigned char* row = smem + (q / D) * WG::STAGE + (NGRP - 1) * WG::A_BYTES + (WG::ONES / 8) * SBO + (q % D) * 16;
-        *reinterpret_cast<uint32_t*>(row) = 0x3F80u;   // BF16 1.0 in channel slot 0 of the row group
+        *reinterpret_cast<uint4*>(row) = make_uint4(0x3F80u, 0u, 0u, 0u);   // BF16 1.0 in channel slot 0 of the row group
     }
     fence_proxy_async_smem();
     if (tid == 0) {
@@ -565,67 +560,65 @@ k_wgrad_tc(const uint4* __restrict__ a, const uint4* __restrict__ d, float* __re
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *holder;
-    if (tid == 0) {
-        const uint32_t s_u = smem_u32(smem);
-        const int first = blockIdx.x, stride = gridDim.x;
-        const int nmine = first < nlines ? (nlines - first + stride - 1) / stride : 0;
-        uint32_t ph_full = 0u, ph_done = 0u, pend_full = 0u, pend_done = 0u;   // one bit per stage
-        auto load = [&](int line, int st) {
-            const int x = line >> LOGD, y = line & (D - 1);
+    const int first = blockIdx.x, stride = gridDim.x;
+    const int nmine = first < nlines ? (nlines - first + stride - 1) / stride : 0;
+    if (warp == 1) {
+        // copies: line i into stage i % NST once line i - NST's MMAs are done, one copy per lane
+        // (the nine tap lines of A, the B line)
+        int i = 0;
+#pragma unroll 1
+        for (; i < nmine; ++i) {
+            const int st = i % NST, turn = i / NST;
+            bool ok = true;
+            if (turn > 0 && lane == 0) ok = mbar_wait(&done[st], (uint32_t)(turn - 1) & 1u);
+            if (!__shfl_sync(0xffffffffu, (int)ok, 0)) {
+                if (lane == 0) {
+                    s_ok = 0;
+                    atomicExch(status, kStatusTimeout);
+                }
+                break;
+            }
+            const int line = first + i * stride, x = line >> LOGD, y = line & (D - 1);
             unsigned char* sa = smem + st * WG::STAGE;
-            mbar_arrive_expect_tx(&full[st], 9u * WG::TAP_BYTES + WG::B_BYTES);
-#pragma unroll 1
-            for (int t9 = 0; t9 < 9; ++t9) {
-                const int gx = (x + t9 / 3 - 1) & (D - 1), gy = (y + t9 % 3 - 1) & (D - 1);
-                bulk_g2s(sa + (t9 / TG) * WG::A_BYTES + (t9 % TG) * WG::TAP_BYTES,
+            if (lane == 0) mbar_arrive_expect_tx(&full[st], 9u * WG::TAP_BYTES + WG::B_BYTES);
+            __syncwarp();
+            if (lane < 9) {
+                const int gx = (x + lane / 3 - 1) & (D - 1), gy = (y + lane % 3 - 1) & (D - 1);
+                bulk_g2s(sa + (lane / TG) * WG::A_BYTES + (lane % TG) * WG::TAP_BYTES,
                          a + ((((long long)gx << LOGD) + gy) * (CI / 8)) * D, WG::TAP_BYTES, &full[st]);
+            } else if (lane == 9) {
+                bulk_g2s(sa + WG::A_REGION, d + (((long long)x << LOGD) + y) * 3 * (NB / 8) * D, WG::B_BYTES,
+                         &full[st]);
             }
-            bulk_g2s(sa + WG::A_REGION, d + (((long long)x << LOGD) + y) * 3 * (NB / 8) * D, WG::B_BYTES,
-                     &full[st]);
-            pend_full |= 1u << st;
-        };
-        bool ok = true;
-        for (int st = 0; st < NST && st < nmine; ++st) load(first + st * stride, st);
+        }
+        // the copies still in flight land before the CTA exits
+        if (lane == 0)
+            for (int q = i > NST ? i - NST : 0; q < i; ++q) (void)mbar_wait(&full[q % NST], (uint32_t)(q / NST) & 1u);
+    } else if (tid == 0) {
+        const uint64_t dA = smem_desc(smem_u32(smem), 128, SBO), dB = dA + (WG::A_REGION >> 4);
+        int i = 0;
 #pragma unroll 1
-        for (int i = 0; i < nmine && ok; ++i) {
+        for (; i < nmine; ++i) {
             const int st = i % NST;
-            ok = mbar_wait(&full[st], (ph_full >> st) & 1u);
-            if (!ok) break;
-            ph_full ^= 1u << st;
-            pend_full &= ~(1u << st);
-            tc_fence_after();
-            const uint32_t a0 = s_u + st * WG::STAGE, b0 = a0 + WG::A_REGION;
-#pragma unroll 1
-            for (int g = 0; g < NGRP; ++g)
-#pragma unroll 1
-                for (int ks = 0; ks < D / 16; ++ks)
-                    mma_bf16(tmem + g * NN, smem_desc(a0 + g * WG::A_BYTES + ks * 256, 128, SBO),
-                             smem_desc(b0 + ks * 256, 128, SBO), idesc, (i > 0 || ks > 0) ? 1u : 0u);
-            mma_commit(&done[st]);
-            pend_done |= 1u << st;
-            // the MMAs of line i - 1 (queued before these) are done: refill their stage
-            if (i >= 1) {
-                const int ps = (i - 1) % NST;
-                ok = mbar_wait(&done[ps], (ph_done >> ps) & 1u);
-                if (!ok) break;
-                ph_done ^= 1u << ps;
-                pend_done &= ~(1u << ps);
-                if (i - 1 + NST < nmine) load(first + (i - 1 + NST) * stride, ps);
+            if (!mbar_wait(&full[st], (uint32_t)(i / NST) & 1u)) {
+                s_ok = 0;
+                atomicExch(status, kStatusTimeout);
+                break;
             }
+            tc_fence_after();
+            const uint32_t so = (uint32_t)st * (WG::STAGE >> 4);
+#pragma unroll
+            for (int g = 0; g < NGRP; ++g)
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks)
+                    mma_bf16(tmem + g * NN, dA + so + ((g * WG::A_BYTES + ks * 256) >> 4), dB + so + ((ks * 256) >> 4),
+                             idesc, (i > 0 || ks > 0) ? 1u : 0u);
+            mma_commit(&done[st]);
         }
-        if (ok && nmine > 0) {
-            const int ls = (nmine - 1) % NST;
-            ok = mbar_wait(&done[ls], (ph_done >> ls) & 1u);
-            if (ok) pend_done &= ~(1u << ls);
-        }
-        if (!ok) {
+        // every MMA completes (they do so in order) before the accumulators are read
+        if (i > 0 && !mbar_wait(&done[(i - 1) % NST], (uint32_t)((i - 1) / NST) & 1u)) {
             s_ok = 0;
             atomicExch(status, kStatusTimeout);
-            // one more bounded wait for the copies and MMAs in flight
-            for (int st = 0; st < NST; ++st) {
-                if (pend_full & (1u << st)) (void)mbar_wait(&full[st], (ph_full >> st) & 1u);
-                if (pend_done & (1u << st)) (void)mbar_wait(&done[st], (ph_done >> st) & 1u);
-            }
         }
     }
     tc_fence_before();
