@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tma.cuh"
+
 namespace ns3d {
 namespace cnn {
 
@@ -147,12 +149,30 @@ __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ t, 
     if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// the loss of one sample: the k_mse partial sums in block order, / denom
-__global__ void k_loss_store(const double* __restrict__ part, int nparts, double denom, double* __restrict__ out) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        double s = 0.0;
-        for (int i = 0; i < nparts; ++i) s += part[i];
-        *out = s / denom;
+// a warp's sum of x[0 .. n): lane-strided, then a butterfly (a fixed order)
+template <typename T> __device__ __forceinline__ T warp_total(const T* __restrict__ x, int n) {
+    T s = T(0);
+#pragma unroll 8
+    for (int i = threadIdx.x & 31; i < n; i += 32) s += x[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+// the loss of one sample: the sum of the per-CTA losses / denom, by warp 0; with chan, warps
+// 1 .. nch the channel sums of its partials [nch][nparts] into out_chan (one thread over 256
+// partials: 16 us, a warp: 3)
+__global__ void k_loss_store(const double* __restrict__ part, int nparts, double denom, double* __restrict__ out,
+                             const float* __restrict__ chan, int nch, float* __restrict__ out_chan) {
+    const long long dep = pdl_begin();
+    part += dep;
+    chan += dep;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {
+        const double s = warp_total(part, nparts);
+        if (lane == 0) *out = s / denom;
+    } else if (warp <= nch) {
+        const float s = warp_total(chan + (warp - 1) * nparts, nparts);
+        if (lane == 0) out_chan[warp - 1] = s;
     }
 }
 

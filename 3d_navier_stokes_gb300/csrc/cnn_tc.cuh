@@ -110,6 +110,7 @@ template <int LOGD>
 __global__ void k_to_blocked(const float* __restrict__ u, float in_scale, uint4* __restrict__ dst) {
     constexpr int D = 1 << LOGD;
     constexpr long long D3 = (long long)D * D * D;
+    u += pdl_begin();
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < D3; p += (long long)gridDim.x * blockDim.x) {
         const int z = (int)(p & (D - 1)), y = (int)((p >> LOGD) & (D - 1)), x = (int)(p >> (2 * LOGD));
         uint4 v;
@@ -184,8 +185,6 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
     const int first = blockIdx.x, stride = gridDim.x;
     const int nmine = first < ntiles ? (ntiles - first + stride - 1) / stride : 0;
 
-    for (uint32_t q = tid; q < b_bytes / 16; q += kConvThreads) reinterpret_cast<uint4*>(sB)[q] = wpk[q];
-    fence_proxy_async_smem();   // B (generic stores) -> visible to the tensor cores
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
             mbar_init(&done[b], 1);
@@ -198,6 +197,13 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
         tmem_alloc(holder, kTcTmemCols);
         tmem_relinquish();
     }
+    const long long dep = pdl_begin();
+    in += dep;
+    wpk += dep;
+    bias += dep;
+    zbuf += dep;
+    for (uint32_t q = tid; q < b_bytes / 16; q += kConvThreads) reinterpret_cast<uint4*>(sB)[q] = wpk[q];
+    fence_proxy_async_smem();   // B (generic stores) -> visible to the tensor cores
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -275,9 +281,24 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
 #pragma unroll
         for (int j = 0; j < 8; ++j) bv[j] = bias[8 * part + j < cout ? 8 * part + j : 0];
         uint32_t ph_done = 0u;
+        // OUT_MODE 3: the pre-activations, one tile ahead (they come from HBM; loaded where they
+        // are used 39.0, before the wait for the tile's MMAs 43, a tile ahead 32.8 us)
+        float zn[8] = {};
+        auto load_z = [&](int tile) {
+            if constexpr (OUT_MODE == 3) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) zn[j] = zbuf[(long long)(8 * part + j) * D3 + (long long)tile * 128 + m];
+            }
+        };
+        if (nmine > 0) load_z(first);
 #pragma unroll 1
         for (int i = 0; i < nmine; ++i) {
             const int b = i & 1, tile = first + i * stride;
+            const int x = tile / tiles_per_x, y0 = (tile % tiles_per_x) * R;
+            float zv[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) zv[j] = zn[j];
+            if (i + 1 < nmine) load_z(tile + stride);
             // tile i's MMAs are done (every epilogue thread waits; all agree on the
             // outcome); this barrier also ends every read of sX for tile i - 1
             const bool got = mbar_wait(&done[b], (ph_done >> b) & 1u);
@@ -287,7 +308,6 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
             }
             ph_done ^= 1u << b;
             tc_fence_after();
-            const int x = tile / tiles_per_x, y0 = (tile % tiles_per_x) * R;
             const uint32_t tl = tmem + 128u * b + ((uint32_t)(quarter * 32) << 16) + 8u * part;
             uint32_t gm[8], g0[8], gp[8];
             if (active) {
@@ -329,12 +349,11 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
                     float o[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const long long qi = (long long)(8 * part + j) * D3 + p;
                         if constexpr (OUT_MODE == 2) {
-                            zbuf[qi] = v[j];
+                            zbuf[(long long)(8 * part + j) * D3 + p] = v[j];
                             o[j] = gelu_tc(v[j]);
                         } else {
-                            o[j] = v[j] * gelu_grad_tc(zbuf[qi]);
+                            o[j] = v[j] * gelu_grad_tc(zv[j]);
                         }
                     }
                     uint4* dst = reinterpret_cast<uint4*>(out);
@@ -412,63 +431,86 @@ __global__ void k_pack_jobs(const PackJobs jobs) {
     }
 }
 
-// per-channel sums of an FP32 [nch][n] array in two fixed-order levels:
-// partial[c][blockIdx.x] over a strided share, then the partials in order
-__global__ void k_chan_partial(const float* __restrict__ x, long long n, float* __restrict__ partial) {
-    __shared__ float red[256];
-    const int c = blockIdx.y;
-    const float* xc = x + (long long)c * n;
-    float s = 0.0f;
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
-        s += xc[p];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[c * gridDim.x + blockIdx.x] = red[0];
-}
-__global__ void k_chan_final(const float* __restrict__ partial, int nparts, int nch, float* __restrict__ out) {
-    const int c = threadIdx.x;
-    if (c >= nch) return;
-    float s = 0.0f;
-    for (int q = 0; q < nparts; ++q) s += partial[c * nparts + q];
-    out[c] = s;
-}
-
-// FP32 velocity [3][D^3] x in_scale -> wg-A BF16 with 8 channels (3..7 zero);
-// with one run per line the wg-A index of point p is p
+// FP32 velocity [3][D^3] x in_scale -> the first layer's input, blocked with 16 channels, and its
+// wg-A copy with 8 channels (3..7 zero; with one run per line the wg-A index of point p is p)
 template <int LOGD>
-__global__ void k_to_wga(const float* __restrict__ u, float in_scale, uint4* __restrict__ dst) {
-    constexpr long long D3 = 1ll << (3 * LOGD);
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < D3; p += (long long)gridDim.x * blockDim.x)
-        dst[p] = make_uint4(pack_bf16x2(u[p] * in_scale, u[D3 + p] * in_scale), pack_bf16x2(u[2 * D3 + p] * in_scale, 0.0f),
-                            0u, 0u);
-}
-
-// the output gradient d_4 (FP32 [6][D^3]) -> blocked BF16 with 2 chunks (16
-// channels, 6 used) and its wg-B copies (channels 6..15 zero)
-template <int LOGD>
-__global__ void k_grad_pack(const float* __restrict__ g, uint4* __restrict__ blk, uint4* __restrict__ wg) {
+__global__ void k_input_pack(const float* __restrict__ u, float in_scale, uint4* __restrict__ blk,
+                             uint4* __restrict__ wg) {
     constexpr int D = 1 << LOGD;
-    constexpr long long D3 = (long long)D * D * D;
+    constexpr long long D3 = 1ll << (3 * LOGD);
+    const long long dep = pdl_begin();
+    u += dep;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < D3; p += (long long)gridDim.x * blockDim.x) {
         const int z = (int)(p & (D - 1)), y = (int)((p >> LOGD) & (D - 1)), x = (int)(p >> (2 * LOGD));
-        float v[16];
-#pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = c < 6 ? g[c * D3 + p] : 0.0f;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const uint4 pk =
-                make_uint4(pack_bf16x2(v[q * 8 + 0], v[q * 8 + 1]), pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]),
-                           pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]));
-            blk[blk_index<LOGD, 2>(x, y, z, q)] = pk;
-            wgb_store<LOGD, 16>(wg, x, y, q, z, pk);
-        }
+        const uint4 v = make_uint4(pack_bf16x2(u[p] * in_scale, u[D3 + p] * in_scale),
+                                   pack_bf16x2(u[2 * D3 + p] * in_scale, 0.0f), 0u, 0u);
+        blk[blk_index<LOGD, 2>(x, y, z, 0)] = v;
+        blk[blk_index<LOGD, 2>(x, y, z, 1)] = make_uint4(0u, 0u, 0u, 0u);
+        wg[p] = v;
     }
 }
 
+// Loss and output gradient in one pass: g = 2 (y - t tscale) / n of the 6 channels of a point, as
+// d_4 blocked with 2 chunks (16 channels, 6 used) and its wg-B copies (channels 6..15 zero),
+// and per CTA the squared errors' sum (FP64, loss[blockIdx.x]) and the channels' sums of g
+// (chan[c][blockIdx.x]). Moves 46 MB at 64^3; with a pass each for the loss and g, the packing
+// and the sums 37 us, so 13.
+constexpr int kLossThreads = 256;
+template <int LOGD>
+__global__ void __launch_bounds__(kLossThreads)
+k_loss_pack(const float* __restrict__ y, const float* __restrict__ t, float tscale, uint4* __restrict__ blk,
+            uint4* __restrict__ wg, double* __restrict__ loss, float* __restrict__ chan) {
+    constexpr int D = 1 << LOGD, NW = kLossThreads / 32;
+    constexpr long long D3 = (long long)D * D * D;
+    const long long dep = pdl_begin();
+    y += dep;
+    t += dep;
+    __shared__ double red[NW];
+    __shared__ float redc[6][NW];
+    double s = 0.0;
+    float sc[6] = {};
+    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < D3; p += (long long)gridDim.x * blockDim.x) {
+        const int z = (int)(p & (D - 1)), yy = (int)((p >> LOGD) & (D - 1)), x = (int)(p >> (2 * LOGD));
+        float d[6], v[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) d[c] = y[c * D3 + p] - t[c * D3 + p] * tscale;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            v[c] = 2.0f * d[c] / (float)(6 * D3);
+            s += (double)d[c] * d[c];
+            sc[c] += v[c];
+        }
+        const uint4 pk = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), 0u);
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        blk[blk_index<LOGD, 2>(x, yy, z, 0)] = pk;
+        blk[blk_index<LOGD, 2>(x, yy, z, 1)] = zero;
+        wgb_store<LOGD, 16>(wg, x, yy, 0, z, pk);
+        wgb_store<LOGD, 16>(wg, x, yy, 1, z, zero);
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) sc[c] += __shfl_xor_sync(0xffffffffu, sc[c], o);
+    }
+    if (lane == 0) {
+        red[warp] = s;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) redc[c][warp] = sc[c];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = 0.0;
+        for (int w = 0; w < NW; ++w) a += red[w];
+        loss[blockIdx.x] = a;
+    } else if (threadIdx.x <= 6) {
+        const int c = threadIdx.x - 1;
+        float a = 0.0f;
+        for (int w = 0; w < NW; ++w) a += redc[c][w];
+        chan[c * gridDim.x + blockIdx.x] = a;
+    }
+}
 
 __host__ __device__ constexpr int tc_pow2(int v) {
     int p = 32;
@@ -494,7 +536,7 @@ __host__ __device__ constexpr uint32_t tc_chunk(int r, int k8, int K) {
 // keeps NST stages of copies in flight, a copy per lane, and thread 0 issues the MMAs
 // (bounded waits). 64^3: 32 x 32 channels 49.5 -> 26.7 us, 32 x 6 44 -> 20.6 us, 3 x 32 32 ->
 // 20.6 us against one thread for both; bound by the copies out of L2 (200 MB at 32 x 32).
-// each CTA writes its FP32 partial sums [group][128][3 NB] to part, reduced in
+// Each CTA writes its FP32 partial sums [group][128][3 NB] to part, reduced in
 // a fixed order by k_wgrad_reduce.
 template <int CI, int NB, int LOGD>
 struct WgGeo {
@@ -560,6 +602,9 @@ k_wgrad_tc(const uint4* __restrict__ a, const uint4* __restrict__ d, float* __re
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *holder;
+    const long long dep = pdl_begin();
+    a += dep;
+    d += dep;
     const int first = blockIdx.x, stride = gridDim.x;
     const int nmine = first < nlines ? (nlines - first + stride - 1) / stride : 0;
     if (warp == 1) {
@@ -647,19 +692,40 @@ k_wgrad_tc(const uint4* __restrict__ a, const uint4* __restrict__ d, float* __re
     if (warp == 0) tmem_dealloc(tmem, WG::TCOLS);
 }
 
-// sum of the CTAs' partials in CTA order, scattered to dW[co][ci][27]; the
-// ones row's dz = 0 columns to db[co] when db is given
-__global__ void k_wgrad_reduce(const float* __restrict__ part, int nparts, int CI, int NB, int ngrp, int cin,
-                               int cout, float* __restrict__ dw, float* __restrict__ db) {
+// sum of the CTAs' partials in a fixed order, scattered to dW[co][ci][27]; the ones row's
+// dz = 0 columns to db[co] when db is given. A CTA takes kRedCols columns, its kRedParts thread
+// rows every kRedParts-th partial, eight loads in flight: 18 -> 8.4 us for 152 partials of 32 x 32
+// channels (one thread per column over all of them: a chain of loads on one wave of small CTAs).
+constexpr int kRedCols = 64, kRedParts = 4;
+__global__ void __launch_bounds__(kRedCols* kRedParts)
+k_wgrad_reduce(const float* __restrict__ part, int nparts, int CI, int NB, int ngrp, int cin,
+               int cout, float* __restrict__ dw, float* __restrict__ db) {
+    const long long dep = pdl_begin();
+    part += dep;
+    __shared__ float red[kRedParts][kRedCols];
     const int NN = 3 * NB, TG = 128 / CI, width = ngrp * 128 * NN, ones = (9 - (ngrp - 1) * TG) * CI;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= width) return;
+    const int col = threadIdx.x % kRedCols, row = threadIdx.x / kRedCols;
+    const int e = blockIdx.x * kRedCols + col;   // width is a multiple of kRedCols
     const int g = e / (128 * NN), r = (e / NN) % 128, n = e % NN;
     const int t9 = g * TG + r / CI, ci = r % CI, j = n / NB, co = n % NB;
     const bool bias = db != nullptr && g == ngrp - 1 && r == ones && j == 1 && co < cout;
-    if (!bias && (t9 >= 9 || ci >= cin || co >= cout)) return;
+    const bool used = bias || (t9 < 9 && ci < cin && co < cout);
     float s = 0.0f;
-    for (int q = 0; q < nparts; ++q) s += part[(long long)q * width + e];
+    if (used) {
+        int q = row;
+        for (; q + 7 * kRedParts < nparts; q += 8 * kRedParts) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = part[(long long)(q + k * kRedParts) * width + e];
+            s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        }
+        for (; q < nparts; q += kRedParts) s += part[(long long)q * width + e];
+    }
+    red[row][col] = s;
+    __syncthreads();
+    if (row != 0 || !used) return;
+#pragma unroll
+    for (int k = 1; k < kRedParts; ++k) s += red[k][col];
     if (bias)
         db[co] = s;
     else

@@ -17,6 +17,7 @@
 
 #include "ns3d_base.h"
 #include "fx_passes.cuh"
+#include "launch.cuh"
 #include "ns3d_kernels.cuh"
 
 namespace ns3d {
@@ -36,33 +37,6 @@ void fx_twiddle_table(int n, int* out);   // packed integers of the FP64 engines
 // 4D FP32 tensor map without swizzle (ns3d_misc.cu)
 bool encode_map4_f32(CUtensorMap* map, void* base, const uint64_t dims[4], const uint64_t strides[3],
                      const uint32_t box[4]);
-
-// Launch of a pass kernel with programmatic stream serialization: the launch itself
-// overlaps the previous kernel's end, and the kernel waits for its results (pdl_begin).
-// One RK4 step of 21 kernels, FP32: 32^3 67.6 -> 63.5 us, 64^3 75.7 -> 71.7 us, 128^3
-// 206.9 -> 202.8 us.
-template <typename A> struct ArgOf { using type = A; };
-template <typename... KA> struct Launcher {
-    void (*kernel)(KA...);
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[1];
-    void operator()(typename ArgOf<KA>::type... a) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, kernel, a...);
-    }
-};
-template <typename... KA>
-Launcher<KA...> pass(void (*kernel)(KA...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s) {
-    Launcher<KA...> l{kernel, {}, {}};
-    l.cfg.gridDim = grid;
-    l.cfg.blockDim = dim3(threads);
-    l.cfg.dynamicSmemBytes = smem;
-    l.cfg.stream = s;
-    return l;
-}
 
 template <typename T, int N, int V = 0>
 class Impl final : public Base {

@@ -17,6 +17,7 @@
 
 #include "cnn.cuh"
 #include "cnn_tc.cuh"
+#include "launch.cuh"
 #include "ns3d_ctx.h"
 
 namespace ns3d {
@@ -83,7 +84,6 @@ constexpr int oW1 = 0, ob1 = oW1 + C * 3 * 27, oW2 = ob1 + C, ob2 = oW2 + C * C 
               ob3 = oW3 + C * C * 27, oW4 = ob3 + C, ob4 = oW4 + 6 * C * 27, NPARAM = ob4 + 6;
 constexpr int NPART = 256;
 constexpr int kTrainChunk = 64;   // Adam iterations queued between host checks of the losses
-constexpr int kChanParts = 32;    // CTAs per channel of the output-bias gradient sum
 // packed tensor-core B operands of the four layers (BF16 elements):
 // (KC, NO) = (2, 32), (4, 32), (4, 32), (4, 16); 9 x 3 NO x 8 KC each
 constexpr int kTcW1 = 9 * 96 * 2 * 8, kTcW2 = 9 * 96 * 4 * 8, kTcW4 = 9 * 48 * 4 * 8;
@@ -129,7 +129,7 @@ struct ns3d_les : public ns3d::LesHook {
     double* losses = nullptr;
     double* losses_host = nullptr;
     int* halt = nullptr;
-    float* chanp = nullptr;   // output-bias gradient partial sums [6][kChanParts]
+    float* chanp = nullptr;   // output-bias gradient partial sums [6][NPART]
     int wg_grid = 0;
     int train_path = 0;                                  // 0: tensor cores where compiled, 1: FP32 CUDA cores
     int tc_grid[3] = {0, 0, 0};                          // CTAs of the three kernel shapes
@@ -188,10 +188,11 @@ struct ns3d_les : public ns3d::LesHook {
         using namespace ns3d::cnn;
         using WG = WgGeo<CI, NB, LOGD>;
         const int grid = wg_grid < WG::D * WG::D ? wg_grid : WG::D * WG::D;
-        k_wgrad_tc<CI, NB, LOGD><<<grid, kTcThreads, WG::SMEM, s>>>(reinterpret_cast<const uint4*>(a),
-                                                                     reinterpret_cast<const uint4*>(d), wpart, dstat);
-        k_wgrad_reduce<<<(WG::PART + 255) / 256, 256, 0, s>>>(wpart, grid, CI, NB, WG::NGRP, cin, cout, g + off,
-                                                             boff >= 0 ? g + boff : nullptr);
+        ns3d::pass(k_wgrad_tc<CI, NB, LOGD>, grid, kTcThreads, WG::SMEM, s)(
+            reinterpret_cast<const uint4*>(a), reinterpret_cast<const uint4*>(d), wpart, dstat);
+        static_assert(WG::PART % kRedCols == 0, "whole CTAs");
+        ns3d::pass(k_wgrad_reduce, WG::PART / kRedCols, kRedCols * kRedParts, 0, s)(
+            wpart, grid, CI, NB, WG::NGRP, cin, cout, g + off, boff >= 0 ? g + boff : nullptr);
     }
 
     // loss and gradients of one sample on the tensor cores (BF16 operands, FP32
@@ -209,31 +210,28 @@ struct ns3d_les : public ns3d::LesHook {
         uint4* b2 = reinterpret_cast<uint4*>(act2);
         uint4* b3 = reinterpret_cast<uint4*>(act3);
         const unsigned eg = (unsigned)((D3 + 255) / 256);
-        k_to_blocked<LOGD><<<eg, 256, 0, s>>>(u, is, b0);
-        k_to_wga<LOGD><<<eg, 256, 0, s>>>(u, is, reinterpret_cast<uint4*>(a0cm));
-        k_conv3_tc<2, 32, LOGD, 2><<<tc_grid[0], kConvThreads, tc_smem_bytes(2, 32, D), s>>>(
+        ns3d::pass(k_input_pack<LOGD>, eg, 256, 0, s)(u, is, b0, reinterpret_cast<uint4*>(a0cm));
+        ns3d::pass(k_conv3_tc<2, 32, LOGD, 2>, tc_grid[0], kConvThreads, tc_smem_bytes(2, 32, D), s)(
             b0, W + oT1 / 8, w + ob1, b1, C, 1.f, dstat, z1, a1cm);
-        k_conv3_tc<4, 32, LOGD, 2><<<tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s>>>(
+        ns3d::pass(k_conv3_tc<4, 32, LOGD, 2>, tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s)(
             b1, W + oT2 / 8, w + ob2, b2, C, 1.f, dstat, z2, a2cm);
-        k_conv3_tc<4, 32, LOGD, 2><<<tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s>>>(
+        ns3d::pass(k_conv3_tc<4, 32, LOGD, 2>, tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s)(
             b2, W + oT3 / 8, w + ob3, b3, C, 1.f, dstat, z3, a3cm);
-        k_conv3_tc<4, 16, LOGD, 1><<<tc_grid[2], kConvThreads, tc_smem_bytes(4, 16, D), s>>>(
-            b3, W + oT4 / 8, w + ob4, y, 6, 1.f, dstat);
-        k_mse<<<NPART, 256, 0, s>>>(y, t, (float)(1.0 / s_out), gy, 6 * D3, part);
+        ns3d::pass(k_conv3_tc<4, 16, LOGD, 1>, tc_grid[2], kConvThreads, tc_smem_bytes(4, 16, D), s)(
+            b3, W + oT4 / 8, w + ob4, y, 6, 1.f, dstat, nullptr, nullptr);
         // layer 4: d4 = dloss/dy (blocked into b0, which the forward no longer needs)
-        k_grad_pack<LOGD><<<eg, 256, 0, s>>>(gy, b0, reinterpret_cast<uint4*>(d4cm));
-        k_chan_partial<<<dim3(kChanParts, 6), 256, 0, s>>>(gy, D3, chanp);
-        k_chan_final<<<1, 32, 0, s>>>(chanp, kChanParts, 6, g + ob4);
+        ns3d::pass(k_loss_pack<LOGD>, NPART, kLossThreads, 0, s)(y, t, (float)(1.0 / s_out), b0,
+                                                           reinterpret_cast<uint4*>(d4cm), part, chanp);
         wgrad_tc<32, 16, LOGD>(a3cm, d4cm, C, 6, oW4, -1, s);
-        k_conv3_tc<2, 32, LOGD, 3><<<tc_grid[0], kConvThreads, tc_smem_bytes(2, 32, D), s>>>(
+        ns3d::pass(k_conv3_tc<2, 32, LOGD, 3>, tc_grid[0], kConvThreads, tc_smem_bytes(2, 32, D), s)(
             b0, WT + oU4 / 8, zeros, b3, C, 1.f, dstat, z3, d3cm);
         // layer 3
         wgrad_tc<32, 32, LOGD>(a2cm, d3cm, C, C, oW3, ob3, s);
-        k_conv3_tc<4, 32, LOGD, 3><<<tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s>>>(
+        ns3d::pass(k_conv3_tc<4, 32, LOGD, 3>, tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s)(
             b3, WT + oU3 / 8, zeros, b2, C, 1.f, dstat, z2, d2cm);
         // layer 2
         wgrad_tc<32, 32, LOGD>(a1cm, d2cm, C, C, oW2, ob2, s);
-        k_conv3_tc<4, 32, LOGD, 3><<<tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s>>>(
+        ns3d::pass(k_conv3_tc<4, 32, LOGD, 3>, tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s)(
             b2, WT + oU2 / 8, zeros, b1, C, 1.f, dstat, z1, d1cm);
         // layer 1
         wgrad_tc<8, 32, LOGD>(a0cm, d1cm, 3, C, oW1, ob1, s);
@@ -246,9 +244,12 @@ struct ns3d_les : public ns3d::LesHook {
     // the training path's gradients (tensor cores where compiled and selected), and
     // the sample's loss into the device slot *loss_slot
     void fwd_bwd_train(const float* u, const float* t, double* loss_slot, cudaStream_t s) {
-        if (tc_train()) fwd_bwd_tc(u, t, s);
+        const bool tc = tc_train();
+        if (tc) fwd_bwd_tc(u, t, s);
         else fwd_bwd(u, t, s);
-        ns3d::cnn::k_loss_store<<<1, 32, 0, s>>>(part, NPART, (double)(6 * D3), loss_slot);
+        // (the tensor-core path's output-bias gradient as well)
+        ns3d::pass(ns3d::cnn::k_loss_store, 1, tc ? 7 * 32 : 32, 0, s)(part, NPART, (double)(6 * D3), loss_slot, chanp, 6,
+                                                                 g + ob4);
     }
     // the same, synchronously: the loss, or NaN when a bounded wait gave up
     double fwd_bwd_sync(const float* u, const float* t, cudaStream_t s) {
@@ -282,15 +283,15 @@ struct ns3d_les : public ns3d::LesHook {
         uint4* a1 = reinterpret_cast<uint4*>(act1);
         uint4* a2 = reinterpret_cast<uint4*>(act2);
         uint4* a3 = reinterpret_cast<uint4*>(act3);
-        k_to_blocked<LOGD><<<(unsigned)((D3 + 255) / 256), 256, 0, s>>>(u, in_scale, a0);
-        k_conv3_tc<2, 32, LOGD, 0><<<tc_grid[0], kConvThreads, tc_smem_bytes(2, 32, D), s>>>(
-            a0, W + oT1 / 8, w + ob1, a1, C, 1.f, dstat);
-        k_conv3_tc<4, 32, LOGD, 0><<<tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s>>>(
-            a1, W + oT2 / 8, w + ob2, a2, C, 1.f, dstat);
-        k_conv3_tc<4, 32, LOGD, 0><<<tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s>>>(
-            a2, W + oT3 / 8, w + ob3, a3, C, 1.f, dstat);
-        k_conv3_tc<4, 16, LOGD, 1><<<tc_grid[2], kConvThreads, tc_smem_bytes(4, 16, D), s>>>(
-            a3, W + oT4 / 8, w + ob4, tau, 6, out_scale, dstat);
+        ns3d::pass(k_to_blocked<LOGD>, (unsigned)((D3 + 255) / 256), 256, 0, s)(u, in_scale, a0);
+        ns3d::pass(k_conv3_tc<2, 32, LOGD, 0>, tc_grid[0], kConvThreads, tc_smem_bytes(2, 32, D), s)(
+            a0, W + oT1 / 8, w + ob1, a1, C, 1.f, dstat, nullptr, nullptr);
+        ns3d::pass(k_conv3_tc<4, 32, LOGD, 0>, tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s)(
+            a1, W + oT2 / 8, w + ob2, a2, C, 1.f, dstat, nullptr, nullptr);
+        ns3d::pass(k_conv3_tc<4, 32, LOGD, 0>, tc_grid[1], kConvThreads, tc_smem_bytes(4, 32, D), s)(
+            a2, W + oT3 / 8, w + ob3, a3, C, 1.f, dstat, nullptr, nullptr);
+        ns3d::pass(k_conv3_tc<4, 16, LOGD, 1>, tc_grid[2], kConvThreads, tc_smem_bytes(4, 16, D), s)(
+            a3, W + oT4 / 8, w + ob4, tau, 6, out_scale, dstat, nullptr, nullptr);
     }
     void infer_tc(const float* u, float* tau, float in_scale, float out_scale, cudaStream_t s) {
         if (Nc == 16) infer_tc_d<4>(u, tau, in_scale, out_scale, s);
@@ -399,7 +400,7 @@ ns3d_status ns3d_les_create(int Nc, int capacity, uint64_t seed, ns3d_les** out)
         cudaMalloc(&l->losses, sizeof(double) * kTrainChunk) != cudaSuccess ||
         cudaMallocHost(&l->losses_host, sizeof(double) * kTrainChunk) != cudaSuccess ||
         cudaMalloc(&l->halt, sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&l->chanp, sizeof(float) * 6 * kChanParts) != cudaSuccess ||
+        cudaMalloc(&l->chanp, sizeof(float) * 6 * NPART) != cudaSuccess ||
         (capacity > 0 && (cudaMalloc(&l->data_u, f * 3 * l->D3 * capacity) != cudaSuccess ||
                           cudaMalloc(&l->data_t, f * 6 * l->D3 * capacity) != cudaSuccess))) {
         delete l;
