@@ -138,7 +138,7 @@ __global__ void k_to_blocked(const float* __restrict__ u, float in_scale, uint4*
 // mbarriers only: full[b] (the copies of A buffer b landed), done[b] (the MMAs
 // into accumulator b completed, also freeing A buffer b), aempty[b] (the 16
 // epilogue warps have read accumulator b); the epilogue warps synchronise among
-// themselves on a named barrier, so that the MMAs of tile i + 1 run while tile i's
+// themselves on named barriers, so that the MMAs of tile i + 1 run while tile i's
 // epilogue does. 64^3, 32 -> 32 channels: 41.0 -> 24.6 us, the 6-channel output layer 33.5 ->
 // 16.5 us, against one thread that formed the descriptors in a loop and issued MMAs and copies
 // in turn; now bound by the epilogue's instructions (GELU, the dz exchange).
@@ -146,15 +146,29 @@ constexpr int kConvWarps = 16;                        // epilogue warps
 constexpr int kConvThreads = 32 * (kConvWarps + 2);   // and the copy and MMA warps
 constexpr int kTcThreads = 256;                       // the weight-gradient kernel
 
-// the epilogue warps' named barrier 1 (512 threads), and the same with an AND
-// of a predicate across them
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kConvWarps) : "memory"); }
-__device__ __forceinline__ bool epi_sync_and(bool v) {
+// Barrier of GW epilogue warps (named barrier 1 + id), and the same with an AND of a predicate
+// across them. The dz exchange stays within a z line and 8 channels: in the input-gradient mode,
+// whose loads and stores take the warps unequal times, only the warps that hold those
+// synchronise (two at D = 64, one below; 64^3 32.8 -> 30.8 us); in the others all 16 (where
+// the finer groups measured 23.7 and 26.7 us against 22.6 and 24.6).
+template <int GW> __device__ __forceinline__ void epi_sync(int id) {
+    if constexpr (GW == 1) __syncwarp();
+    else if constexpr (GW == kConvWarps) asm volatile("bar.sync 1, %0;" ::"n"(32 * GW) : "memory");
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + id), "n"(32 * GW) : "memory");
+}
+template <int GW> __device__ __forceinline__ bool epi_sync_and(int id, bool v) {
+    if constexpr (GW == 1) return __all_sync(0xffffffffu, v);
     uint32_t r;
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, 1, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+    if constexpr (GW == kConvWarps)
+        asm volatile(
+            "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, 1, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(r)
+            : "r"((uint32_t)v), "n"(32 * GW)
+            : "memory");
+    else asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, %3, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(r)
-        : "r"((uint32_t)v), "n"(32 * kConvWarps)
+        : "r"((uint32_t)v), "n"(32 * GW), "r"(1 + id)
         : "memory");
     return r != 0;
 }
@@ -277,6 +291,8 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
         const int quarter = warp & 3, part = warp >> 2;   // lane quarter, 8-channel group
         const int m = quarter * 32 + lane;
         const bool active = (NO == 32) || part < 2;
+        constexpr int GW = OUT_MODE != 3 ? kConvWarps : (D > 32 ? D / 32 : 1);
+        const int grp = (4 * part + quarter) / GW;
         float bv[8];   // this thread's 8 biases, once
 #pragma unroll
         for (int j = 0; j < 8; ++j) bv[j] = bias[8 * part + j < cout ? 8 * part + j : 0];
@@ -299,11 +315,11 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
 #pragma unroll
             for (int j = 0; j < 8; ++j) zv[j] = zn[j];
             if (i + 1 < nmine) load_z(tile + stride);
-            // tile i's MMAs are done (every epilogue thread waits; all agree on the
-            // outcome); this barrier also ends every read of sX for tile i - 1
+            // tile i's MMAs are done (every epilogue thread waits; the group agrees on the
+            // outcome); this barrier also ends the group's reads of sX for tile i - 1
             const bool got = mbar_wait(&done[b], (ph_done >> b) & 1u);
-            if (!epi_sync_and(got)) {
-                if (tid == 0) atomicExch(status, kStatusTimeout);
+            if (!epi_sync_and<GW>(grp, got)) {
+                if (lane == 0) atomicExch(status, kStatusTimeout);
                 break;
             }
             ph_done ^= 1u << b;
@@ -329,7 +345,7 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
                     sX[(NO + 8 * part + j) * 128 + m] = __uint_as_float(gp[j]);
                 }
             }
-            epi_sync();
+            epi_sync<GW>(grp);
             if (active) {
                 const int line = m & ~(D - 1), zz = m & (D - 1), yy = y0 + (m >> LOGD);
                 const int left = line | ((zz - 1) & (D - 1)), right = line | ((zz + 1) & (D - 1));
