@@ -194,7 +194,8 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
     uint64_t* done = reinterpret_cast<uint64_t*>(sA + 2 * a_bytes + tc_x_bytes(NO));   // MMAs into accumulator b done
     uint64_t* full = done + 2;                                                 // copies into buffer b landed
     uint64_t* aempty = full + 2;                                               // accumulator b read by the epilogue
-    uint32_t* holder = reinterpret_cast<uint32_t*>(aempty + 2);
+    uint64_t* wfull = aempty + 2;                                              // B landed
+    uint32_t* holder = reinterpret_cast<uint32_t*>(wfull + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int first = blockIdx.x, stride = gridDim.x;
     const int nmine = first < ntiles ? (ntiles - first + stride - 1) / stride : 0;
@@ -205,6 +206,7 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
             mbar_init(&full[b], 1);
             mbar_init(&aempty[b], kConvWarps);
         }
+        mbar_init(wfull, 1);
         fence_barrier_init();
     }
     if (warp == 0) {
@@ -216,8 +218,6 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
     wpk += dep;
     bias += dep;
     zbuf += dep;
-    for (uint32_t q = tid; q < b_bytes / 16; q += kConvThreads) reinterpret_cast<uint4*>(sB)[q] = wpk[q];
-    fence_proxy_async_smem();   // B (generic stores) -> visible to the tensor cores
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -230,6 +230,11 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
         static_assert(3 * rows <= 32, "a lane per line");
         const int xp = lane / rows, yr = lane % rows;
         int i = 0;
+        if (lane == 0 && nmine > 0) {   // B first, in one copy (stored by all threads before the tiles: 83 us
+                                        // for the four layers at 64^3, so 78.5)
+            mbar_arrive_expect_tx(wfull, b_bytes);
+            bulk_g2s(sB, wpk, b_bytes, wfull);
+        }
 #pragma unroll 1
         for (; i < nmine; ++i) {
             const int b = i & 1;
@@ -250,8 +255,10 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
             }
         }
         // the copies still in flight land before the CTA exits
-        if (lane == 0)
+        if (lane == 0) {
+            if (nmine > 0) (void)mbar_wait(wfull, 0u);
             for (int q = i > 2 ? i - 2 : 0; q < i; ++q) (void)mbar_wait(&full[q & 1], (uint32_t)(q >> 1) & 1u);
+        }
     } else if (warp == kConvWarps + 1) {
         // ------------------------------------------------------------ MMAs
         if (lane == 0) {
@@ -260,7 +267,7 @@ k_conv3_tc(const uint4* __restrict__ in, const uint4* __restrict__ wpk, const fl
 #pragma unroll 1
             for (; i < nmine; ++i) {
                 const int b = i & 1;
-                bool ok = mbar_wait(&full[b], (uint32_t)(i >> 1) & 1u);
+                bool ok = (i > 0 || mbar_wait(wfull, 0u)) && mbar_wait(&full[b], (uint32_t)(i >> 1) & 1u);
                 // the epilogue of tile i - 2 has read accumulator b
                 if (ok && i >= 2) ok = mbar_wait(&aempty[b], (uint32_t)((i >> 1) - 1) & 1u);
                 if (!ok) {
