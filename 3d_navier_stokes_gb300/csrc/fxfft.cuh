@@ -18,9 +18,10 @@
 // elements to a common scale. Doubles are read and written on the sphere's modes only
 // (the x passes), and the integers' range does not end at FP64's exponents.
 //
-// Measured on a GB300 against FP64 butterflies (one RK4 step): 128^3 3.55 -> 0.78 ms, 256^3
-// 28.3 -> 5.6 ms, 512^3 250 -> 54 ms; the nonlinear term's error against a 113-bit
-// evaluation at 16^3 .. 48^3 falls from 3.1e-16 .. 9.9e-16 to 1.5e-16 .. 2.9e-16.
+// Measured on a GB300 against FP64 butterflies (one RK4 step): 32^3 0.312 -> 0.074 ms, 128^3
+// 3.55 -> 0.62 ms, 256^3 28.3 -> 4.64 ms, 512^3 250 -> 44.8 ms; the nonlinear term's error
+// against a 113-bit evaluation at 16^3 .. 48^3 falls from 3.1e-16 .. 9.9e-16 to 7.4e-17 ..
+// 2.4e-16.
 //
 // Lines that hold a NaN or Inf carry the scale kFxBad and end as NaN throughout, as any
 // transform of them does; lines of doubles whose L1 norm is below 2^-900 (values under
