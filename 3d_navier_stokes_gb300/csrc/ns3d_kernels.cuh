@@ -162,13 +162,14 @@ template <typename T, int N, int V = 0, bool INV = true> constexpr int tile_a() 
 // two CTAs per SM), else 4.
 template <int N, bool FWD = false> constexpr int fx_tile() { return FxPlan<N>::X::P * 8 <= (FWD ? 128 : 256) ? 8 : 4; }
 // FP32: at most 128 threads per CTA up to 64 points (64^3, tiles of 16 -> 8 pencils: 61.4 ->
-// 55.3 us per step), 8 pencils with S.
+// 55.3 us per step), 8 pencils with S, and in the inverse pass of variant 0 at 192 and 256
+// points (27.9 -> 25.3 and 65.5 -> 53.6 us per launch; 384 points 222 -> 240 us).
 template <typename T, int N, int V = 0, bool FWD = false, bool S = false> constexpr int tile_x() {
     if constexpr (sizeof(T) == 8) return fx_tile<N, FWD>();
     else {
         constexpr int P = PlansV<N, V>::X::P;
         constexpr int W = clip_tile<P, (FWD ? TileVar<V>::XF : TileVar<V>::X)>();
-        return (S || (N <= 64 && P * W > 128)) && W > 8 ? 8 : W;
+        return (S || (N <= 64 && P * W > 128) || (V == 0 && !FWD && (N == 192 || N == 256))) && W > 8 ? 8 : W;
     }
 }
 // Launches of few members with x tiles of 8 pencils instead of 16 (the transforms are the
