@@ -273,6 +273,12 @@ struct ns3d_les : public ns3d::LesHook {
         k_pack_jobs<<<dim3(64, 4), 256, 0, s>>>(jobs);
     }
 
+    // every packed form of the weights (both are read by the tensor-core gradients)
+    void pack_all(cudaStream_t s) {
+        pack_tc(s);
+        pack_tc_t(s);
+    }
+
     // tensor-core inference: four implicit-GEMM convolutions on blocked BF16 activations
     template <int LOGD>
     void infer_tc_d(const float* u, float* tau, float in_scale, float out_scale, cudaStream_t s) {
@@ -448,8 +454,7 @@ ns3d_status ns3d_les_create(int Nc, int capacity, uint64_t seed, ns3d_les** out)
             cudaGetLastError();
             return NS3D_ERR_NOMEM;
         }
-        l->pack_tc(l->stream);
-        l->pack_tc_t(l->stream);
+        l->pack_all(l->stream);
     }
     if (cudaStreamSynchronize(l->stream) != cudaSuccess) {
         delete l;
@@ -560,10 +565,7 @@ ns3d_status ns3d_les_train(ns3d_les* l, int iterations, double lr, double* mean_
             const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
             ns3d::cnn::k_adam<<<(NPARAM + 255) / 256, 256, 0, l->stream>>>(
                 l->w, l->wb, l->g, l->m, l->v, NPARAM, (float)lr, b1, b2, 1e-8f, c1, c2, l->losses + k, l->dstat, l->halt);
-            if (l->tc_train()) {   // the next sample's tensor-core layers read the updated weights
-                l->pack_tc(l->stream);
-                l->pack_tc_t(l->stream);
-            }
+            if (l->tc_train()) l->pack_all(l->stream);   // the next sample's layers read the updated weights
         }
         LES_CK(cudaMemcpyAsync(l->losses_host, l->losses, sizeof(double) * n, cudaMemcpyDeviceToHost, l->stream));
         LES_CK(cudaMemcpyAsync(l->part_host + NPART, l->dstat, sizeof(int), cudaMemcpyDeviceToHost, l->stream));
@@ -571,7 +573,7 @@ ns3d_status ns3d_les_train(ns3d_les* l, int iterations, double lr, double* mean_
         for (int k = 0; k < n; ++k) {
             if (!isfinite(l->losses_host[k]) || *reinterpret_cast<const int*>(l->part_host + NPART) != 0) {
                 l->adam_t += k;   // the updates before the first bad sample were applied
-                l->pack_tc(l->stream);
+                l->pack_all(l->stream);
                 cudaStreamSynchronize(l->stream);
                 if (*reinterpret_cast<const int*>(l->part_host + NPART) != 0)
                     return les_fail(l, NS3D_ERR_TIMEOUT, "a bounded wait in a tensor-core training kernel gave up");
@@ -585,7 +587,7 @@ ns3d_status ns3d_les_train(ns3d_les* l, int iterations, double lr, double* mean_
         }
         l->adam_t += n;
     }
-    l->pack_tc(l->stream);
+    l->pack_all(l->stream);
     LES_CK(cudaStreamSynchronize(l->stream));
     if (mean_loss) *mean_loss = nacc ? acc / nacc : 0.0;
     return NS3D_OK;
@@ -615,7 +617,7 @@ ns3d_status ns3d_les_weights_host(ns3d_les* l, float* w, int set) {
     if (set) {
         LES_CK(cudaMemcpy(l->w, w, sizeof(float) * NPARAM, cudaMemcpyHostToDevice));
         ns3d::cnn::k_to_bf16<<<(NPARAM + 255) / 256, 256, 0, l->stream>>>(l->w, l->wb, NPARAM);
-        l->pack_tc(l->stream);
+        l->pack_all(l->stream);
         LES_CK(cudaStreamSynchronize(l->stream));
     } else {
         LES_CK(cudaMemcpy(w, l->w, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
