@@ -391,7 +391,7 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 // real_out [3][N][N][N]). A CTA takes ZP pairs of adjacent lines; three groups of P
 // threads own one complex transform each. Per line the velocity and the vorticity
 // get one scale each (2^60 bounds the L1 norm of every component), group g turns
-// fields 2g, 2g+1 into real space, the threads form u x w >> 60 from the 32-bit
+// fields 2g, 2g+1 into real space, the threads form u x w >> 60 from the 30-bit
 // halves, and the groups transform (Nx, Ny) of both lines and (Nz_a, Nz_b) back,
 // every real line with a shift of its own that bounds its L1 norm by 2^60. The
 // transforms exchange through the group's own third of the line's buffer, which
@@ -424,11 +424,11 @@ template <int P> struct SyncLine {   // the P threads of a line transform
         else __syncthreads();
     }
 };
-// (a b - c d) >> 60 for |a|, |b|, |c|, |d| < 2^60, from 31-bit halves (the products of
-// the low halves are below the last bits kept); a4 = 4 a.ad, c4 = 4 c.ad
-__device__ __forceinline__ q64 fx_cross(FxSplit a, int a4, FxSplit b, FxSplit c, int c4, FxSplit d) {
+// (a b - c d) >> 60 for |a|, |b|, |c|, |d| < 2^60, from 30-bit halves (the products of the
+// low halves would each add less than one unit)
+__device__ __forceinline__ q64 fx_cross(FxSplit a, FxSplit b, FxSplit c, FxSplit d) {
     const q64 mid = madw(a.ad, b.a0, mulw(a.a0, b.ad)) - madw(c.ad, d.a0, mulw(c.a0, d.ad));
-    return madw(a4, b.ad, mid >> 29) - mulw(c4, d.ad);
+    return madw(a.ad, b.ad, mid >> 30) - mulw(c.ad, d.ad);
 }
 
 // scale of a product spectrum (twice itself) from the scales of u and w and the line's shift
@@ -550,9 +550,8 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                     const cx<q64> v1 = r[0], v2 = r[XS], v3 = r[2 * XS];
                     const FxSplit ux = fx_split(v1.x), uy = fx_split(v1.y), uz = fx_split(v2.x);
                     const FxSplit wx = fx_split(v2.y), wy = fx_split(v3.x), wz = fx_split(v3.y);
-                    const int ux4 = 4 * ux.ad, uy4 = 4 * uy.ad, uz4 = 4 * uz.ad;
-                    r[0] = mk<q64>(fx_cross(uy, uy4, wz, uz, uz4, wy), fx_cross(uz, uz4, wx, ux, ux4, wz));
-                    r[XS].x = fx_cross(ux, ux4, wy, uy, uy4, wx);
+                    r[0] = mk<q64>(fx_cross(uy, wz, uz, wy), fx_cross(uz, wx, ux, wz));
+                    r[XS].x = fx_cross(ux, wy, uy, wx);
                     if (want_umax) {
                         const q64 sp = llabs(v1.x) + llabs(v1.y) + llabs(v2.x);
                         um = fmax(um, fx_to_any(mk<q64>(sp, 0), scale[line / 2][line % 2].x).x);

@@ -7,7 +7,7 @@
 // a DFT is a sum of inputs times numbers of modulus <= 1, so it is bounded by the
 // line's L1 norm. Each line is therefore scaled by the power of two that keeps its
 // L1 norm below 2^61, held in 64-bit integers and transformed with exact 64-bit
-// additions and 64x61-bit twiddle products (both parts of the product that reach the
+// additions and 64x60-bit twiddle products (both parts of the product that reach the
 // result's last bit). No stage needs a shift and nothing can overflow. The absolute
 // error is about one unit of 2^-61 of the L1 norm per input and per twiddle product,
 // below the rounding errors of the FP64 butterflies it replaces (measured against
@@ -44,41 +44,41 @@ __device__ __forceinline__ q64 mulw(int a, int b) {
     return d;
 }
 
-// A twiddle component c in [-1, 1] is c1 2^-31 + c0 2^-62 with |c1| < 2^31 and
-// |c0| <= 2^30 (c = +-1: +-(2^31 - 1) for both, off by 2^-62). fx_tw packs
-// (cos, sin) as (c1, c0) pairs from the numbers rounded to 2^-62.
-__host__ __device__ constexpr int fx_hi(q64 q) {
-    const q64 h = (q + (1ll << 30)) >> 31;
-    return (int)(h > 2147483647ll ? 2147483647ll : (h < -2147483647ll ? -2147483647ll : h));
-}
-__host__ __device__ constexpr int fx_lo(q64 q) {
-    const q64 l = q - (q64)fx_hi(q) * (1ll << 31);
-    return (int)(l > 2147483647ll ? 2147483647ll : (l < -2147483647ll ? -2147483647ll : l));
-}
+// A twiddle component c in [-1, 1] is c1 2^-30 + c0 2^-60 with |c1| <= 2^30 and
+// |c0| <= 2^29, so that quarter turns are exact: equal numbers cancel, as they do in
+// FP64. fx_hi and fx_lo give c1 and c0 from c rounded to 2^-60 (a component's error then
+// stays below half a unit of a result bounded by 2^61, and is far smaller for lines
+// whose values are spread).
+constexpr double kQOne = 1152921504606846976.0;   // 2^60
+__host__ __device__ constexpr int fx_hi(q64 q) { return (int)((q + (1ll << 29)) >> 30); }
+__host__ __device__ constexpr int fx_lo(q64 q) { return (int)(q - (q64)fx_hi(q) * (1ll << 30)); }
 
-// An integer a as 2^31 ad + a0, 0 <= a0 < 2^31: one funnel shift and one mask
+// An integer a, |a| < 2^61, as 2^30 ad + a0, 0 <= a0 < 2^30: one funnel shift and one mask
 struct FxSplit {
     int ad, a0;
 };
 __device__ __forceinline__ FxSplit fx_split(q64 a) {
     FxSplit s;
-    s.ad = (int)__funnelshift_l((unsigned)a, (unsigned)(a >> 32), 1);
-    s.a0 = (int)((unsigned)a & 0x7fffffffu);
+    s.ad = (int)__funnelshift_l((unsigned)a, (unsigned)(a >> 32), 2);
+    s.a0 = (int)((unsigned)a & 0x3fffffffu);
     return s;
 }
-// a * c for a real c = (c1, c0); the product a0 c0 lies below the last bit
-__device__ __forceinline__ q64 fx_rmul(q64 a, int c1, int c0) {
-    const FxSplit s = fx_split(a);
-    const q64 mid = madw(s.a0, c1, mulw(s.ad, c0));
-    return madw(s.ad, c1, mid >> 31);
+// a * c, |a| < 2^62 (the sum of an element's parts may reach sqrt(2) 2^61), for a constant
+// c in (0, 1) given as 2^62 c, from 31-bit halves; the product a0 c0 lies below half the last bit
+template <q64 Q> __device__ __forceinline__ q64 fx_rmul(q64 a) {
+    constexpr int c1 = (int)((Q + (1ll << 30)) >> 31), c0 = (int)(Q - (q64)c1 * (1ll << 31));
+    const int ad = (int)__funnelshift_l((unsigned)a, (unsigned)(a >> 32), 1);
+    const int a0 = (int)((unsigned)a & 0x7fffffffu);
+    const q64 mid = madw(a0, c1, mulw(ad, c0));
+    return madw(ad, c1, mid >> 31);
 }
-// a * (cr + i ci). With |a| <= 2^61 the middle sums stay below 2^63: the low words
-// add at most sqrt(2) 2^62, the high ones sqrt(2) 2^60 (|ad| <= 2^30, |c0| <= 2^30).
+// a * (cr + i ci). The middle sums stay below 2^62: |ad| <= 2^31 times |c0| <= 2^29 and
+// a0 < 2^30 times |c1| <= 2^30, at most sqrt(2) 2^60 from each pair.
 __device__ __forceinline__ cx<q64> fx_cmul(cx<q64> a, int cr1, int cr0, int ci1, int ci0) {
     const FxSplit r = fx_split(a.x), i = fx_split(a.y);
     const q64 mr = madw(i.a0, -ci1, madw(i.ad, -ci0, madw(r.a0, cr1, mulw(r.ad, cr0))));
     const q64 mi = madw(i.a0, cr1, madw(i.ad, cr0, madw(r.a0, ci1, mulw(r.ad, ci0))));
-    return mk<q64>(madw(i.ad, -ci1, madw(r.ad, cr1, mr >> 31)), madw(i.ad, cr1, madw(r.ad, ci1, mi >> 31)));
+    return mk<q64>(madw(i.ad, -ci1, madw(r.ad, cr1, mr >> 30)), madw(i.ad, cr1, madw(r.ad, ci1, mi >> 30)));
 }
 __device__ __forceinline__ cx<q64> cmul(cx<q64> a, int4 w) { return fx_cmul(a, w.x, w.y, w.z, w.w); }
 __device__ __forceinline__ void bfly_w(cx<q64> e, cx<q64> o, int4 w, cx<q64>& lo, cx<q64>& hi) {
@@ -87,9 +87,11 @@ __device__ __forceinline__ void bfly_w(cx<q64> e, cx<q64> o, int4 w, cx<q64>& lo
     hi = e - t;
 }
 
-// cos(2 pi k / 16), cos(2 pi k / 12) times 2^62, the codelets' constants
-__device__ constexpr q64 kQ1 = 1ll << 62, kQc16 = 4260642322793532497ll, kQr2 = 3260954456333195553ll,
-                         kQs16 = 1764815834521887442ll, kQh3 = 3993837246235628775ll;
+// cos(2 pi k / 16), cos(2 pi k / 12) times 2^60, the codelets' constants, and sqrt(1/2) and
+// sqrt(3/4) times 2^62 (fx_rmul)
+__device__ constexpr q64 kQ1 = 1ll << 60, kQc16 = 1065160580698383124ll, kQr2 = 815238614083298888ll,
+                         kQs16 = 441203958630471860ll, kQh3 = 998459311558907194ll;
+constexpr q64 kQr2x4 = 3260954456333195553ll, kQh3x4 = 3993837246235628775ll;
 __device__ constexpr q64 kQC16[16] = {kQ1, kQc16, kQr2, kQs16, 0, -kQs16, -kQr2, -kQc16,
                                       -kQ1, -kQc16, -kQr2, -kQs16, 0, kQs16, kQr2, kQc16};
 __device__ constexpr q64 kQC12[12] = {kQ1, kQh3, kQ1 / 2, 0, -kQ1 / 2, -kQh3, -kQ1, -kQh3, -kQ1 / 2, 0, kQ1 / 2, kQh3};
@@ -110,8 +112,7 @@ __device__ __forceinline__ void bfly(cx<q64> e, cx<q64> o, cx<q64>& lo, cx<q64>&
         t = mul_i(o);
     } else if constexpr (R % 3 != 0 && (8 * k) % R == 0) {
         constexpr int e8 = 8 * k / R;   // 1, 3, 5, 7 eighths of a turn
-        constexpr int c1 = fx_hi(kQr2), c0 = fx_lo(kQr2);
-        const q64 u = fx_rmul(o.x + o.y, c1, c0), v = fx_rmul(o.y - o.x, c1, c0);
+        const q64 u = fx_rmul<kQr2x4>(o.x + o.y), v = fx_rmul<kQr2x4>(o.y - o.x);
         t = e8 == 1 ? mk<q64>(u, v) : e8 == 3 ? mk<q64>(v, -u) : e8 == 5 ? mk<q64>(-u, -v) : mk<q64>(-v, u);
     } else {
         constexpr bool tri = (R % 3 == 0);
@@ -130,8 +131,7 @@ template <bool PK> struct Dft<3, cx<q64>, PK> {
     __device__ __forceinline__ static void run(C* a) {
         const C s = a[1] + a[2], d = a[1] - a[2];
         const C m = mk<q64>(a[0].x - (s.x >> 1), a[0].y - (s.y >> 1));
-        constexpr int c1 = fx_hi(kQh3), c0 = fx_lo(kQh3);
-        const C jd = mk<q64>(fx_rmul(d.y, c1, c0), -fx_rmul(d.x, c1, c0));   // -i sin(60) d
+        const C jd = mk<q64>(fx_rmul<kQh3x4>(d.y), -fx_rmul<kQh3x4>(d.x));   // -i sin(60) d
         a[0] = a[0] + s;
         a[1] = m + jd;
         a[2] = m - jd;
@@ -151,7 +151,7 @@ template <> struct TwOf<cx<q64>> {
     using tab = int4;
     using type = int4;
     __device__ __forceinline__ static int4 at(const int4* tw, int i) { return __ldg(&tw[i]); }
-    __device__ __forceinline__ static int4 one() { return make_int4(2147483647, 2147483647, 0, 0); }
+    __device__ __forceinline__ static int4 one() { return make_int4(1 << 30, 0, 0, 0); }
 };
 
 // ---------------------------------------------------------------------------
@@ -252,10 +252,11 @@ __device__ __forceinline__ int fx_scale_of(FxBound b, int spare) {
     const int k = fx_scale(b, spare, kFxNoFlush);
     return k == kFxBad || k == kFxZero ? k : min(k, 38 - b.e);
 }
-// v 2^k as an integer, cut towards zero (|v| 2^k < 2^61)
+// v 2^k as an integer, cut towards zero (|v| 2^k < 2^61); zero throughout a line of scale
+// kFxZero, whose elements' own exponents would leave them the leading bit of a normal number
 __device__ __forceinline__ q64 fx_from(double v, int k) {
     const int hi = __double2hiint(v), lo = __double2loint(v);
-    const int sh = min(max(1083 - k - (int)(((unsigned)hi << 1) >> 21), 0), 63);
+    const int sh = k == kFxZero ? 63 : min(max(1083 - k - (int)(((unsigned)hi << 1) >> 21), 0), 63);
     const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
     const q64 r = (q64)((((unsigned long long)mh << 32 | (unsigned)lo) << 8) >> sh);
     const q64 sgn = hi >> 31;

@@ -56,12 +56,12 @@ void twiddle_table(int n, double* re, double* im) {
         im[m] = -(double)s;
     }
 }
-// the same as packed 62-bit integers (fxfft.cuh): four ints per entry
+// the same as packed 60-bit integers (fxfft.cuh): four ints per entry
 void fx_twiddle_table(int n, int* out) {
     for (long m = 0; m < n; ++m) {
         long double c, s;
         unit_circle(n, m, &c, &s);
-        const q64 qc = (q64)roundl(c * 4611686018427387904.0L), qs = (q64)roundl(-s * 4611686018427387904.0L);
+        const q64 qc = (q64)roundl(c * kQOne), qs = (q64)roundl(-s * kQOne);
         out[4 * m] = fx_hi(qc);
         out[4 * m + 1] = fx_lo(qc);
         out[4 * m + 2] = fx_hi(qs);

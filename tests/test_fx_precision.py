@@ -1,0 +1,48 @@
+"""What the integer line transforms of the FP64 engines (csrc/fxfft.cuh, fx_passes.cuh) keep of
+double precision: exact zeros, small components beside large ones, the whole range of doubles, and
+the rounding errors at every grid size."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def wavenumbers(N):
+    k = np.array([i if i <= N // 2 else i - N for i in range(N)], dtype=np.float64)
+    return k[:, None, None], k[None, :, None], np.arange(N // 2 + 1, dtype=np.float64)[None, None, :]
+
+
+def white(N, seed=0):
+    """Dealiased transform of a white real field [N][N][N/2+1][3]."""
+    rng = np.random.default_rng(seed + N)
+    f = np.fft.rfftn(rng.standard_normal((N, N, N, 3)), axes=(0, 1, 2))
+    kx, ky, kz = wavenumbers(N)
+    f[kx * kx + ky * ky + kz * kz > (N // 3) ** 2] = 0
+    return f
+
+
+def rel(a, b):
+    return float(np.linalg.norm((a - b).ravel()) / np.linalg.norm(b.ravel()))
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("N", [8, 24, 32, 48, 96, 192])
+def test_lines_of_zeros(ns3d, N, axis):
+    """A flow in a plane stays in it: with no modes along an axis and no velocity in it, the
+    term has exact zeros in those modes, as sums of equal numbers have."""
+    f = white(N)
+    k = wavenumbers(N)[axis]
+    f[np.broadcast_to(k != 0, f.shape[:3])] = 0
+    f[..., axis] = 0
+    s = ns3d.Solver(N, dt=1e-4)
+    out = s.NonlinearRHSBatch(f)
+    assert np.any(out != 0)
+    assert np.all(out[np.broadcast_to(k != 0, f.shape[:3])] == 0)
+    s.set_state(f)
+    if axis == 2:   # u_z and the vorticity of the plane are lines of their own in every transform
+        assert np.all(out[..., 2] == 0)
+        u, w = s.real_space()
+        assert np.all(u[..., 2] == 0) and np.all(w[..., :2] == 0)
+    s.RK4Step(2)
+    g = s.get_state()
+    assert np.all(g[np.broadcast_to(k != 0, f.shape[:3])] == 0)
