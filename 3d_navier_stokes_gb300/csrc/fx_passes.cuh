@@ -106,7 +106,7 @@ k_xinv_fx(const cx<double>* __restrict__ U, cx<q64>* __restrict__ W, int* __rest
         for (int s = 0; s < E; ++s)
             if (!(P * s > G::KC && P * s + P - 1 < N - G::KC)) v[s] = v[s] * (1.0 / ((double)N * N * N));
     }
-    const int k = fx_scale(fx_line_bound<P, TT, NT>(fx_bound(v), sync), 0, kFxFlush);
+    const int k = fx_scale_in(fx_line_bound<P, TT, NT>(fx_bound(v), sync), 0);
     cx<q64> a[E];
 #pragma unroll
     for (int s = 0; s < E; ++s)
@@ -277,9 +277,15 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 #pragma unroll
             for (int s = 0; s < E; ++s) a[s] = fx_align(a[s], ke[s], k);
             PL::template fwd<false>(a, reinterpret_cast<cx<q64>*>(sbuf), p, tw, sidx, sync);
+            const int kn = fx_near(k);
 #pragma unroll
             for (int s = 0; s < E; ++s)
-                if (!fx_outside<PL>(s)) sbuf[(p + P * s) * TT + t] = fx_to_any(a[s], k);
+                if (!fx_outside<PL>(s)) sbuf[(p + P * s) * TT + t] = mk(fx_to(a[s].x, kn), fx_to(a[s].y, kn));
+            if (k != kn) {   // rare; a branch around the conversions would part them from the last stage's
+                             // additions, which cover them (96^3 22 -> 28 us, 256^3 0.163 -> 0.175 ms)
+#pragma unroll 1
+                for (int s = 0; s < E; ++s) sbuf[(p + P * s) * TT + t] = sbuf[(p + P * s) * TT + t] * fx_far(k);
+            }
         };
         if constexpr (NG % 32 == 0) transform(SyncGroup{1 + g, NG});
         else transform(SyncBlock());
@@ -554,7 +560,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                     r[XS].x = fx_cross(ux, wy, uy, wx);
                     if (want_umax) {
                         const q64 sp = llabs(v1.x) + llabs(v1.y) + llabs(v2.x);
-                        um = fmax(um, fx_to_any(mk<q64>(sp, 0), scale[line / 2][line % 2].x).x);
+                        um = fmax(um, fx_to_any(sp, scale[line / 2][line % 2].x));
                     }
                 }
                 if (want_umax) {
@@ -612,7 +618,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
 #pragma unroll
                     for (int w = 1; w < NW; ++w) b = fx_join(b, bound[lp][g][w]);
                 }
-                const int k = fx_scale(b, 1, kFxFlush);
+                const int k = fx_scale_in(b, 1);
 #pragma unroll
                 for (int s = 0; s < E; ++s) a[s] = mk<q64>(fx_from(v[s].x, k), fx_from(v[s].y, k));
                 kA = kB = k == kFxZero || k == kFxBad ? k : k + 1;
@@ -629,8 +635,8 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
             double* r = real + (long long)2 * g * N * N * N + (la + L) * N;
 #pragma unroll
             for (int s = 0; s < E; ++s) {
-                r[p + P * s] = fx_to_any(mk<q64>(a[s].y, 0), kA).x;
-                r[(long long)N * N * N + p + P * s] = fx_to_any(mk<q64>(a[s].x, 0), kB).x;
+                r[p + P * s] = fx_to_any(a[s].y, kA);
+                r[(long long)N * N * N + p + P * s] = fx_to_any(a[s].x, kB);
             }
             __syncthreads();
         } else {

@@ -24,8 +24,9 @@
 // 2.4e-16.
 //
 // Lines that hold a NaN or Inf carry the scale kFxBad and end as NaN throughout, as any
-// transform of them does; lines of doubles whose L1 norm is below 2^-900 (values under
-// about 1e-274) are taken as zero, scale kFxZero.
+// transform of them does; lines of zeros the scale kFxZero. The range of inputs and results is
+// that of doubles, subnormals among them, and what a line's transform passes through on the
+// way has no exponent range to leave.
 #pragma once
 #include "fft_engine.cuh"
 
@@ -164,14 +165,17 @@ struct FxBound {
     int e;
 };
 // Doubles: FP32 numbers cut from the high words with the exponent rebased on the multiply
-// pipe (largest field base + kFxSpan: room for sums); smaller values count as zero.
+// pipe (largest field base + kFxSpan: room for sums); smaller values count as zero, and a
+// thread with nothing in its high words (below 2^-1042) as one unit of them.
 constexpr int kFxSpan = 190;
 template <int E>
 __device__ __forceinline__ FxBound fx_bound(const cx<double> (&v)[E]) {
-    unsigned top = 0u;
+    unsigned top = 0u, low_words = 0u;
 #pragma unroll
-    for (int s = 0; s < E; ++s)
+    for (int s = 0; s < E; ++s) {
         top = max(top, max((unsigned)__double2hiint(v[s].x) & 0x7fffffffu, (unsigned)__double2hiint(v[s].y) & 0x7fffffffu));
+        low_words |= (unsigned)__double2loint(v[s].x) | (unsigned)__double2loint(v[s].y);
+    }
     const int lo = max((int)(top >> 20) - kFxSpan, 0);
     const unsigned low = (unsigned)lo << 20;
     const int base = (int)(0u - ((unsigned)lo << 23));
@@ -184,6 +188,7 @@ __device__ __forceinline__ FxBound fx_bound(const cx<double> (&v)[E]) {
         b.sum += __int_as_float(x);
         b.sum += __int_as_float(y);
     }
+    if (top == 0u && low_words != 0u) b.sum = __int_as_float(8);
     return b;
 }
 // Integers (|a| <= 2^61) with their scales: sums of the high words' upper bits, aligned to
@@ -239,28 +244,33 @@ __device__ __forceinline__ FxBound fx_line_bound(FxBound b, Sync sync) {
     return b;
 }
 // The largest scale at which a line of this bound sums to less than 2^(61 - spare), kFxZero
-// or kFxBad; doubles below 2^flush count as zero.
-__device__ __forceinline__ int fx_scale(FxBound b, int spare, int flush) {
+// or kFxBad
+__device__ __forceinline__ int fx_scale(FxBound b, int spare) {
     if (b.e >= -kFxBad - 1000) return kFxBad;
     const float f = b.sum * 1.0001f;
     const int e = (int)(__float_as_uint(f) >> 23) - 127 + b.e;
-    return f < 1e-30f || e < flush ? kFxZero : 60 - spare - e;
+    return f == 0.f || e < -20000 ? kFxZero : 60 - spare - e;
 }
-constexpr int kFxFlush = -900, kFxNoFlush = -20000;
-// and for integers: no finer than the finest common scale of the elements
+// of doubles: no finer than the smallest normal number needs (fx_from)
+__device__ __forceinline__ int fx_scale_in(FxBound b, int spare) {
+    const int k = fx_scale(b, spare);
+    return k == kFxZero ? k : min(k, 1082);
+}
+// and of integers: no finer than the finest common scale of the elements
 __device__ __forceinline__ int fx_scale_of(FxBound b, int spare) {
-    const int k = fx_scale(b, spare, kFxNoFlush);
+    const int k = fx_scale(b, spare);
     return k == kFxBad || k == kFxZero ? k : min(k, 38 - b.e);
 }
-// v 2^k as an integer, cut towards zero (|v| 2^k < 2^61); zero throughout a line of scale
-// kFxZero, whose elements' own exponents would leave them the leading bit of a normal number
+// v 2^k as an integer, cut towards zero (|v| 2^k < 2^61, k <= 1082 unless v is zero)
 __device__ __forceinline__ q64 fx_from(double v, int k) {
     const int hi = __double2hiint(v), lo = __double2loint(v);
-    const int sh = k == kFxZero ? 63 : min(max(1083 - k - (int)(((unsigned)hi << 1) >> 21), 0), 63);
-    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    const q64 r = (q64)((((unsigned long long)mh << 32 | (unsigned)lo) << 8) >> sh);
+    const unsigned mag = (unsigned)hi & 0x7fffffffu;
+    const unsigned mh = min(mag, ((unsigned)hi & 0xfffffu) | 0x100000u);   // subnormals: no leading bit,
+    const int sh = min(1083 - k - (int)(mag >> 20), 1082 - k);             // the smallest normal's exponent
+    unsigned long long r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(((unsigned long long)mh << 32 | (unsigned)lo) << 8), "r"(sh));   // 0 past 63
     const q64 sgn = hi >> 31;
-    return (r ^ sgn) - sgn;
+    return ((q64)r ^ sgn) - sgn;
 }
 // an integer at scale k0 to the line's scale k <= k0, rounded to nearest
 __device__ __forceinline__ cx<q64> fx_align(cx<q64> a, int k0, int k) {
@@ -275,11 +285,15 @@ __device__ __forceinline__ double fx_to(q64 i, int k) {
     const int hi = __double2hiint(d);
     return __hiloint2double(hi ? hi - (k << 20) : 0, __double2loint(d));
 }
-// the same over all scales: zero below FP64's range, NaN above it and for bad lines
-__device__ __forceinline__ cx<double> fx_to_any(cx<q64> a, int k) {
-    if (k > 1020) return czero<double>();
-    if (k < -900) return mk(__hiloint2double(0x7ff80000, 0), __hiloint2double(0x7ff80000, 0));
-    return mk(fx_to(a.x, k), fx_to(a.y, k));
+// Scales beyond the ones fx_to takes: convert at fx_near(k), then multiply by fx_far(k), a power
+// of two whose product rounds to a subnormal, zero or infinity; NaN for bad lines
+__device__ __forceinline__ int fx_near(int k) { return min(max(k, -900), 1020); }
+__device__ __forceinline__ double fx_far(int k) {
+    return __hiloint2double(k == kFxBad ? 0x7ff80000 : (1023 + min(max(fx_near(k) - k, -1022), 1023)) << 20, 0);
+}
+__device__ __forceinline__ double fx_to_any(q64 a, int k) {
+    const double d = fx_to(a, fx_near(k));
+    return fx_near(k) == k ? d : d * fx_far(k);
 }
 // slot s of every thread lies outside the kept band |k| <= KC = N / 3: a quarter of the
 // slots of 16, neither loaded nor added by an inverse transform, nor stored by a forward

@@ -46,3 +46,45 @@ def test_lines_of_zeros(ns3d, N, axis):
     s.RK4Step(2)
     g = s.get_state()
     assert np.all(g[np.broadcast_to(k != 0, f.shape[:3])] == 0)
+
+
+# one term of six passes, as in test_fx_fft.py
+TOL_RHS = 5e-15
+TOL_INV = 2.4e-15
+
+
+@pytest.mark.parametrize("a", [-500, -480, 480, 495])
+@pytest.mark.parametrize("N", [24, 32])
+def test_rhs_range(ns3d, N, a):
+    """RHS(2^a f) = 2^(2a) RHS(f) as far as the products are normal numbers."""
+    f = white(N)
+    s = ns3d.Solver(N)
+    got = s.NonlinearRHSBatch(f * 2.0 ** a) * 2.0 ** -a
+    assert rel(got * 2.0 ** -a, s.NonlinearRHSBatch(f)) < TOL_RHS
+
+
+@pytest.mark.parametrize("a", [-1000, -955, 905, 1005])
+@pytest.mark.parametrize("N", [24, 32])
+def test_real_space_range(ns3d, N, a):
+    f = white(N)
+    s = ns3d.Solver(N)
+    s.set_state(f * 2.0 ** a)
+    got = s.real_space()
+    s.set_state(f)
+    for x, y in zip(got, s.real_space()):
+        assert rel(x * 2.0 ** (-a // 2) * 2.0 ** (-a - -a // 2), y) < TOL_INV
+
+
+@pytest.mark.parametrize("a", [-1040, -1060, -1072])
+def test_subnormal_fields(ns3d, a):
+    """Subnormal modes: the transform keeps their bits and rounds its results once (to within
+    one of the spacing, half of it for the double-rounded conversion)."""
+    N = 32
+    f = white(N) * 2.0 ** a          # cut to multiples of 2^-1074
+    s = ns3d.Solver(N)
+    s.set_state(f)
+    u, _ = s.real_space()
+    big = (f * 2.0 ** 600) * 2.0 ** (-a - 600)
+    ref = np.fft.irfftn(big, s=(N, N, N), axes=(0, 1, 2)) * 2.0 ** (a + 1074)
+    assert np.abs(u[:, :, :N] * 2.0 ** 600 * 2.0 ** 474 - ref).max() <= 1.0
+    assert np.any(u != 0) or a < -1065
