@@ -395,10 +395,10 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 // ---------------------------------------------------------------------------
 // P3, MODE as in k_zpass (0: c2r, u x w, r2c; 1: c2r to real_out [6][N][N][N]; 2: r2c of
 // real_out [3][N][N][N]). A CTA takes ZP pairs of adjacent lines; three groups of P
-// threads own one complex transform each. Per line the velocity and the vorticity
-// get one scale each (2^60 bounds the L1 norm of every component), group g turns
-// fields 2g, 2g+1 into real space, the threads form u x w >> 60 from the 30-bit
-// halves, and the groups transform (Nx, Ny) of both lines and (Nz_a, Nz_b) back,
+// threads own one complex transform each. Each of a line's fields gets a scale of its own
+// (2^60 bounds its L1 norm), group g turns fields 2g, 2g+1 into real space, the threads
+// form the products >> 60 of u x w from the 30-bit halves and bring the two of a
+// component to one scale, and the groups transform (Nx, Ny) of both lines and (Nz_a, Nz_b) back,
 // every real line with a shift of its own that bounds its L1 norm by 2^60. The
 // transforms exchange through the group's own third of the line's buffer, which
 // then holds its real-space output, so 96 bytes of shared memory per grid point of
@@ -430,18 +430,28 @@ template <int P> struct SyncLine {   // the P threads of a line transform
         else __syncthreads();
     }
 };
-// (a b - c d) >> 60 for |a|, |b|, |c|, |d| < 2^60, from 30-bit halves (the products of the
-// low halves would each add less than one unit)
-__device__ __forceinline__ q64 fx_cross(FxSplit a, FxSplit b, FxSplit c, FxSplit d) {
-    const q64 mid = madw(a.ad, b.a0, mulw(a.a0, b.ad)) - madw(c.ad, d.a0, mulw(c.a0, d.ad));
-    return madw(a.ad, b.ad, mid >> 30) - mulw(c.ad, d.ad);
+// (a b) >> 60 for |a|, |b| < 2^60, from 30-bit halves (the product of the low halves would
+// add less than one unit)
+__device__ __forceinline__ q64 fx_product(FxSplit a, FxSplit b) {
+    return madw(a.ad, b.ad, madw(a.ad, b.a0, mulw(a.a0, b.ad)) >> 30);
 }
-
-// scale of a product spectrum (twice itself) from the scales of u and w and the line's shift
-__device__ __forceinline__ int fx_product_scale(int2 k, int sh) {
-    if (k.x == kFxBad || k.y == kFxBad) return kFxBad;
-    if (k.x == kFxZero || k.y == kFxZero) return kFxZero;
-    return k.x + k.y - 60 - sh + 1;
+// a b - c d with shifts that bring both to one scale
+__device__ __forceinline__ q64 fx_cross(FxSplit a, FxSplit b, FxSplit c, FxSplit d, int2 sh) {
+    return (fx_product(a, b) >> sh.x) - (fx_product(c, d) >> sh.y);
+}
+// scale k of a difference of products a and b of scales ka, kb, and the shifts that bring them to it
+struct FxCross {
+    int k;
+    int2 sh;
+};
+__device__ __forceinline__ FxCross fx_cross_scale(int ka, int kb) {
+    const int k = min(ka, kb);
+    return FxCross{k, make_int2(min(ka - k, 63), min(kb - k, 63))};
+}
+// scale of a spectrum (twice itself) from the scale of the products (sums of two lines' scales,
+// so that a bad or zero line shows) and the real line's shift
+__device__ __forceinline__ int fx_product_scale(int k, int sh) {
+    return k < kFxBad / 2 ? kFxBad : k > kFxZero / 2 ? kFxZero : k - 60 - sh + 1;
 }
 
 template <int N, int MODE>
@@ -463,7 +473,8 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
     cx<q64>* buf = reinterpret_cast<cx<q64>*>(smem_raw);   // [ZP][2 lines][3 groups][XS]
     __shared__ FxBound bound[ZP][6][NW];                    // a line's L1 norm per field
     __shared__ uint2 count[ZP][3][NW];                      // a real line's sums (P > 32)
-    __shared__ int2 scale[ZP][2];                           // per line: ku, kw
+    __shared__ int scale[2 * ZP][6];                        // per line: its fields' scales
+    __shared__ int product[2 * ZP][3];                      // and those of its products
     const int p = threadIdx.x % P;
     const int g = (threadIdx.x / P) % 3;
     const int lp = threadIdx.x / (3 * P);
@@ -507,23 +518,18 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                 bound[lp][2 * g + 1][p / 32] = bb;
             }
             __syncthreads();
-            // one scale each for u and w: every mode but the mean counts twice (its conjugate), so a
-            // component's modes sum to half of 2^60
-            int kk[2];
+            // a scale for each field, so that a component far below the others keeps its bits: every
+            // mode but the mean counts twice (its conjugate), so its modes sum to half of 2^60
+            int kfield[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                kk[h] = kFxZero;
+                FxBound b = bound[lp][2 * g + h][0];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    FxBound b = bound[lp][3 * h + c][0];
-#pragma unroll
-                    for (int w = 1; w < NW; ++w) b = fx_join(b, bound[lp][3 * h + c][w]);
-                    kk[h] = min(kk[h], fx_scale_of(b, 2));
-                }
+                for (int w = 1; w < NW; ++w) b = fx_join(b, bound[lp][2 * g + h][w]);
+                kfield[h] = fx_scale_of(b, 2);
+                if (p == 0) scale[2 * lp + L][2 * g + h] = kfield[h];
             }
-            const int ku = kk[0], kw = kk[1];
-            if (p == 0 && g == 0) scale[lp][L] = make_int2(ku, kw);
-            const int ka = g < 2 ? ku : kw, kb = g < 1 ? ku : kw;
+            const int ka = kfield[0], kb = kfield[1];
             if (MODE == 1) {
                 kA = ka;
                 kB = kb;
@@ -548,22 +554,34 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
             cx<q64>* ba = buf + lp * 6 * XS;   // line a's buffers; line b's 3 XS further
             sb = g == 0 ? ba : g == 1 ? ba + 3 * XS : ba + XS;
             if constexpr (MODE == 0) {
-                // u x w: (ux, uy), (uz, wx), (wy, wz) -> (Nx, Ny), (Nz, -)
-                double um = 0.0;
-                for (int idx = threadIdx.x; idx < ZP * 2 * N; idx += 3 * P * ZP) {
-                    const int line = idx / N, n = idx % N;   // line = pair 2 + L
+                // u x w: (ux, uy), (uz, wx), (wy, wz) -> (Nx, Ny), (Nz, -); 3 P / 2 threads per line
+                constexpr int NL = 3 * P / 2;
+                const int line = threadIdx.x / NL;   // of the CTA's 2 ZP
+                const int* k = scale[line];
+                const FxCross cn = fx_cross_scale(k[1] + k[5], k[2] + k[4]), cy = fx_cross_scale(k[2] + k[3], k[0] + k[5]),
+                              cz = fx_cross_scale(k[0] + k[4], k[1] + k[3]);
+                if (threadIdx.x % NL == 0) {
+                    product[line][0] = cn.k;
+                    product[line][1] = cy.k;
+                    product[line][2] = cz.k;
+                }
+                const int ku = min(k[0], min(k[1], k[2]));
+                const int sx = min(k[0] - ku, 63), sy = min(k[1] - ku, 63), sz = min(k[2] - ku, 63);
+                q64 top = 0;   // the largest |ux| + |uy| + |uz|
+                for (int n = threadIdx.x % NL; n < N; n += NL) {
                     cx<q64>* r = buf + line * 3 * XS + sidx(n);
                     const cx<q64> v1 = r[0], v2 = r[XS], v3 = r[2 * XS];
                     const FxSplit ux = fx_split(v1.x), uy = fx_split(v1.y), uz = fx_split(v2.x);
                     const FxSplit wx = fx_split(v2.y), wy = fx_split(v3.x), wz = fx_split(v3.y);
-                    r[0] = mk<q64>(fx_cross(uy, wz, uz, wy), fx_cross(uz, wx, ux, wz));
-                    r[XS].x = fx_cross(ux, wy, uy, wx);
+                    r[0] = mk<q64>(fx_cross(uy, wz, uz, wy, cn.sh), fx_cross(uz, wx, ux, wz, cy.sh));
+                    r[XS].x = fx_cross(ux, wy, uy, wx, cz.sh);
                     if (want_umax) {
-                        const q64 sp = llabs(v1.x) + llabs(v1.y) + llabs(v2.x);
-                        um = fmax(um, fx_to_any(sp, scale[line / 2][line % 2].x));
+                        const q64 sp = (llabs(v1.x) >> sx) + (llabs(v1.y) >> sy) + (llabs(v2.x) >> sz);
+                        top = sp > top ? sp : top;
                     }
                 }
                 if (want_umax) {
+                    double um = fx_to_any(top, ku);
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) um = fmax(um, __shfl_xor_sync(0xffffffffu, um, o));
                     if ((threadIdx.x & 31) == 0) Bits<double>::amax(&sd[blockIdx.y].umax_bits, um);
@@ -599,9 +617,8 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
 #pragma unroll
                 for (int s = 0; s < E; ++s) a[s] = mk<q64>((a[s].x + rx) >> shx, (a[s].y + ry) >> shy);
                 // the spectra's scales (one more for the halves)
-                const int2 s0 = scale[lp][g == 1 ? 1 : 0], s1 = scale[lp][g == 0 ? 0 : 1];
-                kA = fx_product_scale(s0, shx);
-                kB = fx_product_scale(s1, shy);
+                kA = fx_product_scale(product[2 * lp + (g == 1 ? 1 : 0)][g == 2 ? 2 : 0], shx);
+                kB = fx_product_scale(product[2 * lp + (g == 0 ? 0 : 1)][g == 2 ? 2 : 1], shy);
             } else {
                 constexpr long long kReal = (long long)N * N * N;
                 const double* r0 = real + (g == 2 ? 2 * kReal : 0) + (g == 1 ? la + 1 : la) * N;

@@ -88,3 +88,41 @@ def test_subnormal_fields(ns3d, a):
     ref = np.fft.irfftn(big, s=(N, N, N), axes=(0, 1, 2)) * 2.0 ** (a + 1074)
     assert np.abs(u[:, :, :N] * 2.0 ** 600 * 2.0 ** 474 - ref).max() <= 1.0
     assert np.any(u != 0) or a < -1065
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("N", [24, 32, 96, 192])
+def test_small_component_real_space(ns3d, N, axis):
+    """A velocity component far below the others comes back with its own bits."""
+    f = white(N)
+    f[..., axis] *= 1e-10
+    s = ns3d.Solver(N)
+    s.set_state(f)
+    u, _ = s.real_space()
+    ref = np.fft.irfftn(f, s=(N, N, N), axes=(0, 1, 2))
+    for c in range(3):
+        assert rel(u[:, :, :N, c], ref[..., c]) < TOL_INV, c
+
+
+@pytest.mark.parametrize("N", [24, 32, 96, 192])
+def test_small_component_of_a_plane_flow(ns3d, N):
+    """A small velocity across the plane of a two-dimensional flow is advected like a scalar:
+    N_z = u_x w_y - u_y w_x is small itself and has its own bits. (The term's sums are products
+    of the small field with the large one, so that TOL_RHS holds component by component.)"""
+    f = white(N)
+    f[:, :, 1:] = 0
+    f[..., 2] *= 1e-10
+    s = ns3d.Solver(N)
+    got = s.NonlinearRHSBatch(f)
+    s.set_state(f)
+    u, w = s.real_space()
+    kx, ky, kz = wavenumbers(N)
+    curl = 1j * np.stack([ky * f[..., 2], -kx * f[..., 2], kx * f[..., 1] - ky * f[..., 0]], -1)
+    ur = np.fft.ifft2(f[:, :, 0], axes=(0, 1)).real / N
+    wr = np.fft.ifft2(curl[:, :, 0], axes=(0, 1)).real / N
+    for c in range(3):
+        assert rel(u[:, :, 3, c], ur[..., c]) < TOL_INV and rel(w[:, :, 3, c], wr[..., c]) < TOL_INV, c
+    nz = np.fft.fft2(ur[..., 0] * wr[..., 1] - ur[..., 1] * wr[..., 0]) * N
+    nz[(kx ** 2 + ky ** 2)[..., 0] > (N // 3) ** 2] = 0
+    nz[0, 0] = 0
+    assert rel(got[:, :, 0, 2], nz) < TOL_RHS
