@@ -412,6 +412,12 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 // lines XS slots apart. One pad slot per 16 counts 2.0 - 2.1 wavefronts per access at 8, 24 and
 // 48 points and 1.33 at 64, these 1.2 and 1.0; at 96 and 192 points (1.4 to 1.2) nothing was
 // gained.
+// From 256 points on a line's own peaks, not the bound by its modes, set the scales of the products'
+// operands: operands of 2^60 / sqrt(N) each lose log2 N bits between them. White flow in a plane,
+// relative error of the right-hand side at 128, 192, 256, 384 and 512 points without the peaks 2.6,
+// 4.1, 5.9, 6.8 and 8.8e-16 (FP64 butterflies 5.0, 6.1, 5.7, 5.9 and 6.3e-16), with them at 256
+// 4.0e-16; they cost 5 % of this pass.
+template <int N> constexpr bool zfx_peaks() { return N >= 256; }
 template <int N> struct FxLay { static constexpr int A = 4, XS = zpad<N>(); };
 template <> struct FxLay<8> { static constexpr int A = 2, XS = 12; };
 template <> struct FxLay<24> { static constexpr int A = 4, XS = 28; };
@@ -430,7 +436,14 @@ template <int P> struct SyncLine {   // the P threads of a line transform
         else __syncthreads();
     }
 };
-// (a b) >> 60 for |a|, |b| < 2^60, from 30-bit halves (the product of the low halves would
+// The halves of a 2^h, 0 <= h <= 28
+__device__ __forceinline__ FxSplit fx_split(q64 a, int h) {
+    FxSplit s;
+    s.ad = (int)__funnelshift_l((unsigned)a, (unsigned)(a >> 32), h + 2);
+    s.a0 = (int)((unsigned)a << h & 0x3fffffffu);
+    return s;
+}
+// a b 2^-60 for |a|, |b| <= 2^60, from 30-bit halves (the product of the low halves would
 // add less than one unit)
 __device__ __forceinline__ q64 fx_product(FxSplit a, FxSplit b) {
     return madw(a.ad, b.ad, madw(a.ad, b.a0, mulw(a.a0, b.ad)) >> 30);
@@ -474,6 +487,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
     __shared__ FxBound bound[ZP][6][NW];                    // a line's L1 norm per field
     __shared__ uint2 count[ZP][3][NW];                      // a real line's sums (P > 32)
     __shared__ int scale[2 * ZP][6];                        // per line: its fields' scales
+    __shared__ unsigned peak[2 * ZP][3][NW];                // and a group's two peaks (leading zeros)
     __shared__ int product[2 * ZP][3];                      // and those of its products
     const int p = threadIdx.x % P;
     const int g = (threadIdx.x / P) % 3;
@@ -557,7 +571,18 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                 // u x w: (ux, uy), (uz, wx), (wy, wz) -> (Nx, Ny), (Nz, -); 3 P / 2 threads per line
                 constexpr int NL = 3 * P / 2;
                 const int line = threadIdx.x / NL;   // of the CTA's 2 ZP
-                const int* k = scale[line];
+                int h[6], k[6];   // bits to a field's peak, and its scale with them
+#pragma unroll
+                for (int f = 0; f < 6; ++f) {
+                    h[f] = 0;
+                    if constexpr (zfx_peaks<N>()) {
+                        unsigned t = peak[line][f / 2][0];
+#pragma unroll
+                        for (int w = 1; w < NW; ++w) t = __vimin3_u16x2(t, t, peak[line][f / 2][w]);
+                        h[f] = (int)(f % 2 ? t >> 16 : t & 0xffffu) - 4;   // values below 2^60
+                    }
+                    k[f] = scale[line][f] + h[f];
+                }
                 const FxCross cn = fx_cross_scale(k[1] + k[5], k[2] + k[4]), cy = fx_cross_scale(k[2] + k[3], k[0] + k[5]),
                               cz = fx_cross_scale(k[0] + k[4], k[1] + k[3]);
                 if (threadIdx.x % NL == 0) {
@@ -565,14 +590,14 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                     product[line][1] = cy.k;
                     product[line][2] = cz.k;
                 }
-                const int ku = min(k[0], min(k[1], k[2]));
-                const int sx = min(k[0] - ku, 63), sy = min(k[1] - ku, 63), sz = min(k[2] - ku, 63);
+                const int kx = scale[line][0], ky = scale[line][1], kz = scale[line][2], ku = min(kx, min(ky, kz));
+                const int sx = min(kx - ku, 63), sy = min(ky - ku, 63), sz = min(kz - ku, 63);
                 q64 top = 0;   // the largest |ux| + |uy| + |uz|
                 for (int n = threadIdx.x % NL; n < N; n += NL) {
                     cx<q64>* r = buf + line * 3 * XS + sidx(n);
                     const cx<q64> v1 = r[0], v2 = r[XS], v3 = r[2 * XS];
-                    const FxSplit ux = fx_split(v1.x), uy = fx_split(v1.y), uz = fx_split(v2.x);
-                    const FxSplit wx = fx_split(v2.y), wy = fx_split(v3.x), wz = fx_split(v3.y);
+                    const FxSplit ux = fx_split(v1.x, h[0]), uy = fx_split(v1.y, h[1]), uz = fx_split(v2.x, h[2]);
+                    const FxSplit wx = fx_split(v2.y, h[3]), wy = fx_split(v3.x, h[4]), wz = fx_split(v3.y, h[5]);
                     r[0] = mk<q64>(fx_cross(uy, wz, uz, wy, cn.sh), fx_cross(uz, wx, ux, wz, cy.sh));
                     r[XS].x = fx_cross(ux, wy, uy, wx, cz.sh);
                     if (want_umax) {
@@ -646,6 +671,23 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
         if (L < 2 && MODE == 0) {
 #pragma unroll
             for (int s = 0; s < E; ++s) sb[sidx(p + P * s)] = mk<q64>(a[s].y, a[s].x);
+            if constexpr (zfx_peaks<N>()) {
+                int hia = 0, hib = 0, loa = -1, lob = -1;
+#pragma unroll
+                for (int s = 0; s < E; s += 2) {
+                    const int ha = (int)(a[s].y >> 32), hb = (int)(a[s].x >> 32);
+                    const int ga = (int)(a[s + 1].y >> 32), gb = (int)(a[s + 1].x >> 32);
+                    hia = __vimax3_s32(hia, ha, ga);
+                    loa = __vimin3_s32(loa, ha, ga);
+                    hib = __vimax3_s32(hib, hb, gb);
+                    lob = __vimin3_s32(lob, hb, gb);
+                }
+                unsigned zeros = __clz(max(hia, ~loa)) | __clz(max(hib, ~lob)) << 16;
+#pragma unroll
+                for (int o = 1; o < (P < 32 ? P : 32); o <<= 1)
+                    zeros = __vimin3_u16x2(zeros, zeros, __shfl_xor_sync(0xffffffffu, zeros, o));
+                if (p % 32 == 0) peak[2 * lp + L][g][p / 32] = zeros;
+            }
             // the line's real space is complete, and its bounds are read
             __syncthreads();
         } else if (L < 2) {

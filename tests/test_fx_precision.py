@@ -126,3 +126,87 @@ def test_small_component_of_a_plane_flow(ns3d, N):
     nz[(kx ** 2 + ky ** 2)[..., 0] > (N // 3) ** 2] = 0
     nz[0, 0] = 0
     assert rel(got[:, :, 0, 2], nz) < TOL_RHS
+
+
+def plane_flow(N):
+    """White flow in the x-z plane: transforms [N][N/2+1] of u_x and u_z (u_y = 0, no y dependence)."""
+    rng = np.random.default_rng(N)
+    k = np.fft.fftfreq(N, 1.0 / N)[:, None]
+    kz = np.arange(N // 2 + 1, dtype=np.float64)[None, :]
+    keep = k * k + kz * kz <= (N // 3) ** 2
+    return [np.fft.rfft2(rng.standard_normal((N, N))) * keep for _ in range(2)], k, kz, keep
+
+
+def check_plane_flow(ns3d, N):
+    """Real space and the right-hand side against transforms in extended precision. Tolerance: one
+    unit of 2^-53 per radix-2 level, the levels' errors independent: two inverse transforms for a
+    field, and those of both factors and two forward ones for the term."""
+    sfft = pytest.importorskip("scipy.fft")
+    unit = 2.0 ** -53 * np.sqrt(np.log2(N))
+    (fx, fz), k, kz, keep = plane_flow(N)
+    f = np.zeros((N, N, N // 2 + 1, 3), np.complex128)
+    f[:, 0, :, 0], f[:, 0, :, 2] = fx * N, fz * N
+    s = ns3d.Solver(N)
+    got = s.NonlinearRHSBatch(f)[:, 0].copy()
+    s.set_state(f)
+    del f
+    u, w = (a[:, 5, :N].copy() for a in s.real_space())
+    s.close()
+    fx, fz = fx.astype(np.clongdouble), fz.astype(np.clongdouble)
+    ux, uz, wy = (sfft.irfft2(a, s=(N, N)) for a in (fx, fz, 1j * (kz * fx - k * fz)))
+    for a, b in ((u[..., 0], ux), (u[..., 2], uz), (w[..., 1], wy)):
+        assert rel(a, b) < unit * np.sqrt(2)
+    nx, nz = sfft.rfft2(-uz * wy), sfft.rfft2(ux * wy)
+    k2 = np.where(keep & (k * k + kz * kz > 0), k * k + kz * kz, np.inf)
+    d = (k * nx + kz * nz) / k2
+    ref = np.stack([(n - q * d) * np.isfinite(k2) * N for n, q in ((nx, k), (nz, kz))], -1)
+    assert np.all(got[..., 1] == 0)
+    assert rel(got[..., ::2], ref) < unit * np.sqrt(6)
+
+
+@pytest.mark.parametrize("N", [24, 64, 128, 192, 256, 384, 512])
+def test_plane_flow(ns3d, N):
+    check_plane_flow(ns3d, N)
+
+
+@pytest.mark.parametrize("N", [128, 192, 256, 384, 512])
+def test_against_device_transforms(ns3d, N):
+    """White fields through every pass (real space, the right-hand side, real space back to modes),
+    component by component, against FP64 transforms of the device library. Tolerance as in
+    test_plane_flow, three transforms per field and nine for the term, of both sides."""
+    import torch
+    unit = 2 * 2.0 ** -53 * np.sqrt(np.log2(N))
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    k = torch.fft.fftfreq(N, 1.0 / N, dtype=torch.float64, device="cuda")
+    ks = (k[:, None, None], k[None, :, None], torch.arange(N // 2 + 1, dtype=torch.float64, device="cuda"))
+    keep = ks[0] ** 2 + ks[1] ** 2 + ks[2] ** 2 <= (N // 3) ** 2
+    f = [torch.fft.rfftn(torch.randn(N, N, N, dtype=torch.float64, device="cuda", generator=gen)) * keep for _ in range(3)]
+    host = torch.stack(f, -1).cpu().numpy()
+    s = ns3d.Solver(N)
+    got = s.NonlinearRHSBatch(host)
+    s.set_state(host)
+    del host
+    u, w = s.real_space()
+    s.set_state_real(u)
+    back = s.get_state()
+    s.close()
+
+    def err(a, b):
+        return float((torch.from_numpy(np.ascontiguousarray(a)).cuda() - b).norm() / b.norm())
+
+    ur = [torch.fft.irfftn(a, s=(N, N, N)) for a in f]
+    wr = []
+    for c in range(3):
+        a, b = (c + 1) % 3, (c + 2) % 3
+        wr.append(torch.fft.irfftn(1j * (ks[a] * f[b] - ks[b] * f[a]), s=(N, N, N)))
+    for c in range(3):
+        assert err(u[:, :, :N, c], ur[c]) < unit * np.sqrt(3), c
+        assert err(w[:, :, :N, c], wr[c]) < unit * np.sqrt(3), c
+        assert err(back[..., c], f[c]) < unit * np.sqrt(6), c
+    del u, w, back
+    n = [torch.fft.rfftn(ur[(c + 1) % 3] * wr[(c + 2) % 3] - ur[(c + 2) % 3] * wr[(c + 1) % 3]) for c in range(3)]
+    del ur, wr
+    k2 = (ks[0] ** 2 + ks[1] ** 2 + ks[2] ** 2)
+    d = sum(ks[c] * n[c] for c in range(3)) / k2.clamp(min=1)
+    for c in range(3):
+        assert err(got[..., c], (n[c] - ks[c] * d) * keep * (k2 > 0)) < unit * 3, c
