@@ -271,11 +271,18 @@ template <typename T> struct TwOf<cx<T>> {
 //   tw     : table W_N^m = exp(-2 pi i m / N), m < N (read-only path); with
 //            TS > 1 the table of a TS times longer transform, read every TS-th entry
 //   sync() : barrier over all threads sharing sbuf
+//   mid    : applied to the first stage's outputs where another stage follows; names the
+//            type of the stage twiddles, and so the form of their products
 // Plan::inv computes the inverse as conj(DFT(conj(x))).
 // ---------------------------------------------------------------------------
-template <typename C, bool PK, int TS, int N, int E, int Ns, typename SIdx, typename Sync, int R, int... Rest>
+struct AsIs {
+    template <typename W> using Tw = W;
+    template <typename C> __device__ __forceinline__ C operator()(C a) const { return a; }
+};
+template <typename C, bool PK, int TS, int N, int E, int Ns, typename SIdx, typename Sync, typename Mid, int R,
+          int... Rest>
 __device__ __forceinline__ void fft_stages(C (&v)[E], C* sbuf, int p, const typename TwOf<C>::tab* __restrict__ tw,
-                                           SIdx sidx, Sync sync) {
+                                           SIdx sidx, Sync sync, Mid mid) {
     constexpr int P = N / E;
     constexpr int Q = E / R;
     constexpr bool last = (sizeof...(Rest) == 0);
@@ -290,7 +297,7 @@ __device__ __forceinline__ void fft_stages(C (&v)[E], C* sbuf, int p, const type
         if constexpr (Ns > 1) {
             jm = j % Ns;
             constexpr int step = N / (Ns * R);
-            typename TwOf<C>::type w[R];
+            typename Mid::template Tw<typename TwOf<C>::type> w[R];
             w[0] = TwOf<C>::one();
 #pragma unroll
             for (int r = 1; r < R; ++r) w[r] = TwOf<C>::at(tw, TS * r * jm * step);
@@ -304,7 +311,7 @@ __device__ __forceinline__ void fft_stages(C (&v)[E], C* sbuf, int p, const type
         } else {
             const int idxD = (j / Ns) * Ns * R + jm;
 #pragma unroll
-            for (int r = 0; r < R; ++r) sbuf[sidx(idxD + r * Ns)] = a[r];
+            for (int r = 0; r < R; ++r) sbuf[sidx(idxD + r * Ns)] = Ns == 1 ? mid(a[r]) : a[r];
         }
     }
     if constexpr (!last) {
@@ -312,7 +319,7 @@ __device__ __forceinline__ void fft_stages(C (&v)[E], C* sbuf, int p, const type
 #pragma unroll
         for (int s = 0; s < E; ++s) v[s] = sbuf[sidx(p + s * P)];
         sync();
-        fft_stages<C, PK, TS, N, E, Ns * R, SIdx, Sync, Rest...>(v, sbuf, p, tw, sidx, sync);
+        fft_stages<C, PK, TS, N, E, Ns * R, SIdx, Sync, Mid, Rest...>(v, sbuf, p, tw, sidx, sync, mid);
     }
 }
 
@@ -328,17 +335,17 @@ struct Plan {
     static_assert((Rs * ... * 1) == N_ && N_ % E_ == 0, "the radices' product is the length");
     // PK: FP32x2 additions in the butterflies (see vadd); TS: twiddle table of a
     // TS times longer transform
-    template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync>
+    template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync, typename Mid = AsIs>
     __device__ __forceinline__ static void fwd(C (&v)[E_], C* sbuf, int p, const typename TwOf<C>::tab* __restrict__ tw,
-                                               SIdx sidx, Sync sync) {
-        fft_stages<C, PK, TS, N_, E_, 1, SIdx, Sync, Rs...>(v, sbuf, p, tw, sidx, sync);
+                                               SIdx sidx, Sync sync, Mid mid = Mid()) {
+        fft_stages<C, PK, TS, N_, E_, 1, SIdx, Sync, Mid, Rs...>(v, sbuf, p, tw, sidx, sync, mid);
     }
     template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync>
     __device__ __forceinline__ static void inv(C (&v)[E_], C* sbuf, int p, const typename TwOf<C>::tab* __restrict__ tw,
                                                SIdx sidx, Sync sync) {
 #pragma unroll
         for (int s = 0; s < E_; ++s) v[s] = conjg(v[s]);
-        fft_stages<C, PK, TS, N_, E_, 1, SIdx, Sync, Rs...>(v, sbuf, p, tw, sidx, sync);
+        fft_stages<C, PK, TS, N_, E_, 1, SIdx, Sync, AsIs, Rs...>(v, sbuf, p, tw, sidx, sync, AsIs());
 #pragma unroll
         for (int s = 0; s < E_; ++s) v[s] = conjg(v[s]);
     }

@@ -106,13 +106,17 @@ k_xinv_fx(const cx<double>* __restrict__ U, cx<q64>* __restrict__ W, int* __rest
         for (int s = 0; s < E; ++s)
             if (!(P * s > G::KC && P * s + P - 1 < N - G::KC)) v[s] = v[s] * (1.0 / ((double)N * N * N));
     }
-    const int k = fx_scale_in(fx_line_bound<P, TT, NT>(fx_bound(v), sync), 0);
+    constexpr bool TWO = fx_two<N>();
+    FxBound b = fx_bound(v);
+    int first = TWO ? fx_scale_in(b, 0) : 0;
+    b = fx_line_bound<TWO, P, TT, NT>(b, first, sync);
+    const int k = fx_scale_in(b, 0), later = fx_later<TWO>(first, k);
     cx<q64> a[E];
 #pragma unroll
     for (int s = 0; s < E; ++s)
         // an inverse transform is the forward one with real and imaginary parts exchanged
-        a[s] = fx_outside<PL>(s) ? mk<q64>(0, 0) : mk<q64>(fx_from(v[s].y, k), fx_from(v[s].x, k));
-    PL::template fwd<false>(a, sbuf, p, tw, sidx, sync);
+        a[s] = fx_outside<PL>(s) ? mk<q64>(0, 0) : mk<q64>(fx_from(v[s].y, k + later), fx_from(v[s].x, k + later));
+    PL::template fwd<fx_round<N>()>(a, sbuf, p, tw, sidx, sync, fx_mid<N>(later));
     if (rem >= 0) {
 #pragma unroll
         for (int s = 0; s < E; ++s) W[off + (long long)(p + P * s) * xs] = mk<q64>(a[s].y, a[s].x);
@@ -165,14 +169,18 @@ k_ypass_fx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __rest
             ke[s] = kin[INV ? (long long)jj * G::NZP : jj];
         }
     }
-    const int k = fx_scale_of(fx_line_bound<P, TT, NT>(fx_bound(a, ke), sync), 0);
+    constexpr bool TWO = fx_two<N>();
+    FxBound b = fx_bound(a, ke);
+    int first = TWO ? fx_scale_of(b, 0) : 0;
+    b = fx_line_bound<TWO, P, TT, NT>(b, first, sync);
+    const int k = fx_scale_of(b, 0), later = fx_later<TWO>(first, k);
 #pragma unroll
     for (int s = 0; s < E; ++s) {
         if (INV && fx_outside<PL>(s)) continue;
-        const cx<q64> v = fx_align(a[s], ke[s], k);
+        const cx<q64> v = fx_align(a[s], ke[s], k + later);
         a[s] = INV ? mk<q64>(v.y, v.x) : v;
     }
-    PL::template fwd<false>(a, sbuf, p, tw, sidx, sync);
+    PL::template fwd<fx_round<N>()>(a, sbuf, p, tw, sidx, sync, fx_mid<N>(later));
     if (!colok) return;
 #pragma unroll
     for (int s = 0; s < E; ++s) {
@@ -273,10 +281,14 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
         if (g == 0) xfwd_prefetch_state<double, N, INTEG, MODE, E, P, TT>(U, ACC, K, rs, p, t, ky, kz0, j);
         StridedIdx<TT, PL::R1> sidx{t};
         auto transform = [&](auto sync) {
-            const int k = fx_scale_of(fx_line_bound<P, TT, NT>(fx_bound(a, ke), sync), 0);
+            constexpr bool TWO = fx_two<N>();
+            FxBound b = fx_bound(a, ke);
+            int first = TWO ? fx_scale_of(b, 0) : 0;
+            b = fx_line_bound<TWO, P, TT, NT>(b, first, sync);
+            const int k = fx_scale_of(b, 0), later = fx_later<TWO>(first, k);
 #pragma unroll
-            for (int s = 0; s < E; ++s) a[s] = fx_align(a[s], ke[s], k);
-            PL::template fwd<false>(a, reinterpret_cast<cx<q64>*>(sbuf), p, tw, sidx, sync);
+            for (int s = 0; s < E; ++s) a[s] = fx_align(a[s], ke[s], k + later);
+            PL::template fwd<fx_round<N>()>(a, reinterpret_cast<cx<q64>*>(sbuf), p, tw, sidx, sync, fx_mid<N>(later));
             const int kn = fx_near(k);
 #pragma unroll
             for (int s = 0; s < E; ++s)
@@ -485,7 +497,8 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<q64>* buf = reinterpret_cast<cx<q64>*>(smem_raw);   // [ZP][2 lines][3 groups][XS]
     __shared__ FxBound bound[ZP][6][NW];                    // a line's L1 norm per field
-    __shared__ uint2 count[ZP][3][NW];                      // a real line's sums (P > 32)
+    __shared__ uint2 count[ZP][3][NW], most[ZP][3][NW];     // a real line's sums and its threads' largest (P > 32)
+    __shared__ int firsts[ZP][6][NW];                       // scales of a line's first stage
     __shared__ int scale[2 * ZP][6];                        // per line: its fields' scales
     __shared__ unsigned peak[2 * ZP][3][NW];                // and a group's two peaks (leading zeros)
     __shared__ int product[2 * ZP][3];                      // and those of its products
@@ -497,6 +510,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
     PadIdx<FxLay<N>::A, 1> sidx;
     SyncLine<P> sync;
 
+    constexpr bool TWO = fx_two<N>();
     int kA = 0, kB = 0;   // scales of what a group writes
     // lines a and b to real space, then the products back: one copy of the transform's code
     // (instruction fetch is a cost of these long unrolled bodies)
@@ -504,6 +518,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
     for (int L = MODE == 2 ? 2 : 0; L < (MODE == 1 ? 2 : 3); ++L) {
         cx<q64>* sb;
         cx<q64> a[E];
+        int later = 0;   // bits of the scale that come after the first stage
         if (L < 2) {
             sb = buf + ((lp * 2 + L) * 3 + g) * XS;
             const cx<q64>* A = W + (long long)(2 * g) * G::FS + (la + L) * G::NZP;
@@ -525,6 +540,16 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                 }
             }
             FxBound ba = fx_bound(ra, kea), bb = fx_bound(rb, keb);
+            if constexpr (TWO) {
+                // a thread's modes come once as they are and once as the conjugates in another thread's slots:
+                // half of 2^60 for each of the two fields keeps its inputs' sum below 2^61
+                const int fa = fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_of(ba, 2), 0xffffffffu);
+                const int fb = fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_of(bb, 2), 0xffffffffu);
+                if (p % 32 == 0) {
+                    firsts[lp][2 * g][p / 32] = fa;
+                    firsts[lp][2 * g + 1][p / 32] = fb;
+                }
+            }
             fx_warp_bound<1, (P < 32 ? P : 32)>(ba, 0xffffffffu);
             fx_warp_bound<1, (P < 32 ? P : 32)>(bb, 0xffffffffu);
             if (p % 32 == 0) {
@@ -543,10 +568,21 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                 kfield[h] = fx_scale_of(b, 2);
                 if (p == 0) scale[2 * lp + L][2 * g + h] = kfield[h];
             }
-            const int ka = kfield[0], kb = kfield[1];
+            if constexpr (TWO) {
+                // the two fields share the transform, so the shift as well
+                later = 31;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    int f = firsts[lp][2 * g + h][0];
+#pragma unroll
+                    for (int w = 1; w < NW; ++w) f = min(f, firsts[lp][2 * g + h][w]);
+                    if (kfield[h] != kFxZero) later = min(later, fx_later<TWO>(f, kfield[h]));
+                }
+            }
+            const int ka = kfield[0] + later, kb = kfield[1] + later;
             if (MODE == 1) {
-                kA = ka;
-                kB = kb;
+                kA = kfield[0];
+                kB = kfield[1];
             }
 #pragma unroll
             for (int s = 0; s < E; ++s) a[s] = mk<q64>(0, 0);
@@ -621,26 +657,38 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                     hx += ((unsigned)abs((int)(a[s].x >> 32)) >> 10) + 1u;
                     hy += ((unsigned)abs((int)(a[s].y >> 32)) >> 10) + 1u;
                 }
+                unsigned mx = hx, my = hy;
                 // |x| < 2^42 per count: a shift of the bit length over 18 bounds the line's sum by 2^60
 #pragma unroll
                 for (int o = 1; o < (P < 32 ? P : 32); o <<= 1) {
                     hx += __shfl_xor_sync(0xffffffffu, hx, o);
                     hy += __shfl_xor_sync(0xffffffffu, hy, o);
+                    if constexpr (TWO) {
+                        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                        my = max(my, __shfl_xor_sync(0xffffffffu, my, o));
+                    }
                 }
                 if constexpr (NW > 1) {
-                    if (p % 32 == 0) count[lp][g][p / 32] = make_uint2(hx, hy);
+                    if (p % 32 == 0) {
+                        count[lp][g][p / 32] = make_uint2(hx, hy);
+                        most[lp][g][p / 32] = make_uint2(mx, my);
+                    }
                     __syncthreads();
                     hx = hy = 0u;
 #pragma unroll
                     for (int w = 0; w < NW; ++w) {
                         hx += count[lp][g][w].x;
                         hy += count[lp][g][w].y;
+                        mx = max(mx, most[lp][g][w].x);
+                        my = max(my, most[lp][g][w].y);
                     }
                 }
                 const int shx = max(0, 14 - __clz(hx)), shy = max(0, 14 - __clz(hy));
-                const q64 rx = (1ll << shx) >> 1, ry = (1ll << shy) >> 1;
+                if constexpr (TWO) later = min(shx - max(0, 14 - __clz(mx)), shy - max(0, 14 - __clz(my)));
+                const int s0x = shx - later, s0y = shy - later;
+                const q64 rx = (1ll << s0x) >> 1, ry = (1ll << s0y) >> 1;
 #pragma unroll
-                for (int s = 0; s < E; ++s) a[s] = mk<q64>((a[s].x + rx) >> shx, (a[s].y + ry) >> shy);
+                for (int s = 0; s < E; ++s) a[s] = mk<q64>((a[s].x + rx) >> s0x, (a[s].y + ry) >> s0y);
                 // the spectra's scales (one more for the halves)
                 kA = fx_product_scale(product[2 * lp + (g == 1 ? 1 : 0)][g == 2 ? 2 : 0], shx);
                 kB = fx_product_scale(product[2 * lp + (g == 0 ? 0 : 1)][g == 2 ? 2 : 1], shy);
@@ -652,22 +700,29 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
 #pragma unroll
                 for (int s = 0; s < E; ++s) v[s] = mk(r0[p + P * s], r1[p + P * s]);
                 FxBound b = fx_bound(v);
+                int first = TWO ? fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_in(b, 1), 0xffffffffu) : 0;
                 fx_warp_bound<1, (P < 32 ? P : 32)>(b, 0xffffffffu);
                 if constexpr (NW > 1) {
-                    if (p % 32 == 0) bound[lp][g][p / 32] = b;
+                    if (p % 32 == 0) {
+                        bound[lp][g][p / 32] = b;
+                        firsts[lp][g][p / 32] = first;
+                    }
                     __syncthreads();
                     b = bound[lp][g][0];
+                    first = min(firsts[lp][g][0], firsts[lp][g][1]);
 #pragma unroll
                     for (int w = 1; w < NW; ++w) b = fx_join(b, bound[lp][g][w]);
                 }
+                static_assert(NW <= 2, "two warps' firsts");
                 const int k = fx_scale_in(b, 1);
+                later = fx_later<TWO>(first, k);
 #pragma unroll
-                for (int s = 0; s < E; ++s) a[s] = mk<q64>(fx_from(v[s].x, k), fx_from(v[s].y, k));
+                for (int s = 0; s < E; ++s) a[s] = mk<q64>(fx_from(v[s].x, k + later), fx_from(v[s].y, k + later));
                 kA = kB = k == kFxZero || k == kFxBad ? k : k + 1;
             }
             sync();
         }
-        PL::template fwd<false>(a, sb, p, tw, sidx, sync);
+        PL::template fwd<fx_round<N>()>(a, sb, p, tw, sidx, sync, fx_mid<N>(later));
         if (L < 2 && MODE == 0) {
 #pragma unroll
             for (int s = 0; s < E; ++s) sb[sidx(p + P * s)] = mk<q64>(a[s].y, a[s].x);

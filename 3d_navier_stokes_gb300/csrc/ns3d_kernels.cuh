@@ -92,6 +92,7 @@ template <> struct FxPlan<16>  { using A = Plan<16, 2, 2, 2, 2, 2>; using X = A;
 template <> struct FxPlan<32>  { using A = Plan<32, 4, 4, 2, 4>;    using X = A; };
 template <> struct FxPlan<48>  { using A = Plans<48>::A;            using X = Plan<48, 6, 2, 2, 2, 6>; };
 template <> struct FxPlan<64>  { using A = Plans<64>::A;            using X = Plan<64, 4, 4, 4, 4>; };
+template <> struct FxPlan<768> { using A = Plan<768, 12, 12, 4, 4, 4>; using X = A; };
 template <> struct FxPlan<512> { using A = Plan<512, 16, 16, 8, 4>; using X = A; };
 
 // Tile width (pencils per CTA along kz) of the strided passes: one 128-byte

@@ -164,12 +164,12 @@ def check_plane_flow(ns3d, N):
     assert rel(got[..., ::2], ref) < unit * np.sqrt(6)
 
 
-@pytest.mark.parametrize("N", [24, 64, 128, 192, 256, 384, 512])
+@pytest.mark.parametrize("N", [24, 64, 128, 192, 256, 384, 512, 768])
 def test_plane_flow(ns3d, N):
     check_plane_flow(ns3d, N)
 
 
-@pytest.mark.parametrize("N", [128, 192, 256, 384, 512])
+@pytest.mark.parametrize("N", [128, 192, 256, 384, 512, 768])
 def test_against_device_transforms(ns3d, N):
     """White fields through every pass (real space, the right-hand side, real space back to modes),
     component by component, against FP64 transforms of the device library. Tolerance as in
