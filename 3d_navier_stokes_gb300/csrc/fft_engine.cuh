@@ -108,6 +108,17 @@ __device__ __forceinline__ void bfly_w(cx<T> e, cx<T> o, cx<T> w, cx<T>& lo, cx<
     hi = mk(fmat(T(2), e.x, -lo.x), fmat(T(2), e.y, -lo.y));
 }
 
+// The same with lo and hi formed apart: two more FMAs, but hi does not carry lo's rounding
+template <typename T> struct ApartTw : cx<T> {
+    ApartTw() = default;
+    __device__ __forceinline__ ApartTw(cx<T> w) : cx<T>(w) {}
+};
+template <typename T>
+__device__ __forceinline__ void bfly_w(cx<T> e, cx<T> o, ApartTw<T> w, cx<T>& lo, cx<T>& hi) {
+    lo = mk(fmat(o.x, w.x, fmat(-o.y, w.y, e.x)), fmat(o.y, w.x, fmat(o.x, w.y, e.y)));
+    hi = mk(fmat(-o.x, w.x, fmat(o.y, w.y, e.x)), fmat(-o.y, w.x, fmat(-o.x, w.y, e.y)));
+}
+
 // lo = e + W_R^K o, hi = e - W_R^K o with W_R = exp(-2 pi i / R): additions
 // only for the trivial angles, two additions and four FMAs for the odd
 // multiples of 45 degrees, four FMAs and the 2e - lo form otherwise.
@@ -340,14 +351,31 @@ struct Plan {
                                                SIdx sidx, Sync sync, Mid mid = Mid()) {
         fft_stages<C, PK, TS, N_, E_, 1, SIdx, Sync, Mid, Rs...>(v, sbuf, p, tw, sidx, sync, mid);
     }
-    template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync>
+    template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync, typename Mid = AsIs>
     __device__ __forceinline__ static void inv(C (&v)[E_], C* sbuf, int p, const typename TwOf<C>::tab* __restrict__ tw,
+                                               SIdx sidx, Sync sync, Mid mid = Mid()) {
+#pragma unroll
+        for (int s = 0; s < E_; ++s) v[s] = conjg(v[s]);
+        fft_stages<C, PK, TS, N_, E_, 1, SIdx, Sync, Mid, Rs...>(v, sbuf, p, tw, sidx, sync, mid);
+#pragma unroll
+        for (int s = 0; s < E_; ++s) v[s] = conjg(v[s]);
+    }
+};
+
+// A plan whose twiddle butterflies form their two results apart (ApartTw)
+struct ApartMid : AsIs {
+    template <typename W> using Tw = ApartTw<typename RealOf<W>::type>;
+};
+template <typename PL> struct Apart : PL {
+    template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync>
+    __device__ __forceinline__ static void fwd(C (&v)[PL::E], C* sbuf, int p, const typename TwOf<C>::tab* __restrict__ tw,
                                                SIdx sidx, Sync sync) {
-#pragma unroll
-        for (int s = 0; s < E_; ++s) v[s] = conjg(v[s]);
-        fft_stages<C, PK, TS, N_, E_, 1, SIdx, Sync, AsIs, Rs...>(v, sbuf, p, tw, sidx, sync, AsIs());
-#pragma unroll
-        for (int s = 0; s < E_; ++s) v[s] = conjg(v[s]);
+        PL::template fwd<PK, TS>(v, sbuf, p, tw, sidx, sync, ApartMid());
+    }
+    template <bool PK = false, int TS = 1, typename C, typename SIdx, typename Sync>
+    __device__ __forceinline__ static void inv(C (&v)[PL::E], C* sbuf, int p, const typename TwOf<C>::tab* __restrict__ tw,
+                                               SIdx sidx, Sync sync) {
+        PL::template inv<PK, TS>(v, sbuf, p, tw, sidx, sync, ApartMid());
     }
 };
 

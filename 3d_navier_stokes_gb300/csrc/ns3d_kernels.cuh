@@ -59,16 +59,19 @@ template <int N> __device__ __forceinline__ int kof(int i) { return i <= N / 2 ?
 // 64 points keep 8 and 12 elements: with 4, 6 and 4 one member of 32^3 and 48^3 would gain (49
 // -> 45, 63 -> 59 us), eight lose (63 -> 70, 127 -> 168, 64^3 174 -> 248 us), and the plan is
 // the same for all, so that a member of an ensemble equals a single run. Small radices stand
-// first where that costs nothing: their twiddles are exact or few. Error of the right-hand side
-// of white fields against FP64, 16 .. 64 points: 2.12, 3.01, 2.87, 4.07, 4.36e-7 -> 2.03, 2.81,
-// 2.89, 4.05, 4.38e-7. (8 points keep one codelet: 2 x 4 would take 1.25e-7, not 1.14e-7.)
+// first where that costs nothing: their twiddles are exact or few. The short plans form the
+// results of a twiddle butterfly apart, the 64-point y lines too, so that the further stages do not
+// round more than the longer codelets did: relative error of the right-hand side of white fields
+// against FP64 at 16 .. 64 points with those 2.14, 3.00, 2.87, 4.07 and 4.34e-7, with short plans
+// and hi = 2 e - lo 2.05, 2.81, 2.88, 4.06 and 4.38e-7, now 2.01, 2.75, 2.84, 4.04 and 4.34e-7, at
+// the same times. (8 points keep one codelet: 2 x 4 would take 1.25e-7, not 1.14e-7.)
 template <int N> struct Plans;
 template <> struct Plans<8>    { using A = Plan<8, 8, 8>;            using X = A; };
-template <> struct Plans<16>   { using A = Plan<16, 4, 4, 4>;        using X = A; };
-template <> struct Plans<24>   { using A = Plan<24, 6, 2, 2, 6>;     using X = A; };
-template <> struct Plans<32>   { using A = Plan<32, 8, 4, 8>;        using X = Plan<32, 4, 4, 2, 4>; };
-template <> struct Plans<48>   { using A = Plan<48, 12, 4, 12>;      using X = Plan<48, 6, 2, 2, 2, 6>; };
-template <> struct Plans<64>   { using A = Plan<64, 8, 8, 8>;        using X = Plan<64, 4, 4, 4, 4>; };
+template <> struct Plans<16>   { using A = Apart<Plan<16, 4, 4, 4>>; using X = A; };
+template <> struct Plans<24>   { using A = Apart<Plan<24, 6, 2, 2, 6>>; using X = A; };
+template <> struct Plans<32>   { using A = Plan<32, 8, 4, 8>;        using X = Apart<Plan<32, 4, 4, 2, 4>>; };
+template <> struct Plans<48>   { using A = Plan<48, 12, 4, 12>;      using X = Apart<Plan<48, 6, 2, 2, 2, 6>>; };
+template <> struct Plans<64>   { using A = Plan<64, 8, 8, 8>;        using X = Apart<Plan<64, 4, 4, 4, 4>>; };
 template <> struct Plans<96>   { using A = Plan<96, 12, 4, 4, 6>;    using X = A; };
 template <> struct Plans<128>  { using A = Plan<128, 16, 16, 8>;     using X = Plan<128, 8, 8, 4, 4>; };
 template <> struct Plans<256>  { using A = Plan<256, 16, 16, 16>;    using X = Plan<256, 8, 8, 8, 4>; };
@@ -89,6 +92,7 @@ template <> struct Plans<768>  { using A = Plan<768, 12, 4, 4, 4, 4, 3>; using X
 template <int N> struct FxPlan { using A = typename Plans<N>::A; using X = A; };
 template <> struct FxPlan<8>   { using A = Plan<8, 2, 2, 2, 2>;      using X = A; };
 template <> struct FxPlan<16>  { using A = Plan<16, 2, 2, 2, 2, 2>; using X = A; };
+template <> struct FxPlan<24>  { using A = Plan<24, 6, 2, 2, 6>;    using X = A; };
 template <> struct FxPlan<32>  { using A = Plan<32, 4, 4, 2, 4>;    using X = A; };
 template <> struct FxPlan<48>  { using A = Plans<48>::A;            using X = Plan<48, 6, 2, 2, 2, 6>; };
 template <> struct FxPlan<64>  { using A = Plans<64>::A;            using X = Plan<64, 4, 4, 4, 4>; };
@@ -138,6 +142,7 @@ template <> struct TileVar<6> { static constexpr int A = 16, AF = 16, X = 8, XF 
 // with it (0.058 -> 0.060 ms). The z lines hold three fields per line and keep 12.
 template <typename T, int N, bool INV> struct YPlan { using A = typename Plans<N>::A; };
 template <int N, bool INV> struct YPlan<double, N, INV> { using A = typename FxPlan<N>::A; };
+template <bool INV> struct YPlan<float, 64, INV> { using A = Apart<typename Plans<64>::A>; };
 template <> struct YPlan<float, 96, true> { using A = Plan<96, 24, 12, 8>; };
 // 384 points in FP32: 24 elements and one stage less in both directions (inverse 0.308 ->
 // 0.286, forward 0.143 -> 0.129 ms; even at 192)
