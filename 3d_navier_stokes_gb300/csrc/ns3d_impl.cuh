@@ -691,6 +691,10 @@ class Impl final : public Base {
         return NS3D_OK;
     }
     static constexpr long long kRefBytes = 48LL * N * N * (N / 2 + 1);   // reference Fourier array
+    // a staging buffer that an output call allocated stays up to this size (192^3: 171 MB), where
+    // allocating it would be a large part of the call; above it (256^3: 406 MB, 1024^3: 26 GB) the
+    // memory goes back, unless state transfers through the buffer keep it anyway
+    static constexpr long long kStageKeep = 256ll << 20;
     // device address of a page-locked host array (16-byte aligned), else nullptr
     static const void* host_dev_ptr(const void* h) {
         cudaPointerAttributes a, z;
@@ -934,6 +938,7 @@ class Impl final : public Base {
 
     // ------------------------------------------------------- real space
     ns3d_status real_space_host(double* u, double* w) override {
+        const bool had_stage = stage_ != nullptr;
         ns3d_status st = ensure_real();
         if (st == NS3D_OK) st = ensure_stage();
         if (st != NS3D_OK) return st;
@@ -951,7 +956,12 @@ class Impl final : public Base {
             e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaMemcpyAsync(dst, d, rb, cudaMemcpyDeviceToHost, s_);
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
+        const cudaError_t done = cudaStreamSynchronize(s_);   // after an error too: no copy into u or w outlives the call
+        if (e == cudaSuccess) e = done;
+        if (!had_stage && kRefBytes > kStageKeep) {
+            cudaFree(stage_);
+            stage_ = nullptr;
+        }
         if (e != cudaSuccess) {
             set_err("real_space: %s", cudaGetErrorString(e));
             return NS3D_ERR_CUDA;
