@@ -603,10 +603,10 @@ class Impl final : public Base {
             set_err("per-kernel profile covers the RK4-family step");
             return NS3D_ERR_UNSUPPORTED;
         }
-        const char* kNames[6] = {"k_xinv", "k_ypass_inv",
-                                 zform_ == 0 ? "k_zline" : zform_ == 2 ? "k_zgemm" : "k_zpass",
-                                 "k_ypass_fwd",
-                                 "k_xfwd", "k_misc"};
+        constexpr bool fx = sizeof(T) == 8;   // the FP64 engines' passes
+        const char* kNames[6] = {fx ? "k_xinv_fx" : "k_xinv", fx ? "k_ypass_fx_inv" : "k_ypass_inv",
+                                 fx ? "k_zfx" : zform_ == 0 ? "k_zline" : zform_ == 2 ? "k_zgemm" : "k_zpass",
+                                 fx ? "k_ypass_fx_fwd" : "k_ypass_fwd", fx ? "k_xfwd_fx" : "k_xfwd", "k_misc"};
         std::vector<cudaEvent_t> ev(2 * 6 * 4 + 2);
         for (auto& e : ev) NS3D_CK(cudaEventCreate(&e));
         double acc[6] = {0, 0, 0, 0, 0, 0};
@@ -646,12 +646,14 @@ class Impl final : public Base {
         // compulsory bytes per launch (loads of non-zero inputs + stores of needed outputs)
         const double w = (double)sizeof(cx<T>);
         const double sph = sphere_modes(), circ = circle_cols(), full = (double)N * N * G::NZ1;
+        // FP64: and the lines' scales, one int per line of the pass that wrote them (FxScales)
+        const double sx = fx ? 4.0 * circ / N : 0.0, sy = fx ? 4.0 * N * G::NZ1 : 0.0, sz = fx ? 4.0 * N * N : 0.0;
         const double b[6] = {
-            w * (3 * sph + 6 * circ),               // P1: u_hat in, 6 fields on the (x, ky^2+kz^2<=KC^2) set
-            w * (6 * circ + 6 * full),              // P2
-            w * (6 * full + 3 * full),              // P3
-            w * (3 * full + 3 * circ),              // P4
-            w * (3 * circ + 9.75 * sph),            // P5: 3 fields in + state (mean over the 4 stages)
+            w * (3 * sph + 6 * circ) + 6 * sx,              // P1: u_hat in, 6 fields on the (x, ky^2+kz^2<=KC^2) set
+            w * (6 * circ + 6 * full) + 6 * (sx + sy),      // P2
+            w * (6 * full + 3 * full) + 6 * sy + 3 * sz,    // P3
+            w * (3 * full + 3 * circ) + 3 * (sz + sy),      // P4
+            w * (3 * circ + 9.75 * sph) + 3 * sy,           // P5: 3 fields in + state (mean over the 4 stages)
             0.0};
         int n = 0;
         for (int k = 0; k < 6 && n < maxc; ++k, ++n) {
