@@ -540,10 +540,6 @@ __host__ __device__ constexpr int tc_pow2(int v) {
     while (p < v) p <<= 1;
     return p;
 }
-// byte offset of the 16-byte chunk (row r, K elements 8 k8 ..) of a canonical K-major operand with K columns
-__host__ __device__ constexpr uint32_t tc_chunk(int r, int k8, int K) {
-    return (uint32_t)(((r >> 3) * (K >> 3) + k8) * 128 + (r & 7) * 16);
-}
 
 // Weight gradient on the tensor cores. For one z line (x, y) of D points, the
 // GEMM D[(t, ci)][(j, co)] += sum_z a[ci][x + dx_t][y + dy_t][z] d[co][x][y][z - (j - 1)]

@@ -280,27 +280,25 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
         // the state rows of this tile into L2 (the groups share the rows)
         if (g == 0) xfwd_prefetch_state<double, N, INTEG, MODE, E, P, TT>(U, ACC, K, rs, p, t, ky, kz0, j);
         StridedIdx<TT, PL::R1> sidx{t};
-        auto transform = [&](auto sync) {
-            constexpr bool TWO = fx_two<N>();
-            FxBound b = fx_bound(a, ke);
-            int first = TWO ? fx_scale_of(b, 0) : 0;
-            b = fx_line_bound<TWO, P, TT, NT>(b, first, sync);
-            const int k = fx_scale_of(b, 0), later = fx_later<TWO>(first, k);
+        static_assert(NG % 32 == 0, "a group has whole warps");
+        SyncGroup sync{1 + g, NG};
+        constexpr bool TWO = fx_two<N>();
+        FxBound b = fx_bound(a, ke);
+        int first = TWO ? fx_scale_of(b, 0) : 0;
+        b = fx_line_bound<TWO, P, TT, NT>(b, first, sync);
+        const int k = fx_scale_of(b, 0), later = fx_later<TWO>(first, k);
 #pragma unroll
-            for (int s = 0; s < E; ++s) a[s] = fx_align(a[s], ke[s], k + later);
-            PL::template fwd<fx_round<N>()>(a, reinterpret_cast<cx<q64>*>(sbuf), p, tw, sidx, sync, fx_mid<N>(later));
-            const int kn = fx_near(k);
+        for (int s = 0; s < E; ++s) a[s] = fx_align(a[s], ke[s], k + later);
+        PL::template fwd<fx_round<N>()>(a, reinterpret_cast<cx<q64>*>(sbuf), p, tw, sidx, sync, fx_mid<N>(later));
+        const int kn = fx_near(k);
 #pragma unroll
-            for (int s = 0; s < E; ++s)
-                if (!fx_outside<PL>(s)) sbuf[(p + P * s) * TT + t] = mk(fx_to(a[s].x, kn), fx_to(a[s].y, kn));
-            if (k != kn) {   // rare; a branch around the conversions would part them from the last stage's
-                             // additions, which cover them (96^3 22 -> 28 us, 256^3 0.163 -> 0.175 ms)
+        for (int s = 0; s < E; ++s)
+            if (!fx_outside<PL>(s)) sbuf[(p + P * s) * TT + t] = mk(fx_to(a[s].x, kn), fx_to(a[s].y, kn));
+        if (k != kn) {   // rare; a branch around the conversions would part them from the last stage's
+                         // additions, which cover them (96^3 22 -> 28 us, 256^3 0.163 -> 0.175 ms)
 #pragma unroll 1
-                for (int s = 0; s < E; ++s) sbuf[(p + P * s) * TT + t] = sbuf[(p + P * s) * TT + t] * fx_far(k);
-            }
-        };
-        if constexpr (NG % 32 == 0) transform(SyncGroup{1 + g, NG});
-        else transform(SyncBlock());
+            for (int s = 0; s < E; ++s) sbuf[(p + P * s) * TT + t] = sbuf[(p + P * s) * TT + t] * fx_far(k);
+        }
     }
     __syncthreads();
 
@@ -543,15 +541,15 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
             if constexpr (TWO) {
                 // a thread's modes come once as they are and once as the conjugates in another thread's slots:
                 // half of 2^60 for each of the two fields keeps its inputs' sum below 2^61
-                const int fa = fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_of(ba, 2), 0xffffffffu);
-                const int fb = fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_of(bb, 2), 0xffffffffu);
+                const int fa = fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_of(ba, 2));
+                const int fb = fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_of(bb, 2));
                 if (p % 32 == 0) {
                     firsts[lp][2 * g][p / 32] = fa;
                     firsts[lp][2 * g + 1][p / 32] = fb;
                 }
             }
-            fx_warp_bound<1, (P < 32 ? P : 32)>(ba, 0xffffffffu);
-            fx_warp_bound<1, (P < 32 ? P : 32)>(bb, 0xffffffffu);
+            fx_warp_bound<1, (P < 32 ? P : 32)>(ba);
+            fx_warp_bound<1, (P < 32 ? P : 32)>(bb);
             if (p % 32 == 0) {
                 bound[lp][2 * g][p / 32] = ba;
                 bound[lp][2 * g + 1][p / 32] = bb;
@@ -700,8 +698,8 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
 #pragma unroll
                 for (int s = 0; s < E; ++s) v[s] = mk(r0[p + P * s], r1[p + P * s]);
                 FxBound b = fx_bound(v);
-                int first = TWO ? fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_in(b, 1), 0xffffffffu) : 0;
-                fx_warp_bound<1, (P < 32 ? P : 32)>(b, 0xffffffffu);
+                int first = TWO ? fx_warp_min<1, (P < 32 ? P : 32)>(fx_scale_in(b, 1)) : 0;
+                fx_warp_bound<1, (P < 32 ? P : 32)>(b);
                 if constexpr (NW > 1) {
                     if (p % 32 == 0) {
                         bound[lp][g][p / 32] = b;

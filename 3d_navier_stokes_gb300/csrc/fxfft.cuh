@@ -230,15 +230,15 @@ __device__ __forceinline__ FxBound fx_join(FxBound a, FxBound b) {
 }
 // combine the bounds of the lanes of a warp that differ in the bits of LO..HI-1
 template <int LO, int HI>
-__device__ __forceinline__ void fx_warp_bound(FxBound& b, unsigned mask) {
+__device__ __forceinline__ void fx_warp_bound(FxBound& b) {
 #pragma unroll
     for (int o = LO; o < HI; o <<= 1)
-        b = fx_join(b, FxBound{__shfl_xor_sync(mask, b.sum, o), __shfl_xor_sync(mask, b.e, o)});
+        b = fx_join(b, FxBound{__shfl_xor_sync(0xffffffffu, b.sum, o), __shfl_xor_sync(0xffffffffu, b.e, o)});
 }
 template <int LO, int HI>
-__device__ __forceinline__ int fx_warp_min(int k, unsigned mask) {
+__device__ __forceinline__ int fx_warp_min(int k) {
 #pragma unroll
-    for (int o = LO; o < HI; o <<= 1) k = min(k, __shfl_xor_sync(mask, k, o));
+    for (int o = LO; o < HI; o <<= 1) k = min(k, __shfl_xor_sync(0xffffffffu, k, o));
     return k;
 }
 // Lines of 512 points and more take their scale in two steps. Scaled by the whole line's L1 norm,
@@ -273,13 +273,11 @@ template <bool TWO> __device__ __forceinline__ int fx_later(int first, int k) {
 // threads each, thread = (tile P + p) TT + t; with TWO the smallest `first` of its threads
 template <bool TWO, int P, int TT, int NT, typename Sync>
 __device__ __forceinline__ FxBound fx_line_bound(FxBound b, int& first, Sync sync) {
+    static_assert(NT % 32 == 0, "whole warps");
     if constexpr (P > 1) {
-        // the lanes of this warp (the last warp of a small block may be short)
-        const unsigned mask =
-            NT % 32 == 0 || (int)(threadIdx.x | 31) < NT ? 0xffffffffu : (1u << (NT % 32 ? NT % 32 : 31)) - 1u;
         constexpr int span = P * TT < 32 ? P * TT : 32;   // lanes that hold parts of one tile
-        fx_warp_bound<TT, span>(b, mask);
-        if constexpr (TWO) first = fx_warp_min<TT, span>(first, mask);
+        fx_warp_bound<TT, span>(b);
+        if constexpr (TWO) first = fx_warp_min<TT, span>(first);
         if constexpr (P * TT > 32) {
             // several warps per tile: one entry per warp and line
             constexpr int NW = P * TT / 32;
