@@ -245,6 +245,7 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
     }
     const long long xs = (long long)N * G::NZP;
     C* sbuf = buf + (size_t)g * N * TT;
+    __shared__ int line_scale[3][TT];
     // the stage algebra's modes of this thread: rows r0 + it RPI, it < NIT, of the band's 2 KC + 1;
     // their state is loaded CH rows at a time, before the transform where that is all of them
     constexpr int RPI = NT / TT, NIT = (2 * G::KC + RPI) / RPI, CH = NIT < 2 ? 1 : 2;
@@ -294,13 +295,14 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 #pragma unroll
         for (int s = 0; s < E; ++s)
             if (!fx_outside<PL>(s)) sbuf[(p + P * s) * TT + t] = mk(fx_to(a[s].x, kn), fx_to(a[s].y, kn));
-        if (k != kn) {   // rare; a branch around the conversions would part them from the last stage's
-                         // additions, which cover them (96^3 22 -> 28 us, 256^3 0.163 -> 0.175 ms)
-#pragma unroll 1
-            for (int s = 0; s < E; ++s) sbuf[(p + P * s) * TT + t] = sbuf[(p + P * s) * TT + t] * fx_far(k);
-        }
+        if (p == 0) line_scale[g][t] = k;
     }
     __syncthreads();
+    // rare scales: the mode loop multiplies by what the conversions left out (a branch beside those
+    // parts them from the last stage's additions, which cover them: 96^3 21.7 -> 23.4 us with a loop
+    // of its own behind them, 28 us with their code in it)
+    const bool far = line_scale[0][t] != fx_near(line_scale[0][t]) || line_scale[1][t] != fx_near(line_scale[1][t]) ||
+                     line_scale[2][t] != fx_near(line_scale[2][t]);
 
     const double* kxs = aux + G::KC2 + 1;
     const double fky = ky;
@@ -322,6 +324,13 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
         C n[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) n[c] = buf[(c * N + i) * TT + t];
+        if (far) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int k = line_scale[c][t];
+                if (k != fx_near(k)) n[c] = n[c] * fx_far(k);
+            }
+        }
         if (MODE != X_PLAIN) {
             // Leray projection; the mean is removed
             const double fkx = __ldg(&kxs[i]), kinv = __ldg(&aux[k2]);
