@@ -34,7 +34,8 @@ constexpr int fx_ctas(int per_sm, int threads) { return per_sm / threads < 1 ? 1
 // threads per line, 512 below (256^3 0.164 -> 0.160 ms, 128^3 0.0253 against 0.0258).
 // Forward: two CTAs of 384 threads or one of 768 (80 registers, a few spills, but one
 // CTA's transforms under the other's FP64 work: 256^3 0.208 -> 0.166 ms, 512^3 1.96 ->
-// 1.51 ms), 576 threads with smaller CTAs (128^3 0.0395 -> 0.0343 ms, 0.0411 with 768).
+// 1.51 ms, now 0.163 and 1.47 ms), 576 threads with smaller CTAs (128^3 0.0395 -> 0.0343 ms,
+// 0.0411 with 768).
 template <int N> constexpr int fxinv_ctas() { return fx_ctas(FxPlan<N>::X::P >= 16 ? 640 : 512, fxinv_threads<N>()); }
 template <int N> constexpr int fxfwd_ctas() { return fx_ctas(fxfwd_threads<N>() >= 384 ? 768 : 576, fxfwd_threads<N>()); }
 template <int N> constexpr int fxinv_smem() { return N * fx_tile<N>() * 16; }
@@ -44,8 +45,8 @@ template <int N> constexpr int fxfwd_smem() { return 3 * N * fx_tile<N, true>() 
 // The curl is formed on the modes of the sphere (a third of a column's rows), where the
 // FP64 pipe has to do less than for the transformed columns, and the six fields are
 // independent CTAs, which fills the chip at small N (32^3: 11 us per launch, 27 us with
-// the six transforms in one CTA; 256^3: 0.19 against 0.25 ms). The inputs' second and
-// third reads hit L2.
+// the six transforms in one CTA, now 8.4 us; 256^3: 0.19 against 0.25 ms, now 0.157). The
+// inputs' second and third reads hit L2.
 template <int N>
 __global__ void __launch_bounds__(fxinv_threads<N>(), fxinv_ctas<N>())
 k_xinv_fx(const cx<double>* __restrict__ U, cx<q64>* __restrict__ W, int* __restrict__ scales,
@@ -197,7 +198,7 @@ k_ypass_fx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __rest
 // algebra. The mode loop's FP64 work is a large part (FP64 pipe 44 % busy at 256^3 with the
 // division and conversions it had), so 1/k2 comes from `aux` and the per-step factors are
 // formed once per thread. Three groups instead of one after the other: 24 -> 14 us per
-// launch at 32^3, 0.226 -> 0.212 ms at 256^3.
+// launch at 32^3, 0.226 -> 0.212 ms at 256^3 (now 10 us and 0.163 ms).
 template <int N, int INTEG, int MODE>
 __global__ void __launch_bounds__(fxfwd_threads<N>(), fxfwd_ctas<N>())
 k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* __restrict__ U,
@@ -423,9 +424,10 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 // then holds its real-space output, so 96 bytes of shared memory per grid point of
 // a pair are enough for four 96-thread CTAs per SM; where a group lies inside a
 // warp it synchronises with its warp only. 1.24 -> 0.60 ms per launch at 256^3 against
-// the CTA-synchronous pass with transforms that convert at both ends and FP64 products;
-// issue bound (49 % of slots, instruction fetch the largest stall: CTAs of 192 and 384
-// threads, whose warps run in step, measured 0.64 and 0.73 ms).
+// the CTA-synchronous pass with transforms that convert at both ends and FP64 products (CTAs
+// of 192 and 384 threads, whose warps run in step, measured 0.64 and 0.73 ms then); with the
+// work array in integers 0.556, with the scales per field and the peaks below 0.567 ms.
+// Issue bound.
 // ---------------------------------------------------------------------------
 // Exchange slots of a line, 16-byte elements, 8 lanes (one wavefront) at a time: m + (m >> A),
 // lines XS slots apart. One pad slot per 16 counts 2.0 - 2.1 wavefronts per access at 8, 24 and
@@ -434,8 +436,8 @@ k_xfwd_fx(const cx<q64>* __restrict__ W, int* __restrict__ scales, cx<double>* _
 // From 256 points on a line's own peaks, not the bound by its modes, set the scales of the products'
 // operands: operands of 2^60 / sqrt(N) each lose log2 N bits between them. White flow in a plane,
 // relative error of the right-hand side at 128, 192, 256, 384 and 512 points without the peaks 2.6,
-// 4.1, 5.9, 6.8 and 8.8e-16 (FP64 butterflies 5.0, 6.1, 5.7, 5.9 and 6.3e-16), with them at 256
-// 4.0e-16; they cost 5 % of this pass.
+// 4.1, 5.9, 6.8 and 8.8e-16 (FP64 butterflies 5.0, 6.1, 5.7, 5.9 and 6.3e-16), with them at 256,
+// 384 and 512 3.9, 5.5 and 7.0e-16; they cost 3.5 % of this pass (0.547 -> 0.567 ms at 256^3).
 template <int N> constexpr bool zfx_peaks() { return N >= 256; }
 template <int N> struct FxLay { static constexpr int A = 4, XS = zpad<N>(); };
 template <> struct FxLay<8> { static constexpr int A = 2, XS = 12; };

@@ -8,20 +8,24 @@
 // line's L1 norm. Each line is therefore scaled by the power of two that keeps its
 // L1 norm below 2^61, held in 64-bit integers and transformed with exact 64-bit
 // additions and 64x60-bit twiddle products (both parts of the product that reach the
-// result's last bit). No stage needs a shift and nothing can overflow. The absolute
-// error is about one unit of 2^-61 of the L1 norm per input and per twiddle product,
-// below the rounding errors of the FP64 butterflies it replaces (measured against
-// 64-bit library transforms in tests/test_fx_fft.py).
+// result's last bit), so that nothing can overflow. The absolute error is about one unit
+// of 2^-61 of the L1 norm per input and per twiddle product. Against the values that
+// grows like sqrt(N), an FP64 butterfly's error only like sqrt(log N); long lines
+// therefore take their scale in two steps (fx_two).
 //
 // Between the passes the fields stay integers, each line with its scale k (value =
 // integer 2^-k) in a table beside them (FxScales); the next pass brings a line's
 // elements to a common scale. Doubles are read and written on the sphere's modes only
 // (the x passes), and the integers' range does not end at FP64's exponents.
 //
-// Measured on a GB300 against FP64 butterflies (one RK4 step): 32^3 0.312 -> 0.074 ms, 128^3
-// 3.55 -> 0.62 ms, 256^3 28.3 -> 4.64 ms, 512^3 250 -> 44.8 ms; the nonlinear term's error
-// against a 113-bit evaluation at 16^3 .. 48^3 falls from 3.1e-16 .. 9.9e-16 to 7.4e-17 ..
-// 2.4e-16.
+// Measured on a GB300 against FP64 butterflies (one RK4 step): 32^3 0.312 -> 0.073 ms, 128^3
+// 3.55 -> 0.63 ms, 256^3 28.3 -> 4.70 ms, 512^3 250 -> 47.1 ms. Relative error of the
+// nonlinear term against double-double transforms, butterflies -> these, at 24, 64, 256 and
+// 512 points: white fields 7.0, 8.3, 34, 73e-16 -> 2.1, 1.8, 4.1, 4.0e-16 (the packed z lines of
+// the butterflies carried u_z beside the larger w_x), k^-5/3 spectra 6.0, 4.7, 6.8, 8.8e-16 ->
+// 2.0, 1.6, 2.5, 2.4e-16; white flows in a plane, which have no such pair, at 24, 96, 256 and
+// 512 points 5.3, 5.6, 5.7, 6.3e-16 -> 2.2, 2.9, 3.9, 3.7e-16. tests/test_fx_precision.py holds
+// plane flows of 24 .. 768 points to a unit of 2^-53 per radix-2 level.
 //
 // Lines that hold a NaN or Inf carry the scale kFxBad and end as NaN throughout, as any
 // transform of them does; lines of zeros the scale kFxZero. The range of inputs and results is
@@ -355,7 +359,7 @@ __device__ __forceinline__ double fx_to_any(q64 a, int k) {
 }
 // slot s of every thread lies outside the kept band |k| <= KC = N / 3: a quarter of the
 // slots of 16, neither loaded nor added by an inverse transform, nor stored by a forward
-// one (256^3 y passes 0.272 + 0.142 -> 0.255 + 0.132 ms)
+// one (256^3 y passes, when they took 0.272 + 0.142 ms: to 0.255 + 0.132; now 0.201 + 0.108)
 template <class PL> constexpr bool fx_outside(int s) {
     return PL::P * s > PL::N / 3 && PL::P * s + PL::P - 1 < PL::N - PL::N / 3;
 }

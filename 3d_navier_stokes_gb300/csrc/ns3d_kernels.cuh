@@ -88,7 +88,9 @@ template <> struct Plans<768>  { using A = Plan<768, 12, 4, 4, 4, 4, 3>; using X
 // us (sixteen 656 -> 668 us; with 6 elements in the y and z lines too 121 and 831 us), 64^3 131
 // -> 121 us (eight 577 -> 583 us; y and z lines too: 141 us). 96 and 128 points: 6 and 8
 // elements in the x lines gave nothing (375 and 632 us). 512 points: 16 x 8 x 4 has fewer
-// twiddle products than 8 x 8 x 8 (45.9 -> 44.8 ms).
+// twiddle products than 8 x 8 x 8 (45.9 -> 44.8 ms, before the scale in two steps). 768 points:
+// 12 first, because the first stage's growth is what the second scale step keeps (fx_two): with
+// 4 first the right-hand side of a white plane flow has an error of 8.7e-16, so 4.4e-16.
 template <int N> struct FxPlan { using A = typename Plans<N>::A; using X = A; };
 template <> struct FxPlan<8>   { using A = Plan<8, 2, 2, 2, 2>;      using X = A; };
 template <> struct FxPlan<16>  { using A = Plan<16, 2, 2, 2, 2, 2>; using X = A; };
@@ -169,7 +171,8 @@ template <typename T, int N, int V = 0, bool INV = true> constexpr int tile_a() 
 template <int N, bool FWD = false> constexpr int fx_tile() { return FxPlan<N>::X::P * 8 <= (FWD ? 128 : 256) ? 8 : 4; }
 // FP32: at most 128 threads per CTA up to 64 points (64^3, tiles of 16 -> 8 pencils: 61.4 ->
 // 55.3 us per step), 8 pencils with S, and in the inverse pass of variant 0 at 192 and 256
-// points (27.9 -> 25.3 and 65.5 -> 53.6 us per launch; 384 points 222 -> 240 us).
+// points (27.9 -> 25.3 and 65.5 -> 53.6 us per launch; 384 points 222 -> 240 us). The shipped
+// shapes run 256 points in variant 6: this is what a context without them gets.
 template <typename T, int N, int V = 0, bool FWD = false, bool S = false> constexpr int tile_x() {
     if constexpr (sizeof(T) == 8) return fx_tile<N, FWD>();
     else {
@@ -182,7 +185,8 @@ template <typename T, int N, int V = 0, bool FWD = false, bool S = false> conste
 // same, so that a member's result does not depend on how many there are): more, smaller CTAs.
 // One RK4 step of 48^3 65.3 -> 63.4 us (four members 86 -> 80, eight 129 -> 121, 24 262 -> 268
 // us), of 96^3 133 -> 129 us (two members 191 -> 188 us), of 128^3 187 -> 184 us (two members
-// 324 -> 328 us).
+// 324 -> 328 us; the shipped shapes run 128 points in variant 2). The other sizes fill the chip
+// with 16 pencils or have 8 already.
 template <int N, int V> constexpr bool x_small(int members) {
     return V == 0 && ((N == 48 && members <= 8) || (N == 96 && members <= 2) || (N == 128 && members == 1));
 }

@@ -19,10 +19,11 @@ constexpr long long kWaitCycles = 4000000000LL;
 constexpr int kStatusTimeout = 6;
 
 // Start of a kernel launched with programmatic stream serialization (Launcher,
-// ns3d_impl.cuh): waits until the kernels before it have completed and their writes
+// launch.cuh): waits until the kernels before it have completed and their writes
 // are visible (no kernel lets its successor's blocks start earlier than that: measured
-// slower, 256^3 FP32 1.36 -> 1.59 ms per step, 64^3 72 -> 84 us). Returns 0, added to every pointer to data that earlier kernels write, so that no
-// load of it can be moved above the wait.
+// slower, 256^3 FP32 1.36 -> 1.59 ms per step, 64^3 72 -> 84 us). Returns 0, added to
+// every pointer to data that earlier kernels write, so that no load of it can be moved
+// above the wait.
 __device__ __forceinline__ long long pdl_begin() {
     long long zero;
     asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(zero)::"memory");
