@@ -615,6 +615,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
             if constexpr (MODE == 0) {
                 // u x w: (ux, uy), (uz, wx), (wy, wz) -> (Nx, Ny), (Nz, -); 3 P / 2 threads per line
                 constexpr int NL = 3 * P / 2;
+                static_assert(P % 2 == 0 && (E % 2 == 0 || !zfx_peaks<N>()), "whole threads per line, elements in pairs");
                 const int line = threadIdx.x / NL;   // of the CTA's 2 ZP
                 int h[6], k[6];   // bits to a field's peak, and its scale with them
 #pragma unroll
@@ -624,7 +625,7 @@ k_zfx(cx<q64>* __restrict__ W, int* __restrict__ scales, const int4* __restrict_
                         unsigned t = peak[line][f / 2][0];
 #pragma unroll
                         for (int w = 1; w < NW; ++w) t = __vimin3_u16x2(t, t, peak[line][f / 2][w]);
-                        h[f] = (int)(f % 2 ? t >> 16 : t & 0xffffu) - 4;   // values below 2^60
+                        h[f] = max((int)(f % 2 ? t >> 16 : t & 0xffffu) - 4, 0);   // values below 2^60
                     }
                     k[f] = scale[line][f] + h[f];
                 }
