@@ -210,3 +210,50 @@ def test_against_device_transforms(ns3d, N):
     d = sum(ks[c] * n[c] for c in range(3)) / k2.clamp(min=1)
     for c in range(3):
         assert err(got[..., c], (n[c] - ks[c] * d) * keep * (k2 > 0)) < unit * 3, c
+
+
+def test_stage_weights_are_rounded_once(ns3d):
+    """The IF-RK4 weights h / 6 and h / 3 are the nearest doubles. With a step h whose sixth rounds to
+    2e-17, while the product h (1 / 6) is off by 9e-17, the error of one step's increment along
+    itself tells the two apart: the other errors are random over the modes."""
+    sfft = pytest.importorskip("scipy.fft")
+    from fractions import Fraction as F
+    if np.finfo(np.longdouble).nmant < 63:
+        pytest.skip("no extended precision")
+    N = 48
+    (fx, fz), k, kz, keep = plane_flow(N)
+    k2 = np.where(keep & (k * k + kz * kz > 0), k * k + kz * kz, np.inf)
+    d = (k * fx + kz * fz) / k2
+    fx, fz = (fx - k * d) * np.isfinite(k2), (fz - kz * d) * np.isfinite(k2)
+
+    def rhs(a):
+        ux, uz, wy = (sfft.irfft2(q, s=(N, N)) for q in (a[0], a[1], 1j * (kz * a[0] - k * a[1])))
+        n = [sfft.rfft2(-uz * wy), sfft.rfft2(ux * wy)]
+        e = (k * n[0] + kz * n[1]) / k2
+        return np.stack([(n[0] - k * e) * np.isfinite(k2), (n[1] - kz * e) * np.isfinite(k2)])
+
+    u = np.stack([fx, fz])
+    scale = np.linalg.norm(u.ravel()) / np.linalg.norm(rhs(u).ravel())
+    rng = np.random.default_rng(0)
+    best, h = 0, None
+    for c in scale * rng.uniform(0.7, 1.0, 20000):
+        six = F(float(c)) / 6
+        off = [abs(float((F(q) - six) / six)) for q in (float(c) * (1.0 / 6.0), float(c) / 6.0)]
+        if off[0] - off[1] > best:
+            best, h = off[0] - off[1], float(c)
+    assert best > 7e-17
+    f = np.zeros((N, N, N // 2 + 1, 3), np.complex128)
+    f[:, 0, :, 0], f[:, 0, :, 2] = fx * N, fz * N
+    s = ns3d.Solver(N, nu=1e-30, dt=h, integrator="ifrk4")
+    s.set_state(f)
+    s.RK4Step(1)
+    g = s.get_state()[:, 0]
+    s.close()
+    u, h = u.astype(np.clongdouble), np.longdouble(h)
+    k1 = rhs(u)
+    k2_ = rhs(u + h / 2 * k1)
+    k3 = rhs(u + h / 2 * k2_)
+    step = h / 6 * (k1 + 2 * k2_ + 2 * k3 + rhs(u + h * k3))
+    err = np.stack([g[..., 0], g[..., 2]]) / N - (u + step)
+    slope = float(np.sum((err * np.conj(step)).real) / np.sum(np.abs(step) ** 2))
+    assert abs(slope) < 5e-17
